@@ -226,6 +226,10 @@ TaskDev make_task(const qk_contract &b, int ppt, int lane_mode) {
     const float Lf = t.cf.exp_m_lambda_dt;
     const double kd = std::ceil(static_cast<double>(Lf) * 8388608.0 - 0.5);
     t.jump_kmin = static_cast<uint32_t>(std::min(std::max(kd, 0.0), 8388608.0));
+    // FP64: (w + 1/2) 2^-32 >= L  <=>  w >= ceil(L 2^32 - 1/2) (both exact); capped, so that at
+    // L = 1 the largest word still reaches the exact test
+    t.jump_kmin64 = static_cast<uint32_t>(
+        std::min(std::max(std::ceil(t.cd.exp_m_lambda_dt * 4294967296.0 - 0.5), 0.0), 4294967295.0));
     t.lane_mode = b.antithetic ? kLanePair : lane_mode;
     t.track = needs_path_state(b) ? 1 : 0;
     const int64_t units = lane_units(b.n_paths, t.lane_mode);

@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 
 #include "qk_internal.h"
+#include "qk_math64.cuh"
 
 namespace qk {
 
@@ -70,8 +71,8 @@ __device__ __forceinline__ U4 philox4x32_10(U4 c, const PhiloxRoundKeys &rk) {
 }
 
 // ============================================================================
-// Arithmetic policy.  FP32 uses the SFU (MUFU) approximations explicitly;
-// FP64 uses the correctly-rounded / IEEE CUDA library functions.
+// Arithmetic policy.  FP32 uses the SFU (MUFU) approximations explicitly; FP64 uses the
+// functions of qk_math64.cuh in the path loop and the CUDA library in rare code.
 // ============================================================================
 template <class R>
 struct Math;
@@ -155,11 +156,7 @@ struct Math<float> {
 template <>
 struct Math<double> {
     static __device__ __forceinline__ double exp(double x) { return ::exp(x); }
-    static __device__ __forceinline__ double log(double x) { return ::log(x); }
     static __device__ __forceinline__ double sqrt(double x) { return ::sqrt(x); }
-    static __device__ __forceinline__ double rcp(double x) { return 1.0 / x; }
-    static __device__ __forceinline__ double div(double a, double b) { return a / b; }
-    static __device__ __forceinline__ double erf(double x) { return ::erf(x); }
     static __device__ __forceinline__ double u01(uint32_t w) {
         return (static_cast<double>(w) + 0.5) * (1.0 / 4294967296.0);
     }
@@ -251,97 +248,19 @@ struct FedStep {
 };
 
 // ============================================================================
-// Scheme steps.  Each follows the reference's evolve_step line for line; the
-// only rewrite is QE's quadratic-branch martingale term, where
-// log(exp(X)/sqrt(t)) is evaluated as X - log(t)/2 (the same quantity without
-// an exp/rsqrt/log round trip).
+// Scheme steps: Heston + Euler (include/core/schemes/markovian/MSchemes.hpp:133-156),
+// + implicit Milstein (MSchemes.hpp:229-253), + Andersen QE with martingale correction
+// (MSchemes.hpp:363-442), in FP32 on the spot and in FP64 on its logarithm.  QE's
+// quadratic-branch martingale term log(exp(X)/sqrt(t)) is evaluated as X - log(t)/2 (the
+// same quantity without an exp/rsqrt/log round trip).
 // ============================================================================
 
-// Heston + Euler: include/core/schemes/markovian/MSchemes.hpp:133-156
-template <class R>
-__device__ __forceinline__ void step_euler(const StepConst<R> &p, R &S, R &v, R Z1, R Z2) {
-    const R Zv = Z1;
-    const R ZS = p.rho * Z1 + p.rho_c * Z2;
-    const R sqv = Math<R>::sqrt(v);
-    const R ex = p.r_minus_q_dt - v * p.half_dt + (sqv * p.sqrt_dt) * ZS;
-    const R Sn = S * Math<R>::exp(ex);
-    const R vn = v * p.one_minus_k_dt + p.k_theta_dt + (p.sigma_sqrt_dt * sqv) * Zv;
-    S = Sn;
-    v = rmax(vn, R(0));
-}
-
-// Heston + implicit Milstein: MSchemes.hpp:229-253
-template <class R>
-__device__ __forceinline__ void step_milstein(const StepConst<R> &p, R &S, R &v, R Z1, R Z2) {
-    const R Zv = Z1;
-    const R ZS = p.rho * Z1 + p.rho_c * Z2;
-    const R sqv = Math<R>::sqrt(v);
-    const R ex = p.r_minus_q_dt - v * p.half_dt + (sqv * p.sqrt_dt) * ZS;
-    const R Sn = S * Math<R>::exp(ex);
-    const R corr = p.quarter_sigma_sq_dt * (Zv * Zv - R(1));
-    const R vn = p.implicit_den * (v + p.k_theta_dt + (p.sigma_sqrt_dt * sqv) * Zv + corr);
-    S = Sn;
-    v = rmax(vn, R(0));
-}
-
-// Heston + Andersen QE with martingale correction: MSchemes.hpp:363-442
-template <class R>
-__device__ __forceinline__ void step_qe(const StepConst<R> &p, R &S, R &v, R Zv, R Zind) {
-    const R m = v * p.exp_mkdt + p.theta_m;
-    const R s2 = v * p.s2f1 + p.s2f2;
-    R vn;
-    R logM;  // log of the martingale factor M
-    if (m <= p.eps) {
-        vn = R(0);
-        logM = R(0);
-    } else {
-        // psi = s2 / m^2 is compared as s2 against eps m^2 and psi_c m^2 (m > 0)
-        const R m2 = m * m;
-        if (s2 <= p.eps * m2) {
-            vn = m;
-            logM = R(0);
-        } else if (s2 <= p.psi_c * m2) {
-            const R two_ip = R(2) * m2 * Math<R>::rcp(s2);  // 2 / psi
-            const R b2 = two_ip - R(1) + Math<R>::sqrt(two_ip * (two_ip - R(1)));
-            const R a = m * Math<R>::rcp(R(1) + b2);
-            const R bz = Math<R>::sqrt(b2) + Zv;
-            vn = a * bz * bz;
-            // min(A, 0.5/a - eps) enters only through its product with a > 0:
-            // safe_A a = min(A a, 0.5 - eps a)
-            const R Aa = rmin(p.A * a, R(0.5) - p.eps * a);
-            const R term = R(1) - R(2) * Aa;
-            // M = exp(A b2 a / term) / sqrt(term)  =>  log M = A b2 a / term - log(term) / 2
-            logM = Aa * b2 * Math<R>::rcp(term) - R(0.5) * Math<R>::log(term);
-        } else {
-            const R inv_m = Math<R>::rcp(m);
-            const R psi = s2 * inv_m * inv_m;
-            const R pz = Math<R>::div(psi - R(1), psi + R(1));
-            const R beta = (R(1) - pz) * inv_m;
-            const R U = R(0.5) * (R(1) + Math<R>::erf(Zv * p.inv_sqrt2));
-            if (U <= pz) {
-                vn = R(0);
-            } else {
-                const R safe_U = rmin(U, R(1) - p.eps);
-                vn = Math<R>::div(Math<R>::log(Math<R>::div(R(1) - pz, R(1) - safe_U)), beta);
-            }
-            const R safe_A = rmin(p.A, beta - p.eps);
-            const R M = pz + Math<R>::div(beta * (R(1) - pz), beta - safe_A);
-            logM = Math<R>::log(M);
-        }
-    }
-    const R K0 = -logM - p.K1_half_K3 * v;
-    const R isig = p.K3 * v + p.K4 * vn;
-    const R ex = p.r_minus_q_dt + K0 + (p.K1 * v + p.K2 * vn) + Math<R>::sqrt(isig) * Zind;
-    S = S * Math<R>::exp(ex);
-    v = vn;
-}
-
 // ----------------------------------------------------------------------------
-// FP32 QE and Euler with an explicit rounding order.  Every FP32 operation below
+// FP32 steps with an explicit rounding order.  Every FP32 operation below
 // is an IEEE-rounded intrinsic (no compiler contraction), and the paired two-path
 // forms further down perform the same operations on float2 pairs with the sm_100
 // paired FP32 instructions, so one path gives the same bits whichever form
-// simulates it.  Same algebra as the generic steps above.
+// simulates it.
 __device__ __forceinline__ void qe_quadratic_f32(const StepConst<float> &p, float m, float m2, float s2, float Zv,
                                                  float &vn, float &logM) {
     const float two_ip = __fmul_rn(__fmul_rn(2.0f, m2), ptx_rcp(s2));
@@ -364,8 +283,7 @@ __device__ __forceinline__ void qe_spot_f32(const StepConst<float> &p, float &S,
     S = __fmul_rn(S, ptx_ex2(__fmul_rn(ex, Math<float>::kLog2e)));
 }
 
-template <>
-__device__ __forceinline__ void step_qe<float>(const StepConst<float> &p, float &S, float &v, float Zv, float Zind) {
+__device__ __forceinline__ void step_qe_f32(const StepConst<float> &p, float &S, float &v, float Zv, float Zind) {
     const float m = __fmaf_rn(v, p.exp_mkdt, p.theta_m);
     const float s2 = __fmaf_rn(v, p.s2f1, p.s2f2);
     const float m2 = __fmul_rn(m, m);
@@ -380,7 +298,7 @@ __device__ __forceinline__ void step_qe<float>(const StepConst<float> &p, float 
         vn = m;
         logM = 0.0f;
     } else if (!(s2 <= __fmul_rn(p.psi_c, m2))) {
-        // exponential branch (rare at the usual parameters): as the generic step
+        // exponential branch (rare at the usual parameters)
         const float inv_m = ptx_rcp(m);
         const float psi = s2 * inv_m * inv_m;
         const float pz = Math<float>::div(psi - 1.0f, psi + 1.0f);
@@ -400,8 +318,7 @@ __device__ __forceinline__ void step_qe<float>(const StepConst<float> &p, float 
     v = vn;
 }
 
-template <>
-__device__ __forceinline__ void step_euler<float>(const StepConst<float> &p, float &S, float &v, float Z1, float Z2) {
+__device__ __forceinline__ void step_euler_f32(const StepConst<float> &p, float &S, float &v, float Z1, float Z2) {
     const float ZS = __fmaf_rn(p.rho, Z1, __fmul_rn(p.rho_c, Z2));
     const float sqv = ptx_sqrt(v);
     const float ex = __fmaf_rn(__fmul_rn(sqv, p.sqrt_dt), ZS, __fmaf_rn(v, -p.half_dt, p.r_minus_q_dt));
@@ -416,9 +333,7 @@ __device__ __forceinline__ float milstein_variance_f32(const StepConst<float> &p
     return fmaxf(__fmul_rn(p.implicit_den, t), 0.0f);
 }
 
-template <>
-__device__ __forceinline__ void step_milstein<float>(const StepConst<float> &p, float &S, float &v, float Z1,
-                                                     float Z2) {
+__device__ __forceinline__ void step_milstein_f32(const StepConst<float> &p, float &S, float &v, float Z1, float Z2) {
     const float ZS = __fmaf_rn(p.rho, Z1, __fmul_rn(p.rho_c, Z2));
     const float sqv = ptx_sqrt(v);
     const float ex = __fmaf_rn(__fmul_rn(sqv, p.sqrt_dt), ZS, __fmaf_rn(v, -p.half_dt, p.r_minus_q_dt));
@@ -436,7 +351,7 @@ __device__ __forceinline__ float2 min2(float2 a, float2 b) { return make_float2(
 __device__ __forceinline__ float2 max0_2(float2 a) { return make_float2(fmaxf(a.x, 0.0f), fmaxf(a.y, 0.0f)); }
 
 // QE step of two paths (spot S, variance v as pairs): paired when both take the
-// quadratic branch (the common case), otherwise each path through step_qe<float>.
+// quadratic branch (the common case), otherwise each path through step_qe_f32.
 __device__ __forceinline__ void step_qe_two_f32(const StepConst<float> &p, float2 &S, float2 &v, float2 Zv,
                                                 float2 Zind) {
     const float2 m = __ffma2_rn(v, f2(p.exp_mkdt), f2(p.theta_m));
@@ -474,7 +389,7 @@ __device__ __forceinline__ void step_qe_two_f32(const StepConst<float> &p, float
 #pragma unroll 1
         for (int i = 0; i < 2; ++i) {
             float Si = i ? S.y : S.x, vi = i ? v.y : v.x;
-            step_qe<float>(p, Si, vi, i ? Zv.y : Zv.x, i ? Zind.y : Zind.x);
+            step_qe_f32(p, Si, vi, i ? Zv.y : Zv.x, i ? Zind.y : Zind.x);
             if (i) {
                 S.y = Si;
                 v.y = vi;
@@ -507,15 +422,123 @@ __device__ __forceinline__ void step_euler_two_f32(const StepConst<float> &p, fl
                           __ffma2_rn(v, f2(p.one_minus_k_dt), f2(p.k_theta_dt))));
 }
 
-template <class R, int SCHEME>
-__device__ __forceinline__ void heston_step(const StepConst<R> &p, R &S, R &v, R Z1, R Z2) {
-    if constexpr (SCHEME == kEuler) {
-        step_euler<R>(p, S, v, Z1, Z2);
-    } else if constexpr (SCHEME == kMilstein) {
-        step_milstein<R>(p, S, v, Z1, Z2);
-    } else {
-        step_qe<R>(p, S, v, Z1, Z2);
+template <int SCHEME>
+__device__ __forceinline__ void heston_step_f32(const StepConst<float> &p, float &S, float &v, float Z1, float Z2) {
+    if constexpr (SCHEME == kEuler) step_euler_f32(p, S, v, Z1, Z2);
+    else if constexpr (SCHEME == kMilstein) step_milstein_f32(p, S, v, Z1, Z2);
+    else step_qe_f32(p, S, v, Z1, Z2);
+}
+
+// ----------------------------------------------------------------------------
+// FP64 steps on the base-2 logarithm x of S / S0: one path-step then needs no
+// exponential (a spot is formed only where something reads it), and every operation is
+// one of qk_math64.cuh's.
+//
+// QE, quadratic regime, with h = s^2 / 2, G = sqrt(m^2 - h) (h < m^2 as psi <= psi_c < 2)
+// and q = m + G.  The textbook's b^2 = 2/psi - 1 + sqrt(2/psi (2/psi - 1)) and
+// a = m / (1 + b^2) are, multiplied out, a b^2 = G and a = h / q, so that
+//   vn = a (b + Zv)^2,  b = G / sqrt(a G),
+//   1 - 2 A a = u / q,  u = q - 2 A h,   A a b^2 / (1 - 2 A a) = A G q / u,
+// and one reciprocal of q u serves both q and u: a square root, a reciprocal and a
+// reciprocal square root in place of three reciprocals and two square roots.  The
+// martingale factor's sqrt(1 - 2 A a) goes into the running product P, folded into x by
+// one logarithm per 16 steps.
+// ----------------------------------------------------------------------------
+struct Path64 {
+    double x, P, v;  // log2(S / S0) = x + log2(P) / 2
+};
+
+// The regimes of a QE step as the reference branches between them (MSchemes.hpp:363-442);
+// (vn, log M).  Reached when a step is not plainly inside the quadratic regime.
+__device__ __noinline__ inline double2 qe_regimes64(double m, double s2, double Zv, double psi_c, double eps, double A) {
+    if (m <= eps) return make_double2(0.0, 0.0);
+    const double m2 = m * m;
+    if (s2 <= eps * m2) return make_double2(m, 0.0);
+    if (s2 <= psi_c * m2) {
+        const double two_ip = 2.0 * m2 / s2;
+        const double b2 = two_ip - 1.0 + ::sqrt(two_ip * (two_ip - 1.0));
+        const double a = m / (1.0 + b2);
+        const double bz = ::sqrt(b2) + Zv;
+        const double Aa = fmin(A * a, 0.5 - eps * a);  // min(A, 1/(2a) - eps) a
+        const double term = 1.0 - 2.0 * Aa;
+        return make_double2(a * bz * bz, Aa * b2 / term - 0.5 * ::log(term));
     }
+    const double inv_m = 1.0 / m;
+    const double psi = s2 * inv_m * inv_m;
+    const double pz = (psi - 1.0) / (psi + 1.0);
+    const double beta = (1.0 - pz) * inv_m;
+    const double U = 0.5 * (1.0 + ::erf(Zv * 0.70710678118654752440));
+    const double vn = U <= pz ? 0.0 : ::log((1.0 - pz) / (1.0 - fmin(U, 1.0 - eps))) / beta;
+    const double safe_A = fmin(A, beta - eps);
+    return make_double2(vn, ::log(pz + beta * (1.0 - pz) / (beta - safe_A)));
+}
+
+__device__ __forceinline__ bool below_hi64(double a, double b) { return __double2hiint(a) < __double2hiint(b); }
+
+template <int SCHEME>
+__device__ __forceinline__ void step64(const StepConst<double> &p, Path64 &s, double Z1, double Z2) {
+    const double v = s.v;
+    if constexpr (SCHEME != kQE) {
+        const double sq = sqrt64(v);
+        const double ZS = fma(p.rho, Z1, p.rho_c * Z2);
+        s.x += fma(sq * p.l_sqrt_dt, ZS, fma(v, -p.l_half_dt, p.l_drift));
+        const double noise = (p.sigma_sqrt_dt * sq) * Z1;
+        if constexpr (SCHEME == kEuler) {
+            s.v = max0_64(fma(v, p.one_minus_k_dt, p.k_theta_dt) + noise);
+        } else {
+            const double corr = p.quarter_sigma_sq_dt * fma(Z1, Z1, -1.0);
+            s.v = max0_64(p.implicit_den * (((v + p.k_theta_dt) + noise) + corr));
+        }
+    } else {
+        const double m = fma(v, p.exp_mkdt, p.theta_m);
+        const double h = fma(v, p.h_f1, p.h_f2);
+        const double m2 = m * m;
+        const double G = sqrt_pos64(m2 - h);
+        const double q = m + G;
+        const double u = fma(-p.two_A, h, q);
+        const double R = rcp64(q * u);
+        const double iq = u * R;
+        const double a = h * iq;
+        const double b = G * rsqrt64(a * G);
+        const double bz = b + Z1;
+        double vn = (a * bz) * bz;
+        const double term = u * iq;
+        double dx = -p.l_A * ((G * q) * (q * R));
+        // Inside the quadratic regime (m, s^2 > eps m^2, s^2 <= psi_c m^2) with the clamp of
+        // A inactive (term far from 0)?  Compared by the high words of the (positive) values,
+        // strictly, so a value next to a threshold takes the exact branches.  eps and the
+        // bounds on m and term: m in (eps, 2^19), term in (2^-20, 2^40).
+        const bool quad =
+            static_cast<uint32_t>(__double2hiint(m) - __double2hiint(p.eps) - 1) <
+                static_cast<uint32_t>(0x41200000 - __double2hiint(p.eps) - 1) &&
+            below_hi64(h, p.h_psi * m2) && below_hi64(p.h_eps * m2, h) &&
+            static_cast<uint32_t>(__double2hiint(term) - 0x3EB00000) < 0x03C00000u;
+        if (!quad) {
+            const double2 r = qe_regimes64(m, 2.0 * h, Z1, p.psi_c, p.eps, p.A);
+            vn = r.x;
+            dx = -1.44269504088896340736 * r.y;
+        } else {
+            s.P *= term;
+        }
+        s.x += fma(sqrt64(v + vn), p.l_sqrt_K3 * Z2, fma(p.l_K2, vn, fma(p.l_c1, v, p.l_drift)) + dx);
+        s.v = vn;
+    }
+}
+
+// P into x (at the latest every 16 steps, so that P stays in range).
+template <int SCHEME>
+__device__ __forceinline__ void fold64(const Tab64 &t, Path64 &s) {
+    if constexpr (SCHEME == kQE) {
+        s.x = fma(neg2_log64(t, s.P, 0), -0.25 * 1.44269504088896340736, s.x);
+        s.P = 1.0;
+    }
+}
+
+// S / S0
+template <int SCHEME>
+__device__ __forceinline__ double rel_spot64(const Tab64 &t, const Path64 &s) {
+    if constexpr (SCHEME == kQE) return exp2_64(t, s.x) * sqrt_pos64(s.P);
+    else return exp2_64(t, s.x);
 }
 
 // Bates jump part after the (drift-compensated) Heston step: MSchemes.hpp:493-526.
@@ -556,11 +579,20 @@ __device__ __forceinline__ void bates_jump(const StepConst<R> &p, R &S, Draws &d
     if (first >= p.exp_m_lambda_dt) S *= jump_factor<R>(p, first, d);
 }
 
+// One step on the spot itself, with the pricing kernels' step code (the fed-draw trace).
 template <class R, int MODEL, int SCHEME, class Draws>
-__device__ __forceinline__ void evolve_step(const StepConst<R> &p, R &S, R &v, Draws &d) {
+__device__ __forceinline__ void evolve_step(const Tab64 *tab, const StepConst<R> &p, R &S, R &v, Draws &d) {
     R Z1, Z2;
     d.normal_pair(Z1, Z2);
-    heston_step<R, SCHEME>(p, S, v, Z1, Z2);
+    if constexpr (sizeof(R) == 4) {
+        heston_step_f32<SCHEME>(p, S, v, Z1, Z2);
+    } else {
+        Path64 s{0.0, 1.0, v};
+        step64<SCHEME>(p, s, Z1, Z2);
+        fold64<SCHEME>(*tab, s);
+        S *= exp2_64(*tab, s.x);
+        v = s.v;
+    }
     if constexpr (MODEL == kBates) bates_jump<R>(p, S, d);
 }
 

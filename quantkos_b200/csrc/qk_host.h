@@ -81,6 +81,19 @@ inline StepConst<R> make_step_const(const qk_contract &c, double dt, double eps)
     d.exp_m_lambda_dt = std::exp(-lambda_dt);
     d.mu_j = c.mu_j;
     d.sigma_j = c.sigma_j;
+    constexpr double kLog2e = 1.44269504088896340736;
+    d.l_drift = d.r_minus_q_dt * kLog2e;
+    d.l_half_dt = d.half_dt * kLog2e;
+    d.l_sqrt_dt = d.sqrt_dt * kLog2e;
+    d.l_K2 = d.K2 * kLog2e;
+    d.l_A = d.A * kLog2e;
+    d.l_c1 = -0.5 * d.K3 * kLog2e;  // K1 - (K1 + K3 / 2)
+    d.l_sqrt_K3 = std::sqrt(d.K3) * kLog2e;
+    d.h_f1 = 0.5 * d.s2f1;
+    d.h_f2 = 0.5 * d.s2f2;
+    d.h_psi = 0.5 * d.psi_c;
+    d.h_eps = 0.5 * d.eps;
+    d.two_A = 2.0 * d.A;
     if constexpr (sizeof(R) == sizeof(double)) {
         return d;
     } else {

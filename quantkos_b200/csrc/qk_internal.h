@@ -50,6 +50,10 @@ struct StepConst {
     R quarter_sigma_sq_dt, implicit_den;           // Milstein
     R eps, psi_c, inv_sqrt2, exp_mkdt, theta_m, s2f1, s2f2, K1, K2, K3, K4, A, K1_half_K3;  // QE
     R exp_m_lambda_dt, mu_j, sigma_j;              // Bates
+    // The steps on the base-2 logarithm of the spot: increments scaled by log2(e)
+    R l_drift, l_half_dt, l_sqrt_dt;               // (r - q) dt, dt / 2, sqrt(dt)
+    R l_K2, l_A, l_c1, l_sqrt_K3;                  // QE: K2, A, -K3 / 2 (the coefficient of v), sqrt(K3) (K3 = K4)
+    R h_f1, h_f2, h_psi, h_eps, two_A;             // QE: s^2 / 2 = v h_f1 + h_f2, psi_c / 2, eps / 2, 2 A
 };
 
 struct PayoffSpec {
@@ -76,6 +80,7 @@ struct TaskDev {
     uint32_t key0, key1;   // Philox key = seed
     uint32_t stream;       // Philox counter word 2 (common random numbers across bumps)
     uint32_t jump_kmin;    // FP32 jump test: a step jumps iff (first Poisson word >> 9) >= jump_kmin
+    uint32_t jump_kmin64;  // FP64: a first Poisson word below this cannot jump (exact test beyond it)
     int64_t n_paths;
     int64_t tile_begin;    // first queue slot of the task (tiles of a task are consecutive)
     int64_t partial_base;  // first per-tile moments record of the task

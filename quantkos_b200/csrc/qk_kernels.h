@@ -20,6 +20,13 @@ constexpr int kWarpTilePaths = 32;  // paths per round of a warp tile (one per l
 #endif
 constexpr int kPathMinBlocksFp32 = QK_PATH_MIN_BLOCKS_FP32;  // resident blocks per SM the FP32 path kernel is register-budgeted for
 
+// Resident 256-thread blocks per SM the FP64 path kernels are register-budgeted for: with
+// the one-path Euler kernel 2, 3 and 4 blocks measure 1287, 1291 and 1251 us
+// (1,048,576 x 252), with QE (12 pricings of 100,003 x 126, Asian) 2 and 3 blocks 2147 and
+// 2119 us: a few spilled registers against more warps to hide the FP64 latency.
+constexpr int kPathMinBlocks64 = 4;
+constexpr int kPathMinBlocksQe64 = 3;
+
 // uniform_key: every task of the launch has Philox key `seed` (round keys go in the
 // kernel parameters); otherwise each task's key is read from its descriptor.
 // lane_mode: what a lane simulates for every task of the launch (TaskDev::lane_mode).

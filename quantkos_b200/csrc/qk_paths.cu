@@ -13,7 +13,7 @@ namespace qk {
 // One path of one task.  Mirrors MarkovianIntegrationKernel::operator()
 // (include/core/schemes/markovian/MSolver.hpp:98-130): start at (S0, v0), step
 // n_steps times, track the running average / max / min after every step.
-// SINK is called after each step with (step index, S, v).
+// SINK is called after each step with (step index, S, v) (FP64: a function giving S).
 // ----------------------------------------------------------------------------
 template <class R>
 struct PathState {
@@ -23,8 +23,24 @@ struct PathState {
 };
 
 struct NoSink {
-    template <class R>
-    __device__ __forceinline__ void operator()(int, R, R) const {}
+    template <class S, class R>
+    __device__ __forceinline__ void operator()(int, S, R) const {}
+};
+
+// The FP64 functions' tables of a block (FP32 kernels hold none).
+template <class R>
+struct BlockTables {
+    Tab64 tab;
+    __device__ __forceinline__ void fill() {
+        fill_tab64(tab);
+        __syncthreads();
+    }
+    __device__ __forceinline__ const Tab64 *get() const { return &tab; }
+};
+template <>
+struct BlockTables<float> {
+    __device__ __forceinline__ void fill() {}
+    __device__ __forceinline__ const Tab64 *get() const { return nullptr; }
 };
 
 template <class R>
@@ -36,10 +52,12 @@ struct SlabSink {
     int stride;     // steps between stored dates
     int left;       // steps until the next stored date
     // Called once per step, in order: every stride-th step is stored.
-    __device__ __forceinline__ void operator()(int, R S, R v) {
+    template <class Spot>
+    __device__ __forceinline__ void operator()(int, Spot spot, R v) {
         if (--left == 0) {
             left = stride;
-            slab_S[pos] = S;
+            if constexpr (sizeof(R) == 8) slab_S[pos] = spot();
+            else slab_S[pos] = spot;
             if (slab_v) slab_v[pos] = v;
             pos += ld;
         }
@@ -111,119 +129,184 @@ __device__ __forceinline__ uint32_t poisson_hi_f32(uint32_t wa, uint32_t wb) {
     return ((wa & 0x1FFu) << 9) | (wb & 0x1FFu);
 }
 
-// pois: FP32 the 18 high bits (poisson_hi_f32), FP64 the full word.  On a jump,
-// `word` holds the full first-uniform word (top 23 bits k in FP32).
-template <class R>
-__device__ __forceinline__ bool jump_first(uint32_t pois, const StepConst<R> &p, uint32_t kmin, uint32_t k0,
-                                           uint32_t k1, uint32_t path, uint32_t stream, int n, uint32_t &word) {
-    if constexpr (sizeof(R) == 4) {
-        if (pois < (kmin >> 5)) return false;
-        const U4 q = philox4x32_10(U4{static_cast<uint32_t>(n >> 2), path, stream, 2u}, k0, k1);
-        const int j = n & 3;
-        const uint32_t w = j == 0 ? q.x : (j == 1 ? q.y : (j == 2 ? q.z : q.w));
-        word = ((pois << 5) | (w >> 27)) << 9;
-        return (word >> 9) >= kmin;
-    } else {
-        word = pois;
-        return Math<R>::u01(pois) >= p.exp_m_lambda_dt;
-    }
+// pois: the 18 high bits (poisson_hi_f32).  On a jump, `word` holds the full
+// first-uniform word (top 23 bits k).
+__device__ __forceinline__ bool jump_first_f32(uint32_t pois, uint32_t kmin, uint32_t k0, uint32_t k1, uint32_t path,
+                                               uint32_t stream, int n, uint32_t &word) {
+    if (pois < (kmin >> 5)) return false;
+    const U4 q = philox4x32_10(U4{static_cast<uint32_t>(n >> 2), path, stream, 2u}, k0, k1);
+    const int j = n & 3;
+    const uint32_t w = j == 0 ? q.x : (j == 1 ? q.y : (j == 2 ? q.z : q.w));
+    word = ((pois << 5) | (w >> 27)) << 9;
+    return (word >> 9) >= kmin;
 }
 
-// First-Poisson-uniform inputs of steps n and n+1 (n even): FP32 the high bits from
-// the normal block w of those steps; FP64 word n mod 4 of the domain-2 block wp
-// (fetched by the caller every fourth step).
-template <class R>
-__device__ __forceinline__ void poisson_words(const U4 &w, const U4 &wp, int n, uint32_t &p0, uint32_t &p1) {
-    if constexpr (sizeof(R) == 4) {
-        p0 = poisson_hi_f32(w.x, w.y);
-        p1 = poisson_hi_f32(w.z, w.w);
-    } else {
-        const bool lo = (n & 3) == 0;
-        p0 = lo ? wp.x : wp.z;
-        p1 = lo ? wp.y : wp.w;
-    }
-}
-
-template <class R, int MODEL, int SCHEME>
-__device__ __forceinline__ void one_step_z(const StepConst<R> &p, PathState<R> &st, R z1, R z2, uint32_t wpois,
-                                           uint32_t kmin, uint32_t k0, uint32_t k1, uint32_t path, uint32_t stream,
-                                           int n) {
-    heston_step<R, SCHEME>(p, st.S, st.v, z1, z2);
+template <int MODEL, int SCHEME>
+__device__ __forceinline__ void one_step_z(const StepConst<float> &p, PathState<float> &st, float z1, float z2,
+                                           uint32_t wpois, uint32_t kmin, uint32_t k0, uint32_t k1, uint32_t path,
+                                           uint32_t stream, int n) {
+    heston_step_f32<SCHEME>(p, st.S, st.v, z1, z2);
     if constexpr (MODEL == kBates) {
         uint32_t word;
-        if (jump_first<R>(wpois, p, kmin, k0, k1, path, stream, n, word)) {
-            PhiloxJumpDraws<R> d{k0, k1, path, stream, static_cast<uint32_t>(n), Math<R>::u01(word), 1, 0, U4{0, 0, 0, 0}};
-            st.S *= jump_factor<R>(p, d.first, d);
+        if (jump_first_f32(wpois, kmin, k0, k1, path, stream, n, word)) {
+            PhiloxJumpDraws<float> d{k0, k1, path, stream, static_cast<uint32_t>(n), Math<float>::u01(word), 1, 0, U4{0, 0, 0, 0}};
+            st.S *= jump_factor<float>(p, d.first, d);
         }
     }
 }
 
-template <class R, int MODEL, int SCHEME>
-__device__ __forceinline__ void one_step(const StepConst<R> &p, PathState<R> &st, uint32_t wa, uint32_t wb,
-                                         uint32_t wpois, uint32_t kmin, uint32_t k0, uint32_t k1, uint32_t path,
-                                         uint32_t stream, int n) {
-    R z1, z2;
-    Math<R>::box_muller(wa, wb, z1, z2);
-    one_step_z<R, MODEL, SCHEME>(p, st, z1, z2, wpois, kmin, k0, k1, path, stream, n);
+// FP64 jumps: log2 of the jump factor of a step whose first Poisson word reached the
+// threshold, with the jump normal as drawn (x) and negated (y, antithetic pairs); 0 if the
+// exact test finds no jump.  Arguments by value: nothing of the caller's state has to live
+// in memory for this rare call.
+__device__ __noinline__ double2 jump_log2_f64(uint32_t word, double L, double mu_j, double sigma_j, uint32_t k0,
+                                              uint32_t k1, uint32_t path, uint32_t stream, uint32_t n) {
+    double prod = Math<double>::u01(word);
+    if (!(prod >= L)) return make_double2(0.0, 0.0);
+    PhiloxJumpDraws<double> d{k0, k1, path, stream, n, prod, 1, 0, U4{0, 0, 0, 0}};
+    int N = 0;
+    do {
+        ++N;
+        prod *= d.uniform();
+    } while (prod >= L && N < kMaxJumpsPerStep);
+    const double Z = d.jump_normal();
+    const double m = N * mu_j, s = ::sqrt(static_cast<double>(N)) * sigma_j * Z;
+    return make_double2((m + s) * 1.44269504088896340736, (m - s) * 1.44269504088896340736);
+}
+
+// FP64 paths: NP paths of one lane (1; 2: an antithetic pair, NEG, or two independent
+// paths), stepped on the logarithm of the spot (step64).  Sums, maxima and minima are
+// those of S / S0; st holds the spot's on return.
+template <int MODEL, int SCHEME, bool TRK, int NP, bool NEG, class Gen, class Sink>
+__device__ __forceinline__ void simulate_f64(const Tab64 &tab, const StepConst<double> &p, double S0, double v0,
+                                             int n_steps, const Gen &gen, uint32_t k0, uint32_t k1, uint32_t path,
+                                             uint32_t stream, uint32_t kmin, PathState<double> (&st)[NP], Sink &&sink) {
+    Path64 s[NP];
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+        s[i] = Path64{0.0, 1.0, v0};
+        st[i].ssum = 0.0;
+        st[i].smax = st[i].smin = 1.0;
+    }
+    constexpr int ND = NEG ? 1 : NP;  // draw sequences
+    for (int n0 = 0; n0 < n_steps; n0 += kSumChunk) {
+        const int n1 = min(n0 + kSumChunk, n_steps);
+        double blk[NP];
+#pragma unroll
+        for (int i = 0; i < NP; ++i) blk[i] = 0.0;
+        U4 w[ND], wp[ND];
+        auto step = [&](int n, bool odd) {
+#pragma unroll
+            for (int i = 0; i < NP; ++i) {
+                const U4 &wi = w[NEG ? 0 : i];
+                double z1, z2;
+                box_muller64(tab, odd ? wi.z : wi.x, odd ? wi.w : wi.y, z1, z2);
+                if constexpr (NEG) {
+                    step64<SCHEME>(p, s[0], z1, z2);
+                    step64<SCHEME>(p, s[1], -z1, -z2);
+                    break;
+                } else {
+                    step64<SCHEME>(p, s[i], z1, z2);
+                }
+            }
+            if constexpr (MODEL == kBates) {
+#pragma unroll
+                for (int i = 0; i < ND; ++i) {
+                    // word n mod 4 of the domain-2 block
+                    const uint32_t word = (n & 2) ? (odd ? wp[i].w : wp[i].z) : (odd ? wp[i].y : wp[i].x);
+                    if (word >= kmin) {
+                        const double2 j = jump_log2_f64(word, p.exp_m_lambda_dt, p.mu_j, p.sigma_j, k0, k1, path + i,
+                                                        stream, static_cast<uint32_t>(n));
+                        s[i].x += j.x;
+                        if constexpr (NEG) s[1].x += j.y;
+                    }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < NP; ++i) {
+                if constexpr (TRK) {
+                    const double r = rel_spot64<SCHEME>(tab, s[i]);
+                    blk[i] += r;
+                    st[i].smax = r > st[i].smax ? r : st[i].smax;
+                    st[i].smin = r < st[i].smin ? r : st[i].smin;
+                }
+                sink(n, [&, i] { return S0 * rel_spot64<SCHEME>(tab, s[i]); }, s[i].v);
+            }
+        };
+        for (int n = n0; n < n1; n += 2) {
+#pragma unroll
+            for (int i = 0; i < ND; ++i) {
+                w[i] = gen(U4{static_cast<uint32_t>(n >> 1), path + i, stream, 0u});
+                if constexpr (MODEL == kBates) {
+                    if ((n & 3) == 0) wp[i] = gen(U4{static_cast<uint32_t>(n >> 2), path + i, stream, 2u});
+                }
+            }
+            step(n, false);
+            if (n + 1 < n1) step(n + 1, true);
+        }
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+            if constexpr (TRK) st[i].ssum += blk[i];
+            fold64<SCHEME>(tab, s[i]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+        st[i].S = S0 * exp2_64(tab, s[i].x);
+        st[i].v = s[i].v;
+        if constexpr (TRK) {
+            st[i].ssum *= S0;
+            st[i].smax *= S0;
+            st[i].smin *= S0;
+        } else {
+            st[i].smax = st[i].smin = st[i].S;
+        }
+    }
 }
 
 // TRK: keep the path state that Asian, barrier and lookback legs read (running sum,
 // max, min); false for launches whose legs read only the final spot.
 template <class R, int MODEL, int SCHEME, bool TRK = true, class Gen, class Sink>
-__device__ __forceinline__ void simulate_path(const StepConst<R> &p, R S0, R v0, int n_steps, const Gen &gen,
-                                              uint32_t k0, uint32_t k1, uint32_t path, uint32_t stream, uint32_t kmin,
-                                              PathState<R> &st, Sink &&sink) {
-    st.S = S0;
-    st.v = v0;
-    st.ssum = 0.0;
-    st.smax = S0;
-    st.smin = S0;
-    for (int n0 = 0; n0 < n_steps; n0 += kSumChunk) {
-        const int n1 = min(n0 + kSumChunk, n_steps);
-        R blk = R(0);
-        U4 wp{0u, 0u, 0u, 0u};  // Poisson words of steps 4m .. 4m+3 (n0 is a multiple of 4)
-        int n = n0;
-        for (; n + 1 < n1; n += 2) {
-            const U4 w = gen(U4{static_cast<uint32_t>(n >> 1), path, stream, 0u});
-            uint32_t pw0 = 0u, pw1 = 0u;
-            if constexpr (MODEL == kBates) {
-                if constexpr (sizeof(R) == 8) {
-                    if ((n & 3) == 0) wp = gen(U4{static_cast<uint32_t>(n >> 2), path, stream, 2u});
-                }
-                poisson_words<R>(w, wp, n, pw0, pw1);
-            }
-            if constexpr (sizeof(R) == 4) {
+__device__ __forceinline__ void simulate_path(const Tab64 *tab, const StepConst<R> &p, R S0, R v0, int n_steps,
+                                              const Gen &gen, uint32_t k0, uint32_t k1, uint32_t path, uint32_t stream,
+                                              uint32_t kmin, PathState<R> &st, Sink &&sink) {
+    if constexpr (sizeof(R) == 8) {
+        PathState<double> one[1];
+        simulate_f64<MODEL, SCHEME, TRK, 1, false>(*tab, p, S0, v0, n_steps, gen, k0, k1, path, stream, kmin, one, sink);
+        st = one[0];
+    } else {
+        st.S = S0;
+        st.v = v0;
+        st.ssum = 0.0;
+        st.smax = S0;
+        st.smin = S0;
+        for (int n0 = 0; n0 < n_steps; n0 += kSumChunk) {
+            const int n1 = min(n0 + kSumChunk, n_steps);
+            R blk = R(0);
+            int n = n0;
+            for (; n + 1 < n1; n += 2) {
+                const U4 w = gen(U4{static_cast<uint32_t>(n >> 1), path, stream, 0u});
                 // the normals of both steps (independent of the path state) in one paired
                 // Box-Muller; the same bits as two one-pair calls
                 float2 Z1, Z2;
                 Math<float>::box_muller_two(w.x, w.y, w.z, w.w, Z1, Z2);
-                one_step_z<R, MODEL, SCHEME>(p, st, Z1.x, Z2.x, pw0, kmin, k0, k1, path, stream, n);
+                one_step_z<MODEL, SCHEME>(p, st, Z1.x, Z2.x, poisson_hi_f32(w.x, w.y), kmin, k0, k1, path, stream, n);
                 if constexpr (TRK) track(st, blk);
                 sink(n, st.S, st.v);
-                one_step_z<R, MODEL, SCHEME>(p, st, Z1.y, Z2.y, pw1, kmin, k0, k1, path, stream, n + 1);
-            } else {
-                one_step<R, MODEL, SCHEME>(p, st, w.x, w.y, pw0, kmin, k0, k1, path, stream, n);
+                one_step_z<MODEL, SCHEME>(p, st, Z1.y, Z2.y, poisson_hi_f32(w.z, w.w), kmin, k0, k1, path, stream, n + 1);
+                if constexpr (TRK) track(st, blk);
+                sink(n + 1, st.S, st.v);
+            }
+            if (n < n1) {
+                const U4 w = gen(U4{static_cast<uint32_t>(n >> 1), path, stream, 0u});
+                float z1, z2;
+                Math<float>::box_muller(w.x, w.y, z1, z2);
+                one_step_z<MODEL, SCHEME>(p, st, z1, z2, poisson_hi_f32(w.x, w.y), kmin, k0, k1, path, stream, n);
                 if constexpr (TRK) track(st, blk);
                 sink(n, st.S, st.v);
-                one_step<R, MODEL, SCHEME>(p, st, w.z, w.w, pw1, kmin, k0, k1, path, stream, n + 1);
             }
-            if constexpr (TRK) track(st, blk);
-            sink(n + 1, st.S, st.v);
+            if constexpr (TRK) st.ssum += static_cast<double>(blk);
         }
-        if (n < n1) {
-            const U4 w = gen(U4{static_cast<uint32_t>(n >> 1), path, stream, 0u});
-            uint32_t pw0 = 0u, pw1 = 0u;
-            if constexpr (MODEL == kBates) {
-                if constexpr (sizeof(R) == 8) {
-                    if ((n & 3) == 0) wp = gen(U4{static_cast<uint32_t>(n >> 2), path, stream, 2u});
-                }
-                poisson_words<R>(w, wp, n, pw0, pw1);
-            }
-            one_step<R, MODEL, SCHEME>(p, st, w.x, w.y, pw0, kmin, k0, k1, path, stream, n);
-            if constexpr (TRK) track(st, blk);
-            sink(n, st.S, st.v);
-        }
-        if constexpr (TRK) st.ssum += static_cast<double>(blk);
     }
 }
 
@@ -246,23 +329,23 @@ __device__ __forceinline__ void normals_two_f32(uint32_t wa1, uint32_t wa2, uint
     }
 }
 
-// Bates jumps of both paths of a lane after their Heston step.
-template <class R, int MODEL, bool NEG>
-__device__ __forceinline__ void jumps_two(const StepConst<R> &p, PathState<R> &a, PathState<R> &b, uint32_t pois_a,
-                                          uint32_t pois_b, uint32_t kmin, uint32_t k0, uint32_t k1, uint32_t path_a,
-                                          uint32_t path_b, uint32_t stream, int n) {
+// Bates jumps of both paths of a lane after their Heston step (FP32).
+template <int MODEL, bool NEG>
+__device__ __forceinline__ void jumps_two(const StepConst<float> &p, PathState<float> &a, PathState<float> &b,
+                                          uint32_t pois_a, uint32_t pois_b, uint32_t kmin, uint32_t k0, uint32_t k1,
+                                          uint32_t path_a, uint32_t path_b, uint32_t stream, int n) {
     if constexpr (MODEL == kBates) {
         uint32_t word;
         if constexpr (NEG) {
-            if (jump_first<R>(pois_a, p, kmin, k0, k1, path_a, stream, n, word)) {
-                PhiloxJumpDraws<R> d{k0, k1, path_a, stream, static_cast<uint32_t>(n), Math<R>::u01(word), 1, 0,
-                                     U4{0, 0, 0, 0}};
-                R fa, fb;
-                jump_factor_pair<R>(p, d.first, d, fa, fb);
+            if (jump_first_f32(pois_a, kmin, k0, k1, path_a, stream, n, word)) {
+                PhiloxJumpDraws<float> d{k0, k1, path_a, stream, static_cast<uint32_t>(n), Math<float>::u01(word), 1, 0,
+                                         U4{0, 0, 0, 0}};
+                float fa, fb;
+                jump_factor_pair<float>(p, d.first, d, fa, fb);
                 a.S *= fa;
                 b.S *= fb;
             }
-        } else if constexpr (sizeof(R) == 4) {
+        } else {
             // the one-compare tests of both paths inline; one copy of the rest of the
             // jump code for both (rare; keeps the loop body small)
             const uint32_t kmin_hi = kmin >> 5;
@@ -270,25 +353,14 @@ __device__ __forceinline__ void jumps_two(const StepConst<R> &p, PathState<R> &a
 #pragma unroll 1
                 for (int i = 0; i < 2; ++i) {
                     const uint32_t pois = i ? pois_b : pois_a, path = i ? path_b : path_a;
-                    if (jump_first<R>(pois, p, kmin, k0, k1, path, stream, n, word)) {
-                        PhiloxJumpDraws<R> d{k0, k1, path, stream, static_cast<uint32_t>(n), Math<R>::u01(word), 1, 0,
-                                             U4{0, 0, 0, 0}};
-                        const R f = jump_factor<R>(p, d.first, d);
+                    if (jump_first_f32(pois, kmin, k0, k1, path, stream, n, word)) {
+                        PhiloxJumpDraws<float> d{k0, k1, path, stream, static_cast<uint32_t>(n), Math<float>::u01(word), 1,
+                                                 0, U4{0, 0, 0, 0}};
+                        const float f = jump_factor<float>(p, d.first, d);
                         if (i) b.S *= f;
                         else a.S *= f;
                     }
                 }
-            }
-        } else {
-            if (jump_first<R>(pois_a, p, kmin, k0, k1, path_a, stream, n, word)) {
-                PhiloxJumpDraws<R> d{k0, k1, path_a, stream, static_cast<uint32_t>(n), Math<R>::u01(word), 1, 0,
-                                     U4{0, 0, 0, 0}};
-                a.S *= jump_factor<R>(p, d.first, d);
-            }
-            if (jump_first<R>(pois_b, p, kmin, k0, k1, path_b, stream, n, word)) {
-                PhiloxJumpDraws<R> d{k0, k1, path_b, stream, static_cast<uint32_t>(n), Math<R>::u01(word), 1, 0,
-                                     U4{0, 0, 0, 0}};
-                b.S *= jump_factor<R>(p, d.first, d);
             }
         }
     }
@@ -309,41 +381,17 @@ __device__ __forceinline__ void step_two_z_f32(const StepConst<float> &p, PathSt
     b.S = S2.y;
     a.v = v2.x;
     b.v = v2.y;
-    jumps_two<float, MODEL, NEG>(p, a, b, pois_a, pois_b, kmin, k0, k1, path_a, path_b, stream, n);
-}
-
-template <class R, int MODEL, int SCHEME, bool NEG>
-__device__ __forceinline__ void one_step_two(const StepConst<R> &p, PathState<R> &a, PathState<R> &b, uint32_t wa1,
-                                             uint32_t wa2, uint32_t wb1, uint32_t wb2, uint32_t pois_a,
-                                             uint32_t pois_b, uint32_t kmin, uint32_t k0, uint32_t k1, uint32_t path_a,
-                                             uint32_t path_b, uint32_t stream, int n) {
-    if constexpr (sizeof(R) == 4) {
-        float2 Z1, Z2;
-        normals_two_f32<NEG>(wa1, wa2, wb1, wb2, Z1, Z2);
-        step_two_z_f32<MODEL, SCHEME, NEG>(p, a, b, Z1, Z2, pois_a, pois_b, kmin, k0, k1, path_a, path_b, stream, n);
-    } else {
-        R za1, za2, zb1, zb2;
-        Math<R>::box_muller(wa1, wa2, za1, za2);
-        if constexpr (NEG) {
-            zb1 = -za1;
-            zb2 = -za2;
-        } else {
-            Math<R>::box_muller(wb1, wb2, zb1, zb2);
-        }
-        heston_step<R, SCHEME>(p, a.S, a.v, za1, za2);
-        heston_step<R, SCHEME>(p, b.S, b.v, zb1, zb2);
-        jumps_two<R, MODEL, NEG>(p, a, b, pois_a, pois_b, kmin, k0, k1, path_a, path_b, stream, n);
-    }
+    jumps_two<MODEL, NEG>(p, a, b, pois_a, pois_b, kmin, k0, k1, path_a, path_b, stream, n);
 }
 
 // ssum_slot: where the two paths' Asian running sums (x: path a, y: path b) are kept
 // between the 16-step blocks that add to them: this thread's shared-memory slot (two
 // FP64 sums read and written once per block, four registers fewer in the step loop),
 // or nullptr for a.ssum and b.ssum.
-template <class R, int MODEL, int SCHEME, bool NEG, bool TRK = true, class Gen, class Sink2>
-__device__ __forceinline__ void simulate_two(const StepConst<R> &p, R S0, R v0, int n_steps, const Gen &gen,
+template <int MODEL, int SCHEME, bool NEG, bool TRK = true, class Gen, class Sink2>
+__device__ __forceinline__ void simulate_two(const StepConst<float> &p, float S0, float v0, int n_steps, const Gen &gen,
                                              uint32_t k0, uint32_t k1, uint32_t path_a, uint32_t path_b,
-                                             uint32_t stream, uint32_t kmin, PathState<R> &a, PathState<R> &b,
+                                             uint32_t stream, uint32_t kmin, PathState<float> &a, PathState<float> &b,
                                              Sink2 &&sink, double2 *ssum_slot = nullptr) {
     a.S = b.S = S0;
     a.v = b.v = v0;
@@ -353,46 +401,26 @@ __device__ __forceinline__ void simulate_two(const StepConst<R> &p, R S0, R v0, 
     a.smin = b.smin = S0;
     for (int n0 = 0; n0 < n_steps; n0 += kSumChunk) {
         const int n1 = min(n0 + kSumChunk, n_steps);
-        R blk_a = R(0), blk_b = R(0);
-        U4 pa{0u, 0u, 0u, 0u}, pb{0u, 0u, 0u, 0u};
+        float blk_a = 0.0f, blk_b = 0.0f;
         int n = n0;
         for (; n + 1 < n1; n += 2) {
             const U4 wa = gen(U4{static_cast<uint32_t>(n >> 1), path_a, stream, 0u});
             U4 wb{0u, 0u, 0u, 0u};
             if constexpr (!NEG) wb = gen(U4{static_cast<uint32_t>(n >> 1), path_b, stream, 0u});
-            uint32_t qa0 = 0u, qa1 = 0u, qb0 = 0u, qb1 = 0u;
-            if constexpr (MODEL == kBates) {
-                if constexpr (sizeof(R) == 8) {
-                    if ((n & 3) == 0) {
-                        pa = gen(U4{static_cast<uint32_t>(n >> 2), path_a, stream, 2u});
-                        if constexpr (!NEG) pb = gen(U4{static_cast<uint32_t>(n >> 2), path_b, stream, 2u});
-                    }
-                }
-                poisson_words<R>(wa, pa, n, qa0, qa1);
-                if constexpr (!NEG) poisson_words<R>(wb, pb, n, qb0, qb1);
-            }
-            if constexpr (sizeof(R) == 4 && SCHEME != kQE) {
-                // Euler and Milstein: both steps' normals first, so that the second step's
-                // Box-Muller (independent of the first step) overlaps the first step's work
-                // (QE, whose step holds more live values, measures faster without it)
-                float2 Z1a, Z2a, Z1b, Z2b;
-                normals_two_f32<NEG>(wa.x, wa.y, wb.x, wb.y, Z1a, Z2a);
-                normals_two_f32<NEG>(wa.z, wa.w, wb.z, wb.w, Z1b, Z2b);
-                step_two_z_f32<MODEL, SCHEME, NEG>(p, a, b, Z1a, Z2a, qa0, qb0, kmin, k0, k1, path_a, path_b, stream, n);
-                if constexpr (TRK) track(a, blk_a);
-                if constexpr (TRK) track(b, blk_b);
-                sink(n, a.S, a.v, b.S, b.v);
-                step_two_z_f32<MODEL, SCHEME, NEG>(p, a, b, Z1b, Z2b, qa1, qb1, kmin, k0, k1, path_a, path_b, stream,
-                                                   n + 1);
-            } else {
-            one_step_two<R, MODEL, SCHEME, NEG>(p, a, b, wa.x, wa.y, wb.x, wb.y, qa0, qb0, kmin, k0, k1, path_a,
-                                                path_b, stream, n);
+            const uint32_t qa0 = poisson_hi_f32(wa.x, wa.y), qa1 = poisson_hi_f32(wa.z, wa.w);
+            const uint32_t qb0 = poisson_hi_f32(wb.x, wb.y), qb1 = poisson_hi_f32(wb.z, wb.w);
+            float2 Z1a, Z2a, Z1b, Z2b;
+            normals_two_f32<NEG>(wa.x, wa.y, wb.x, wb.y, Z1a, Z2a);
+            // Euler and Milstein: both steps' normals first, so that the second step's
+            // Box-Muller (independent of the first step) overlaps the first step's work
+            // (QE, whose step holds more live values, measures faster without it)
+            if constexpr (SCHEME != kQE) normals_two_f32<NEG>(wa.z, wa.w, wb.z, wb.w, Z1b, Z2b);
+            step_two_z_f32<MODEL, SCHEME, NEG>(p, a, b, Z1a, Z2a, qa0, qb0, kmin, k0, k1, path_a, path_b, stream, n);
             if constexpr (TRK) track(a, blk_a);
             if constexpr (TRK) track(b, blk_b);
             sink(n, a.S, a.v, b.S, b.v);
-            one_step_two<R, MODEL, SCHEME, NEG>(p, a, b, wa.z, wa.w, wb.z, wb.w, qa1, qb1, kmin, k0, k1, path_a,
-                                                path_b, stream, n + 1);
-            }
+            if constexpr (SCHEME == kQE) normals_two_f32<NEG>(wa.z, wa.w, wb.z, wb.w, Z1b, Z2b);
+            step_two_z_f32<MODEL, SCHEME, NEG>(p, a, b, Z1b, Z2b, qa1, qb1, kmin, k0, k1, path_a, path_b, stream, n + 1);
             if constexpr (TRK) track(a, blk_a);
             if constexpr (TRK) track(b, blk_b);
             sink(n + 1, a.S, a.v, b.S, b.v);
@@ -401,19 +429,10 @@ __device__ __forceinline__ void simulate_two(const StepConst<R> &p, R S0, R v0, 
             const U4 wa = gen(U4{static_cast<uint32_t>(n >> 1), path_a, stream, 0u});
             U4 wb{0u, 0u, 0u, 0u};
             if constexpr (!NEG) wb = gen(U4{static_cast<uint32_t>(n >> 1), path_b, stream, 0u});
-            uint32_t qa0 = 0u, qa1 = 0u, qb0 = 0u, qb1 = 0u;
-            if constexpr (MODEL == kBates) {
-                if constexpr (sizeof(R) == 8) {
-                    if ((n & 3) == 0) {
-                        pa = gen(U4{static_cast<uint32_t>(n >> 2), path_a, stream, 2u});
-                        if constexpr (!NEG) pb = gen(U4{static_cast<uint32_t>(n >> 2), path_b, stream, 2u});
-                    }
-                }
-                poisson_words<R>(wa, pa, n, qa0, qa1);
-                if constexpr (!NEG) poisson_words<R>(wb, pb, n, qb0, qb1);
-            }
-            one_step_two<R, MODEL, SCHEME, NEG>(p, a, b, wa.x, wa.y, wb.x, wb.y, qa0, qb0, kmin, k0, k1, path_a,
-                                                path_b, stream, n);
+            float2 Z1, Z2;
+            normals_two_f32<NEG>(wa.x, wa.y, wb.x, wb.y, Z1, Z2);
+            const uint32_t qa0 = poisson_hi_f32(wa.x, wa.y), qb0 = poisson_hi_f32(wb.x, wb.y);
+            step_two_z_f32<MODEL, SCHEME, NEG>(p, a, b, Z1, Z2, qa0, qb0, kmin, k0, k1, path_a, path_b, stream, n);
             if constexpr (TRK) track(a, blk_a);
             if constexpr (TRK) track(b, blk_b);
             sink(n, a.S, a.v, b.S, b.v);
@@ -443,20 +462,26 @@ __device__ __forceinline__ const StepConst<float> &task_const<float>(const TaskD
 template <>
 __device__ __forceinline__ const StepConst<double> &task_const<double>(const TaskDev &t) { return t.cd; }
 
+// The raw-word jump threshold of the precision.
+template <class R>
+__device__ __forceinline__ uint32_t task_kmin(const TaskDev &t) {
+    return sizeof(R) == 4 ? t.jump_kmin : t.jump_kmin64;
+}
+
 template <class R, class Sink>
-__device__ __forceinline__ void simulate_dispatch(const TaskDev &t, const StepConst<R> &p, uint32_t path,
-                                                  PathState<R> &st, Sink &&sink) {
+__device__ __forceinline__ void simulate_dispatch(const Tab64 *tab, const TaskDev &t, const StepConst<R> &p,
+                                                  uint32_t path, PathState<R> &st, Sink &&sink) {
     const R S0 = static_cast<R>(t.S0);
     const R v0 = static_cast<R>(t.v0);
-    const uint32_t km = t.jump_kmin;
+    const uint32_t km = task_kmin<R>(t);
     const RegKeys g{t.key0, t.key1};
     switch (t.model * 3 + t.scheme) {
-        case 0: simulate_path<R, kHeston, kEuler>(p, S0, v0, t.n_steps, g, t.key0, t.key1, path, t.stream, km, st, sink); break;
-        case 1: simulate_path<R, kHeston, kMilstein>(p, S0, v0, t.n_steps, g, t.key0, t.key1, path, t.stream, km, st, sink); break;
-        case 2: simulate_path<R, kHeston, kQE>(p, S0, v0, t.n_steps, g, t.key0, t.key1, path, t.stream, km, st, sink); break;
-        case 3: simulate_path<R, kBates, kEuler>(p, S0, v0, t.n_steps, g, t.key0, t.key1, path, t.stream, km, st, sink); break;
-        case 4: simulate_path<R, kBates, kMilstein>(p, S0, v0, t.n_steps, g, t.key0, t.key1, path, t.stream, km, st, sink); break;
-        default: simulate_path<R, kBates, kQE>(p, S0, v0, t.n_steps, g, t.key0, t.key1, path, t.stream, km, st, sink); break;
+        case 0: simulate_path<R, kHeston, kEuler>(tab, p, S0, v0, t.n_steps, g, t.key0, t.key1, path, t.stream, km, st, sink); break;
+        case 1: simulate_path<R, kHeston, kMilstein>(tab, p, S0, v0, t.n_steps, g, t.key0, t.key1, path, t.stream, km, st, sink); break;
+        case 2: simulate_path<R, kHeston, kQE>(tab, p, S0, v0, t.n_steps, g, t.key0, t.key1, path, t.stream, km, st, sink); break;
+        case 3: simulate_path<R, kBates, kEuler>(tab, p, S0, v0, t.n_steps, g, t.key0, t.key1, path, t.stream, km, st, sink); break;
+        case 4: simulate_path<R, kBates, kMilstein>(tab, p, S0, v0, t.n_steps, g, t.key0, t.key1, path, t.stream, km, st, sink); break;
+        default: simulate_path<R, kBates, kQE>(tab, p, S0, v0, t.n_steps, g, t.key0, t.key1, path, t.stream, km, st, sink); break;
     }
 }
 
@@ -485,7 +510,8 @@ __device__ __forceinline__ int find_task(const int64_t *__restrict__ prefix, int
 // set for kPathMinBlocksFp32 resident 256-thread blocks per SM (64 registers a thread).
 template <class R, int MODEL, int SCHEME, bool UK, int LANE, bool TRK>
 __global__ void __launch_bounds__(path_block_max<R>(),
-                                  sizeof(R) == 4 ? kPathMinBlocksFp32 * kPathBlock / path_block_max<R>() : 1)
+                                  sizeof(R) == 4 ? kPathMinBlocksFp32 * kPathBlock / path_block_max<R>()
+                                                 : (SCHEME == kQE ? kPathMinBlocksQe64 : kPathMinBlocks64))
     price_tiles_kernel(const TaskDev *__restrict__ tasks, const int64_t *__restrict__ prefix, int32_t n_tasks,
                        int64_t slot_begin, int64_t slot_end, unsigned long long *__restrict__ cursor,
                        Moments *__restrict__ partials, const PhiloxRoundKeys rk) {
@@ -495,12 +521,14 @@ __global__ void __launch_bounds__(path_block_max<R>(),
     __shared__ Moments s_acc[path_block_max<R>() / 32][QK_MAX_PAYOFFS];
     // the Asian running sums of a lane's two independent paths (simulate_two); one slot per
     // thread (antithetic pairs keep theirs in registers, which measures faster there)
-    constexpr bool kSumSlot = LANE == kLaneTwo && TRK;
+    constexpr bool kSumSlot = sizeof(R) == 4 && LANE == kLaneTwo && TRK;
     __shared__ double2 s_ssum[kSumSlot ? path_block_max<R>() : 1];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const R eps_payoff = sizeof(R) == 4 ? R(1e-6) : R(1e-12);  // OptionPricer.hpp:316
     Moments *acc = s_acc[warp];
+    __shared__ BlockTables<R> tables;
+    tables.fill();
 
     for (;;) {
         long long q = 0;
@@ -515,7 +543,7 @@ __global__ void __launch_bounds__(path_block_max<R>(),
         const int np = t.n_payoffs;
         const int n_steps = t.n_steps;
         const int64_t n_paths = t.n_paths;
-        const uint32_t k0 = t.key0, k1 = t.key1, stream = t.stream, kmin = t.jump_kmin;
+        const uint32_t k0 = t.key0, k1 = t.key1, stream = t.stream, kmin = task_kmin<R>(t);
         const R S0 = static_cast<R>(t.S0), v0 = static_cast<R>(t.v0);
         // big tiles of ppt rounds, then the tail in tiles of ppt_tail rounds
         const bool big = tile < t.n_big;
@@ -541,13 +569,21 @@ __global__ void __launch_bounds__(path_block_max<R>(),
                 const bool active_b = NEG ? active : (active && static_cast<int64_t>(pb) < n_paths);
                 PathState<R> sa, sb;
                 if (active) {
-                    if constexpr (UK) {
-                        simulate_two<R, MODEL, SCHEME, NEG, TRK>(p, S0, v0, n_steps, ParamKeys{rk}, k0, k1, pa, pb, stream,
-                                                            kmin, sa, sb, NoSink2{}, kSumSlot ? &s_ssum[threadIdx.x] : nullptr);
-                    } else {
-                        simulate_two<R, MODEL, SCHEME, NEG, TRK>(p, S0, v0, n_steps, RegKeys{k0, k1}, k0, k1, pa, pb,
-                                                            stream, kmin, sa, sb, NoSink2{}, kSumSlot ? &s_ssum[threadIdx.x] : nullptr);
-                    }
+                    const auto simulate = [&](const auto &gen) {
+                        if constexpr (sizeof(R) == 8) {
+                            PathState<double> two[2];
+                            simulate_f64<MODEL, SCHEME, TRK, 2, NEG>(*tables.get(), p, S0, v0, n_steps, gen, k0, k1, pa,
+                                                                     stream, kmin, two, NoSink{});
+                            sa = two[0];
+                            sb = two[1];
+                        } else {
+                            simulate_two<MODEL, SCHEME, NEG, TRK>(p, S0, v0, n_steps, gen, k0, k1, pa, pb, stream, kmin,
+                                                                  sa, sb, NoSink2{},
+                                                                  kSumSlot ? &s_ssum[threadIdx.x] : nullptr);
+                        }
+                    };
+                    if constexpr (UK) simulate(ParamKeys{rk});
+                    else simulate(RegKeys{k0, k1});
                 } else {
                     sa.S = sa.smax = sa.smin = sb.S = sb.smax = sb.smin = R(0);
                     sa.ssum = sb.ssum = 0.0;
@@ -570,10 +606,10 @@ __global__ void __launch_bounds__(path_block_max<R>(),
                 PathState<R> st;
                 if (active) {
                     if constexpr (UK) {
-                        simulate_path<R, MODEL, SCHEME, TRK>(p, S0, v0, n_steps, ParamKeys{rk}, k0, k1,
+                        simulate_path<R, MODEL, SCHEME, TRK>(tables.get(), p, S0, v0, n_steps, ParamKeys{rk}, k0, k1,
                                                         static_cast<uint32_t>(unit), stream, kmin, st, NoSink{});
                     } else {
-                        simulate_path<R, MODEL, SCHEME, TRK>(p, S0, v0, n_steps, RegKeys{k0, k1}, k0, k1,
+                        simulate_path<R, MODEL, SCHEME, TRK>(tables.get(), p, S0, v0, n_steps, RegKeys{k0, k1}, k0, k1,
                                                         static_cast<uint32_t>(unit), stream, kmin, st, NoSink{});
                     }
                 } else {
@@ -753,56 +789,62 @@ __global__ void __launch_bounds__(128) merge_task_chunks_kernel(const TaskDev *_
     }
 }
 
-// Exercise-date slabs (LSM) / full path dump: one path per thread (a two-path
+// Exercise-date slabs (LSM) / full path dump: one path per thread (a two-path FP32
 // variant follows), S (and v)
 // after every `stride`-th step stored as SoA rows slab[date][path] (coalesced:
 // consecutive threads write consecutive columns).  Specialised per kind, with the
-// Philox round keys in the kernel parameters.
+// Philox round keys in the kernel parameters.  FP64: grid-stride over the paths, so that
+// a block's function tables are filled once.
 template <class R, int MODEL, int SCHEME>
 __global__ void __launch_bounds__(kPathBlock) slab_paths_kernel(const TaskDev *__restrict__ task, int64_t first_path,
                                                                int64_t count, int stride, R *__restrict__ slab_S,
                                                                R *__restrict__ slab_v, int64_t ld,
                                                                const PhiloxRoundKeys rk) {
-    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= count) return;
+    __shared__ BlockTables<R> tables;
+    tables.fill();
     const TaskDev &t = *task;
     const StepConst<R> p = task_const<R>(t);
-    SlabSink<R> sink{slab_S, slab_v, ld, i, stride, stride};
-    PathState<R> st;
-    simulate_path<R, MODEL, SCHEME>(p, static_cast<R>(t.S0), static_cast<R>(t.v0), t.n_steps, ParamKeys{rk}, t.key0,
-                                    t.key1, static_cast<uint32_t>(first_path + i), t.stream, t.jump_kmin, st, sink);
+    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < count;
+         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        SlabSink<R> sink{slab_S, slab_v, ld, i, stride, stride};
+        PathState<R> st;
+        simulate_path<R, MODEL, SCHEME, false>(tables.get(), p, static_cast<R>(t.S0), static_cast<R>(t.v0), t.n_steps,
+                                               ParamKeys{rk}, t.key0, t.key1, static_cast<uint32_t>(first_path + i),
+                                               t.stream, task_kmin<R>(t), st, sink);
+    }
 }
 
-// Two paths per thread (first + 2i and first + 2i + 1), interleaved and, in FP32,
-// stepped as pairs; same values as the one-path kernel.
-template <class R, int MODEL, int SCHEME>
+// FP32, two paths per thread (first + 2i and first + 2i + 1), interleaved and stepped as
+// pairs; same values as the one-path kernel.
+template <int MODEL, int SCHEME>
 __global__ void __launch_bounds__(kPathBlock) slab_paths_two_kernel(const TaskDev *__restrict__ task,
                                                                    int64_t first_path, int64_t count, int stride,
-                                                                   R *__restrict__ slab_S, R *__restrict__ slab_v,
-                                                                   int64_t ld, const PhiloxRoundKeys rk) {
+                                                                   float *__restrict__ slab_S,
+                                                                   float *__restrict__ slab_v, int64_t ld,
+                                                                   const PhiloxRoundKeys rk) {
     const int64_t i = 2 * (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x);
     if (i >= count) return;
     const TaskDev &t = *task;
-    const StepConst<R> p = task_const<R>(t);
-    SlabSink2<R> sink{slab_S, slab_v, ld, i, stride, stride, i + 1 < count};
-    PathState<R> sa, sb;
+    const StepConst<float> p = task_const<float>(t);
+    SlabSink2<float> sink{slab_S, slab_v, ld, i, stride, stride, i + 1 < count};
+    PathState<float> sa, sb;
     const uint32_t pa = static_cast<uint32_t>(first_path + i);
-    simulate_two<R, MODEL, SCHEME, false>(p, static_cast<R>(t.S0), static_cast<R>(t.v0), t.n_steps, ParamKeys{rk},
-                                          t.key0, t.key1, pa, pa + 1u, t.stream, t.jump_kmin, sa, sb, sink);
+    simulate_two<MODEL, SCHEME, false, false>(p, static_cast<float>(t.S0), static_cast<float>(t.v0), t.n_steps,
+                                              ParamKeys{rk}, t.key0, t.key1, pa, pa + 1u, t.stream, t.jump_kmin, sa, sb,
+                                              sink);
 }
 
 template <class R>
 using SlabKernel = void (*)(const TaskDev *, int64_t, int64_t, int, R *, R *, int64_t, const PhiloxRoundKeys);
 
-template <class R>
-SlabKernel<R> slab_two_kernel_for(int model, int scheme) {
+SlabKernel<float> slab_two_kernel_for(int model, int scheme) {
     switch (model * 3 + scheme) {
-        case 0: return slab_paths_two_kernel<R, kHeston, kEuler>;
-        case 1: return slab_paths_two_kernel<R, kHeston, kMilstein>;
-        case 2: return slab_paths_two_kernel<R, kHeston, kQE>;
-        case 3: return slab_paths_two_kernel<R, kBates, kEuler>;
-        case 4: return slab_paths_two_kernel<R, kBates, kMilstein>;
-        default: return slab_paths_two_kernel<R, kBates, kQE>;
+        case 0: return slab_paths_two_kernel<kHeston, kEuler>;
+        case 1: return slab_paths_two_kernel<kHeston, kMilstein>;
+        case 2: return slab_paths_two_kernel<kHeston, kQE>;
+        case 3: return slab_paths_two_kernel<kBates, kEuler>;
+        case 4: return slab_paths_two_kernel<kBates, kMilstein>;
+        default: return slab_paths_two_kernel<kBates, kQE>;
     }
 }
 
@@ -823,13 +865,16 @@ SlabKernel<R> slab_kernel_for(int model, int scheme) {
 template <class R>
 __global__ void __launch_bounds__(kPathBlock) payoff_paths_kernel(const TaskDev *__restrict__ task, int64_t first,
                                                                  int64_t count, double *__restrict__ out) {
-    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= count) return;
+    __shared__ BlockTables<R> tables;
+    tables.fill();
     const TaskDev &t = *task;
     const StepConst<R> p = task_const<R>(t);
-    PathState<R> st;
-    simulate_dispatch<R>(t, p, static_cast<uint32_t>(first + i), st, NoSink{});
-    out[i] = static_cast<double>(final_payoff<R>(t.pay[0], st.S, st.ssum, st.smax, st.smin, t.n_steps));
+    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < count;
+         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        PathState<R> st;
+        simulate_dispatch<R>(tables.get(), t, p, static_cast<uint32_t>(first + i), st, NoSink{});
+        out[i] = static_cast<double>(final_payoff<R>(t.pay[0], st.S, st.ssum, st.smax, st.smin, t.n_steps));
+    }
 }
 
 // Payoff of one leg on a fed spot sequence S_1..S_n (one thread): the path kernel's
@@ -858,11 +903,13 @@ __global__ void payoff_trace_kernel(const PayoffSpec ps, const double *__restric
     *out = static_cast<double>(final_payoff<R>(ps, st.S, st.ssum, st.smax, st.smin, n));
 }
 
-// Fed-draw trace of the step functions (one thread).
+// Fed-draw trace of the step functions (one thread steps; the block fills the tables).
 template <class R>
 __global__ void step_trace_kernel(const TaskDev *__restrict__ task, const double *__restrict__ z,
                                   const double *__restrict__ u, int umax, int n, double *__restrict__ S_out,
                                   double *__restrict__ v_out, int *__restrict__ status) {
+    __shared__ BlockTables<R> tables;
+    tables.fill();
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
     const TaskDev &t = *task;
     const StepConst<R> p = task_const<R>(t);
@@ -871,12 +918,12 @@ __global__ void step_trace_kernel(const TaskDev *__restrict__ task, const double
     for (int i = 0; i < n; ++i) {
         FedStep<R> d{z + 3 * static_cast<int64_t>(i), u + static_cast<int64_t>(umax) * i, umax, 0, 0};
         switch (t.model * 3 + t.scheme) {
-            case 0: evolve_step<R, kHeston, kEuler>(p, S, v, d); break;
-            case 1: evolve_step<R, kHeston, kMilstein>(p, S, v, d); break;
-            case 2: evolve_step<R, kHeston, kQE>(p, S, v, d); break;
-            case 3: evolve_step<R, kBates, kEuler>(p, S, v, d); break;
-            case 4: evolve_step<R, kBates, kMilstein>(p, S, v, d); break;
-            default: evolve_step<R, kBates, kQE>(p, S, v, d); break;
+            case 0: evolve_step<R, kHeston, kEuler>(tables.get(), p, S, v, d); break;
+            case 1: evolve_step<R, kHeston, kMilstein>(tables.get(), p, S, v, d); break;
+            case 2: evolve_step<R, kHeston, kQE>(tables.get(), p, S, v, d); break;
+            case 3: evolve_step<R, kBates, kEuler>(tables.get(), p, S, v, d); break;
+            case 4: evolve_step<R, kBates, kMilstein>(tables.get(), p, S, v, d); break;
+            default: evolve_step<R, kBates, kQE>(tables.get(), p, S, v, d); break;
         }
         if (d.overflow) {
             *status = 1;
@@ -935,14 +982,11 @@ cudaError_t launch_slab_paths(int precision, int model, int scheme, uint64_t see
     const PhiloxRoundKeys rk = philox_round_keys(static_cast<uint32_t>(seed & 0xFFFFFFFFull),
                                                  static_cast<uint32_t>(seed >> 32));
     if (paths_per_thread == 2) {
+        if (precision != QK_FP32) return cudaErrorInvalidValue;
         const int64_t threads = (count + 1) / 2;
         const unsigned blocks2 = static_cast<unsigned>((threads + kPathBlock - 1) / kPathBlock);
-        if (precision == QK_FP32)
-            slab_two_kernel_for<float>(model, scheme)<<<blocks2, kPathBlock, 0, s>>>(
-                task, first_path, count, stride, static_cast<float *>(slab_S), static_cast<float *>(slab_v), ld, rk);
-        else
-            slab_two_kernel_for<double>(model, scheme)<<<blocks2, kPathBlock, 0, s>>>(
-                task, first_path, count, stride, static_cast<double *>(slab_S), static_cast<double *>(slab_v), ld, rk);
+        slab_two_kernel_for(model, scheme)<<<blocks2, kPathBlock, 0, s>>>(
+            task, first_path, count, stride, static_cast<float *>(slab_S), static_cast<float *>(slab_v), ld, rk);
         return cudaGetLastError();
     }
     const int64_t blocks = (count + kPathBlock - 1) / kPathBlock;
@@ -958,9 +1002,9 @@ cudaError_t launch_slab_paths(int precision, int model, int scheme, uint64_t see
 cudaError_t launch_step_trace(int precision, cudaStream_t s, const TaskDev *task, const double *z, const double *u,
                               int umax, int n, double *S_out, double *v_out, int *status) {
     if (precision == QK_FP32)
-        step_trace_kernel<float><<<1, 1, 0, s>>>(task, z, u, umax, n, S_out, v_out, status);
+        step_trace_kernel<float><<<1, 32, 0, s>>>(task, z, u, umax, n, S_out, v_out, status);
     else
-        step_trace_kernel<double><<<1, 1, 0, s>>>(task, z, u, umax, n, S_out, v_out, status);
+        step_trace_kernel<double><<<1, 256, 0, s>>>(task, z, u, umax, n, S_out, v_out, status);
     return cudaGetLastError();
 }
 
@@ -1025,7 +1069,7 @@ static cudaError_t preload_path_kernels_of() {
                     for (int trk = 0; trk < 2 && e == cudaSuccess; ++trk)
                         e = cudaFuncGetAttributes(&fa, price_kernel_for<R>(model, scheme, uk != 0, lane, trk != 0));
             if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, slab_kernel_for<R>(model, scheme));
-            if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, slab_two_kernel_for<R>(model, scheme));
+            if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, slab_two_kernel_for(model, scheme));
         }
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, payoff_paths_kernel<R>);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, payoff_trace_kernel<R>);
