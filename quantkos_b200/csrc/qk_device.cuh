@@ -58,17 +58,91 @@ inline PhiloxRoundKeys philox_round_keys(uint32_t k0, uint32_t k1) {
     return rk;
 }
 
-__device__ __forceinline__ U4 philox4x32_10(U4 c, const PhiloxRoundKeys &rk) {
-#pragma unroll
-    for (int r = 0; r < 10; ++r) {
-        const uint64_t p0 = static_cast<uint64_t>(kPhiloxM0) * c.x;
-        const uint64_t p1 = static_cast<uint64_t>(kPhiloxM1) * c.z;
-        const uint32_t lo0 = static_cast<uint32_t>(p0), hi0 = static_cast<uint32_t>(p0 >> 32);
-        const uint32_t lo1 = static_cast<uint32_t>(p1), hi1 = static_cast<uint32_t>(p1 >> 32);
-        c = U4{hi1 ^ c.y ^ rk.k[2 * r], lo1, hi0 ^ c.w ^ rk.k[2 * r + 1], lo0};
-    }
-    return c;
+// Round keys of a launch whose tasks share the seed (from the parameter bank), or of the
+// task's own key.
+struct ParamKeys {
+    const PhiloxRoundKeys &rk;
+    __device__ __forceinline__ uint32_t k0(int r) const { return rk.k[2 * r]; }
+    __device__ __forceinline__ uint32_t k1(int r) const { return rk.k[2 * r + 1]; }
+};
+struct RegKeys {
+    uint32_t key0, key1;
+    __device__ __forceinline__ uint32_t k0(int r) const { return key0 + static_cast<uint32_t>(r) * kPhiloxW0; }
+    __device__ __forceinline__ uint32_t k1(int r) const { return key1 + static_cast<uint32_t>(r) * kPhiloxW1; }
+};
+
+// The path loop's Philox.  A 32x32->64 multiply occupies the FMA pipe for four cycles (an
+// FP32 FMA: one), so the generator's 20 per block are 40 of the pipe's cycles per
+// path-step, more than any step's arithmetic.  In the first three rounds most of the state
+// does not depend on both counter words: with the counter (block, path, stream, domain),
+//   round 1: x = hi(M1 stream) ^ path ^ k0 (per path), z, w from M0 block (per block),
+//   round 2: M0 x per path, M1 z per block,
+//   round 3: M0 x per block, M1 z the first multiply that needs both.
+// What depends on the path alone is computed once per path (PhiloxPath), what depends on
+// the block alone once per warp: lane l of a warp computes the row of block l of the next
+// 32 blocks (64 steps) into shared memory, and a step pair reads its row with one
+// broadcast load.  A block then costs 15 multiplies and 17 XORs instead of 20 and 20.
+// The same words as philox4x32_10.
+struct PhiloxPath {
+    uint32_t hi, lo;  // M0 x after round 1
+};
+__device__ __forceinline__ PhiloxPath philox_path_of(uint32_t x) {
+    const uint64_t p = static_cast<uint64_t>(kPhiloxM0) * x;
+    return PhiloxPath{static_cast<uint32_t>(p >> 32), static_cast<uint32_t>(p)};
 }
+template <class Keys>
+__device__ __forceinline__ uint4 philox_row(const Keys &k, uint32_t block, uint32_t stream, uint32_t domain) {
+    const uint64_t p0 = static_cast<uint64_t>(kPhiloxM0) * block;
+    const uint32_t y1 = kPhiloxM1 * stream;
+    const uint64_t p1 = static_cast<uint64_t>(kPhiloxM1) * (static_cast<uint32_t>(p0 >> 32) ^ domain ^ k.k1(0));
+    const uint64_t p2 = static_cast<uint64_t>(kPhiloxM0) * (static_cast<uint32_t>(p1 >> 32) ^ y1 ^ k.k0(1));
+    return make_uint4(static_cast<uint32_t>(p0) ^ k.k1(1), static_cast<uint32_t>(p1) ^ k.k0(2),
+                      static_cast<uint32_t>(p2 >> 32) ^ k.k1(2), static_cast<uint32_t>(p2) ^ k.k1(3));
+}
+template <class Keys>
+__device__ __forceinline__ U4 philox_rest(const Keys &k, const uint4 &row, const PhiloxPath &pp) {
+    const uint64_t q = static_cast<uint64_t>(kPhiloxM1) * (pp.hi ^ row.x);  // round 3
+    uint32_t x = static_cast<uint32_t>(q >> 32) ^ row.y, y = static_cast<uint32_t>(q), z = row.z ^ pp.lo, w = row.w;
+#pragma unroll
+    for (int r = 3; r < 10; ++r) {
+        const uint64_t p0 = static_cast<uint64_t>(kPhiloxM0) * x;
+        const uint64_t p1 = static_cast<uint64_t>(kPhiloxM1) * z;
+        x = static_cast<uint32_t>(p1 >> 32) ^ y ^ k.k0(r);
+        y = static_cast<uint32_t>(p1);
+        z = r == 3 ? static_cast<uint32_t>(p0 >> 32) ^ w : static_cast<uint32_t>(p0 >> 32) ^ w ^ k.k1(r);  // row.w holds k1(3)
+        w = static_cast<uint32_t>(p0);
+    }
+    return U4{x, y, z, w};
+}
+
+// Rows of a warp: 32 normal blocks, then (FP64 Bates) 16 first-Poisson-word blocks, of the
+// 64 steps from n0 (a multiple of 64).  Every lane of the warp takes part in fill.
+constexpr int kRowSteps = 64;
+template <class R, int MODEL>
+constexpr int philox_rows() {
+    return 32 + (sizeof(R) == 8 && MODEL == kBates ? 16 : 0);
+}
+template <int ROWS, class Keys>
+struct WarpPhilox {
+    Keys keys;
+    uint4 *rows;  // this warp's, in shared memory
+    uint32_t stream;
+    __device__ __forceinline__ void fill(int n0) const {
+        const uint32_t lane = threadIdx.x & 31u;
+        __syncwarp();  // the rows of the previous 64 steps have been read
+        rows[lane] = philox_row(keys, static_cast<uint32_t>(n0 >> 1) + lane, stream, 0u);
+        if (ROWS > 32 && lane < 16) rows[32 + lane] = philox_row(keys, static_cast<uint32_t>(n0 >> 2) + lane, stream, 2u);
+        __syncwarp();
+    }
+    // x after round 1
+    __device__ __forceinline__ uint32_t path_word(uint32_t path) const {
+        return static_cast<uint32_t>((static_cast<uint64_t>(kPhiloxM1) * stream) >> 32) ^ path ^ keys.k0(0);
+    }
+    __device__ __forceinline__ PhiloxPath path(uint32_t path) const { return philox_path_of(path_word(path)); }
+    __device__ __forceinline__ U4 block(const uint4 *row, const PhiloxPath &pp) const {
+        return philox_rest(keys, *row, pp);
+    }
+};
 
 // ============================================================================
 // Arithmetic policy.  FP32 uses the SFU (MUFU) approximations explicitly; FP64 uses the
@@ -116,18 +190,21 @@ struct Math<float> {
     // both are exact and so is the difference (2k + 1) 2^-24, so this equals
     // k * 2^-23 + 2^-24 bit for bit without an integer-to-float conversion.
     static __device__ __forceinline__ float u01(uint32_t w) {
-        return __fsub_rn(__uint_as_float(0x3F800000u | (w >> 9)), 0.99999994039535522f);
+        return __fsub_rn(mantissa(w), 0.99999994039535522f);
+    }
+    // 1 + k 2^-23 (one funnel shift: the exponent bits come in from the left)
+    static __device__ __forceinline__ float mantissa(uint32_t w) {
+        return __uint_as_float(__funnelshift_r(w, 0x7Fu, 9));
     }
     static constexpr float kU01Offset = 0.99999994039535522f;  // 1 - 2^-24
     static constexpr float kTwoPi = 6.28318530717958648f;
     // Box-Muller pair: R = sqrt(-2 ln u1), angle = 2*pi*(u2 - 1/2); IEEE-rounded
-    // operations in a fixed order (box_muller_two repeats them on pairs)
+    // operations in a fixed order (box_muller_two repeats them on pairs).  With
+    // f = 1 + k 2^-23, u2 - 1/2 = (f - 3/2) + 2^-24 exactly, so the angle is one FMA.
     static __device__ __forceinline__ void box_muller(uint32_t w1, uint32_t w2, float &z1, float &z2) {
-        const float u1 = u01(w1);
-        const float u2 = u01(w2);
-        const float rad = ptx_sqrt(__fmul_rn(-2.0f * kLn2, ptx_lg2(u1)));
+        const float rad = ptx_sqrt(__fmul_rn(-2.0f * kLn2, ptx_lg2(u01(w1))));
         float s, c;
-        __sincosf(__fmul_rn(kTwoPi, __fadd_rn(u2, -0.5f)), &s, &c);
+        __sincosf(__fmaf_rn(__fadd_rn(mantissa(w2), -1.5f), kTwoPi, kTwoPi / 16777216.0f), &s, &c);
         z1 = __fmul_rn(rad, c);
         z2 = __fmul_rn(rad, s);
     }
@@ -136,15 +213,13 @@ struct Math<float> {
     // gets the same bits as from box_muller.  z1 = (z1 of a, z1 of b), z2 likewise.
     static __device__ __forceinline__ void box_muller_two(uint32_t a1, uint32_t a2, uint32_t b1, uint32_t b2,
                                                           float2 &z1, float2 &z2) {
-        const float2 off = make_float2(-kU01Offset, -kU01Offset);
-        const float2 u1 = __fadd2_rn(make_float2(__uint_as_float(0x3F800000u | (a1 >> 9)),
-                                                 __uint_as_float(0x3F800000u | (b1 >> 9))), off);
-        const float2 u2 = __fadd2_rn(make_float2(__uint_as_float(0x3F800000u | (a2 >> 9)),
-                                                 __uint_as_float(0x3F800000u | (b2 >> 9))), off);
+        const float2 u1 = __fadd2_rn(make_float2(mantissa(a1), mantissa(b1)), make_float2(-kU01Offset, -kU01Offset));
+        const float2 g = __fadd2_rn(make_float2(mantissa(a2), mantissa(b2)), make_float2(-1.5f, -1.5f));
         const float2 t = __fmul2_rn(make_float2(-2.0f * kLn2, -2.0f * kLn2),
                                     make_float2(ptx_lg2(u1.x), ptx_lg2(u1.y)));
         const float2 rad = make_float2(ptx_sqrt(t.x), ptx_sqrt(t.y));
-        const float2 ang = __fmul2_rn(make_float2(kTwoPi, kTwoPi), __fadd2_rn(u2, make_float2(-0.5f, -0.5f)));
+        const float2 ang = __ffma2_rn(g, make_float2(kTwoPi, kTwoPi),
+                                      make_float2(kTwoPi / 16777216.0f, kTwoPi / 16777216.0f));
         float sa, ca, sb, cb;
         __sincosf(ang.x, &sa, &ca);
         __sincosf(ang.y, &sb, &cb);
@@ -218,7 +293,7 @@ struct PhiloxJumpDraws {
         return Math<R>::u01(word);
     }
     __device__ __forceinline__ R jump_normal() {
-        const U4 j = block(1u);
+        const U4 j = domain == 1 ? wx : block(1u);  // the block of the 2nd and 3rd uniforms
         R z1, z2;
         Math<R>::box_muller(j.x, j.y, z1, z2);
         return z1;
@@ -347,7 +422,6 @@ __device__ __forceinline__ float2 rcp2(float2 x) { return make_float2(ptx_rcp(x.
 __device__ __forceinline__ float2 sqrt2(float2 x) { return make_float2(ptx_sqrt(x.x), ptx_sqrt(x.y)); }
 __device__ __forceinline__ float2 lg2_2(float2 x) { return make_float2(ptx_lg2(x.x), ptx_lg2(x.y)); }
 __device__ __forceinline__ float2 ex2_2(float2 x) { return make_float2(ptx_ex2(x.x), ptx_ex2(x.y)); }
-__device__ __forceinline__ float2 min2(float2 a, float2 b) { return make_float2(fminf(a.x, b.x), fminf(a.y, b.y)); }
 __device__ __forceinline__ float2 max0_2(float2 a) { return make_float2(fmaxf(a.x, 0.0f), fmaxf(a.y, 0.0f)); }
 
 // QE step of two paths (spot S, variance v as pairs): paired when both take the
@@ -355,29 +429,30 @@ __device__ __forceinline__ float2 max0_2(float2 a) { return make_float2(fmaxf(a.
 __device__ __forceinline__ void step_qe_two_f32(const StepConst<float> &p, float2 &S, float2 &v, float2 Zv,
                                                 float2 Zind) {
     const float2 m = __ffma2_rn(v, f2(p.exp_mkdt), f2(p.theta_m));
-    const float2 s2 = __ffma2_rn(v, f2(p.s2f1), f2(p.s2f2));
+    const float2 h = __ffma2_rn(v, f2(p.h_f1), f2(p.h_f2));  // s^2 / 2
     const float2 m2 = __fmul2_rn(m, m);
-    const float2 em2 = __fmul2_rn(f2(p.eps), m2);
-    const float2 pm2 = __fmul2_rn(f2(p.psi_c), m2);
-    const bool quad = m.x > p.eps && m.y > p.eps && s2.x > em2.x && s2.y > em2.y && s2.x <= pm2.x && s2.y <= pm2.y;
+    const float2 em2 = __fmul2_rn(f2(p.h_eps), m2);
+    const float2 pm2 = __fmul2_rn(f2(p.h_psi_plain), m2);
+    const bool quad = m.x > p.eps && m.y > p.eps && h.x > em2.x && h.y > em2.y && h.x <= pm2.x && h.y <= pm2.y;
     // the quadratic form for both paths first (no branch before the long SFU chain);
     // a pair not both in the quadratic regime is redone per path below
     const float2 S_old = S, v_old = v;
-    // qe_quadratic_f32, paired
-    const float2 two_ip = __fmul2_rn(__fmul2_rn(f2(2.0f), m2), rcp2(s2));
+    // qe_quadratic_f32, paired: m2 rcp(s^2 / 2) has the bits of 2 m2 rcp(s^2), and where
+    // h_psi_plain admits the step min(A a, 1/2 - eps a) is A a
+    const float2 two_ip = __fmul2_rn(m2, rcp2(h));
     const float2 t1 = __fadd2_rn(two_ip, f2(-1.0f));
     const float2 b2 = __fadd2_rn(t1, sqrt2(__fmul2_rn(two_ip, t1)));
     const float2 a = __fmul2_rn(m, rcp2(__fadd2_rn(f2(1.0f), b2)));
     const float2 bz = __fadd2_rn(sqrt2(b2), Zv);
     const float2 vn = __fmul2_rn(__fmul2_rn(a, bz), bz);
-    const float2 Aa = min2(__fmul2_rn(f2(p.A), a), __ffma2_rn(f2(-p.eps), a, f2(0.5f)));
+    const float2 Aa = __fmul2_rn(f2(p.A), a);
     const float2 term = __ffma2_rn(f2(-2.0f), Aa, f2(1.0f));
     const float2 logM = __ffma2_rn(__fmul2_rn(Aa, b2), rcp2(term),
                                    __fmul2_rn(f2(-0.5f * Math<float>::kLn2), lg2_2(term)));
     // qe_spot_f32, paired
     const float2 K0n = __ffma2_rn(f2(p.K1_half_K3), v, logM);
     const float2 isig = __ffma2_rn(f2(p.K3), v, __fmul2_rn(f2(p.K4), vn));
-    const float2 e12 = __fadd2_rn(__fadd2_rn(f2(p.r_minus_q_dt), __fmul2_rn(K0n, f2(-1.0f))),
+    const float2 e12 = __fadd2_rn(__ffma2_rn(K0n, f2(-1.0f), f2(p.r_minus_q_dt)),
                                   __ffma2_rn(f2(p.K1), v, __fmul2_rn(f2(p.K2), vn)));
     const float2 ex = __ffma2_rn(sqrt2(isig), Zind, e12);
     S = __fmul2_rn(S, ex2_2(__fmul2_rn(ex, f2(Math<float>::kLog2e))));
@@ -504,15 +579,10 @@ __device__ __forceinline__ void step64(const StepConst<double> &p, Path64 &s, do
         double vn = (a * bz) * bz;
         const double term = u * iq;
         double dx = -p.l_A * ((G * q) * (q * R));
-        // Inside the quadratic regime (m, s^2 > eps m^2, s^2 <= psi_c m^2) with the clamp of
-        // A inactive (term far from 0)?  Compared by the high words of the (positive) values,
-        // strictly, so a value next to a threshold takes the exact branches.  eps and the
-        // bounds on m and term: m in (eps, 2^19), term in (2^-20, 2^40).
-        const bool quad =
-            static_cast<uint32_t>(__double2hiint(m) - __double2hiint(p.eps) - 1) <
-                static_cast<uint32_t>(0x41200000 - __double2hiint(p.eps) - 1) &&
-            below_hi64(h, p.h_psi * m2) && below_hi64(p.h_eps * m2, h) &&
-            static_cast<uint32_t>(__double2hiint(term) - 0x3EB00000) < 0x03C00000u;
+        // Inside the quadratic regime (m > eps, eps m^2 < s^2 <= psi_c m^2), no clamp possible?
+        // Compared by the high words (positive values order as integers), strictly, so a value
+        // next to a threshold, and NaN, take the exact branches.
+        const bool quad = below_hi64(p.eps, m) && below_hi64(p.h_eps * m2, h) && below_hi64(h, p.h_psi_plain * m2);
         if (!quad) {
             const double2 r = qe_regimes64(m, 2.0 * h, Z1, p.psi_c, p.eps, p.A);
             vn = r.x;
@@ -555,6 +625,7 @@ __device__ __noinline__ R jump_factor(const StepConst<R> &p, R prod, Draws &d) {
     const R rN = static_cast<R>(N);
     return Math<R>::exp(rN * p.mu_j + Math<R>::sqrt(rN) * p.sigma_j * Z);
 }
+
 
 // Both members of an antithetic pair: the same jump count, jump sizes with the
 // normal of opposite sign.

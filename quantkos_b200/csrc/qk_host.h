@@ -2,6 +2,7 @@
 // contract validation with the reference's rules, and the per-step invariants.
 #pragma once
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <string>
@@ -91,9 +92,15 @@ inline StepConst<R> make_step_const(const qk_contract &c, double dt, double eps)
     d.l_sqrt_K3 = std::sqrt(d.K3) * kLog2e;
     d.h_f1 = 0.5 * d.s2f1;
     d.h_f2 = 0.5 * d.s2f2;
-    d.h_psi = 0.5 * d.psi_c;
     d.h_eps = 0.5 * d.eps;
     d.two_A = 2.0 * d.A;
+    // QE's a = h / (m + G) <= h / m = (v h_f1 + h_f2) / (v e^{-k dt} + theta_m), a mediant of
+    // two fixed ratios: where 2 (A + eps) times the larger stays below 1 (it does at any usual
+    // parameters) min(A a, 1/2 - eps a) is A a on every step, and the steps' plain form of
+    // the quadratic regime needs no clamp.  Elsewhere no step takes the plain form.
+    const double a_max = std::max(d.h_f1 / d.exp_mkdt, d.theta_m > 0.0 ? d.h_f2 / d.theta_m : 0.0);
+    const bool plain = 2.0 * (d.A + eps) * a_max <= 1.0 - 1.0 / 1024.0 && std::fabs(d.two_A) * a_max < 1e12;
+    d.h_psi_plain = plain ? 0.5 * d.psi_c : -1.0;
     if constexpr (sizeof(R) == sizeof(double)) {
         return d;
     } else {

@@ -51,14 +51,17 @@ struct SlabSink {
     int64_t pos;    // slab index of this path's next stored date: row * ld + column
     int stride;     // steps between stored dates
     int left;       // steps until the next stored date
+    bool has;       // the path exists (a warp's lanes beyond the last path store nothing)
     // Called once per step, in order: every stride-th step is stored.
     template <class Spot>
     __device__ __forceinline__ void operator()(int, Spot spot, R v) {
         if (--left == 0) {
             left = stride;
-            if constexpr (sizeof(R) == 8) slab_S[pos] = spot();
-            else slab_S[pos] = spot;
-            if (slab_v) slab_v[pos] = v;
+            if (has) {
+                if constexpr (sizeof(R) == 8) slab_S[pos] = spot();
+                else slab_S[pos] = spot;
+                if (slab_v) slab_v[pos] = v;
+            }
             pos += ld;
         }
     }
@@ -78,14 +81,14 @@ struct SlabSink2 {
     int64_t pos;   // slab index of path a's next stored date; path b is the next column
     int stride;
     int left;
-    bool has_b;
+    bool has_a, has_b;
     __device__ __forceinline__ void operator()(int, R Sa, R va, R Sb, R vb) {
         if (--left == 0) {
             left = stride;
-            slab_S[pos] = Sa;
+            if (has_a) slab_S[pos] = Sa;
             if (has_b) slab_S[pos + 1] = Sb;
             if (slab_v) {
-                slab_v[pos] = va;
+                if (has_a) slab_v[pos] = va;
                 if (has_b) slab_v[pos + 1] = vb;
             }
             pos += ld;
@@ -104,17 +107,6 @@ __device__ __forceinline__ void track(PathState<R> &st, R &blk) {
     st.smin = rmin(st.smin, st.S);
 }
 
-// Philox with round keys read from the kernel's parameter bank (all tasks of the
-// launch share the seed) or computed per round from the task's key.
-struct ParamKeys {
-    const PhiloxRoundKeys &rk;
-    __device__ __forceinline__ U4 operator()(U4 c) const { return philox4x32_10(c, rk); }
-};
-struct RegKeys {
-    uint32_t k0, k1;
-    __device__ __forceinline__ U4 operator()(U4 c) const { return philox4x32_10(c, k0, k1); }
-};
-
 // The step's first Poisson uniform decides whether a jump happened (Knuth's loop
 // continues only if it is >= exp(-lambda dt)).
 //
@@ -125,19 +117,24 @@ struct RegKeys {
 // u01 >= exp(-lambda dt) in float, kmin precomputed exactly) cannot pass while
 // hi < kmin >> 5, so the common step compares hi alone and lo is drawn only past that
 // threshold (about lambda dt of the steps).
+// The common test compares hi at the top of a word (two shifts, no masks) with kmin >> 5
+// brought there; where that is 2^18 (no jumps at all) the threshold is past every hi.
 __device__ __forceinline__ uint32_t poisson_hi_f32(uint32_t wa, uint32_t wb) {
-    return ((wa & 0x1FFu) << 9) | (wb & 0x1FFu);
+    return __funnelshift_l(wb << 23, wa, 23);  // hi << 14
+}
+__device__ __forceinline__ uint32_t poisson_threshold_f32(uint32_t kmin) {
+    return kmin < (1u << 23) ? (kmin >> 5) << 14 : 0xFFFFFFFFu;
 }
 
-// pois: the 18 high bits (poisson_hi_f32).  On a jump, `word` holds the full
-// first-uniform word (top 23 bits k).
+// Past the threshold: the exact test.  On a jump, `word` holds the full first-uniform
+// word (top 23 bits k).
 __device__ __forceinline__ bool jump_first_f32(uint32_t pois, uint32_t kmin, uint32_t k0, uint32_t k1, uint32_t path,
                                                uint32_t stream, int n, uint32_t &word) {
-    if (pois < (kmin >> 5)) return false;
+    if (pois < poisson_threshold_f32(kmin)) return false;
     const U4 q = philox4x32_10(U4{static_cast<uint32_t>(n >> 2), path, stream, 2u}, k0, k1);
     const int j = n & 3;
     const uint32_t w = j == 0 ? q.x : (j == 1 ? q.y : (j == 2 ? q.z : q.w));
-    word = ((pois << 5) | (w >> 27)) << 9;
+    word = ((pois >> 9) | (w >> 27)) << 9;
     return (word >> 9) >= kmin;
 }
 
@@ -189,11 +186,16 @@ __device__ __forceinline__ void simulate_f64(const Tab64 &tab, const StepConst<d
         st[i].smax = st[i].smin = 1.0;
     }
     constexpr int ND = NEG ? 1 : NP;  // draw sequences
+    PhiloxPath pp[ND];
+#pragma unroll
+    for (int i = 0; i < ND; ++i) pp[i] = gen.path(path + i);
     for (int n0 = 0; n0 < n_steps; n0 += kSumChunk) {
         const int n1 = min(n0 + kSumChunk, n_steps);
         double blk[NP];
 #pragma unroll
         for (int i = 0; i < NP; ++i) blk[i] = 0.0;
+        if ((n0 & (kRowSteps - 1)) == 0) gen.fill(n0);
+        const uint4 *row = gen.rows + ((n0 & (kRowSteps - 1)) >> 1);
         U4 w[ND], wp[ND];
         auto step = [&](int n, bool odd) {
 #pragma unroll
@@ -236,11 +238,12 @@ __device__ __forceinline__ void simulate_f64(const Tab64 &tab, const StepConst<d
         for (int n = n0; n < n1; n += 2) {
 #pragma unroll
             for (int i = 0; i < ND; ++i) {
-                w[i] = gen(U4{static_cast<uint32_t>(n >> 1), path + i, stream, 0u});
+                w[i] = gen.block(row, pp[i]);
                 if constexpr (MODEL == kBates) {
-                    if ((n & 3) == 0) wp[i] = gen(U4{static_cast<uint32_t>(n >> 2), path + i, stream, 2u});
+                    if ((n & 3) == 0) wp[i] = gen.block(gen.rows + 32 + ((n & (kRowSteps - 1)) >> 2), pp[i]);
                 }
             }
+            ++row;
             step(n, false);
             if (n + 1 < n1) step(n + 1, true);
         }
@@ -280,12 +283,15 @@ __device__ __forceinline__ void simulate_path(const Tab64 *tab, const StepConst<
         st.ssum = 0.0;
         st.smax = S0;
         st.smin = S0;
+        const PhiloxPath pp = gen.path(path);
         for (int n0 = 0; n0 < n_steps; n0 += kSumChunk) {
             const int n1 = min(n0 + kSumChunk, n_steps);
+            if ((n0 & (kRowSteps - 1)) == 0) gen.fill(n0);
+            const uint4 *row = gen.rows + ((n0 & (kRowSteps - 1)) >> 1);
             R blk = R(0);
             int n = n0;
-            for (; n + 1 < n1; n += 2) {
-                const U4 w = gen(U4{static_cast<uint32_t>(n >> 1), path, stream, 0u});
+            for (; n + 1 < n1; n += 2, ++row) {
+                const U4 w = gen.block(row, pp);
                 // the normals of both steps (independent of the path state) in one paired
                 // Box-Muller; the same bits as two one-pair calls
                 float2 Z1, Z2;
@@ -298,7 +304,7 @@ __device__ __forceinline__ void simulate_path(const Tab64 *tab, const StepConst<
                 sink(n + 1, st.S, st.v);
             }
             if (n < n1) {
-                const U4 w = gen(U4{static_cast<uint32_t>(n >> 1), path, stream, 0u});
+                const U4 w = gen.block(row, pp);
                 float z1, z2;
                 Math<float>::box_muller(w.x, w.y, z1, z2);
                 one_step_z<MODEL, SCHEME>(p, st, z1, z2, poisson_hi_f32(w.x, w.y), kmin, k0, k1, path, stream, n);
@@ -348,8 +354,8 @@ __device__ __forceinline__ void jumps_two(const StepConst<float> &p, PathState<f
         } else {
             // the one-compare tests of both paths inline; one copy of the rest of the
             // jump code for both (rare; keeps the loop body small)
-            const uint32_t kmin_hi = kmin >> 5;
-            if (pois_a >= kmin_hi || pois_b >= kmin_hi) {
+            const uint32_t thr = poisson_threshold_f32(kmin);
+            if (pois_a >= thr || pois_b >= thr) {
 #pragma unroll 1
                 for (int i = 0; i < 2; ++i) {
                     const uint32_t pois = i ? pois_b : pois_a, path = i ? path_b : path_a;
@@ -399,14 +405,29 @@ __device__ __forceinline__ void simulate_two(const StepConst<float> &p, float S0
     if (TRK && ssum_slot) *ssum_slot = make_double2(0.0, 0.0);
     a.smax = b.smax = S0;
     a.smin = b.smin = S0;
+    // Registers are short in all these loops but Heston Euler's: there the two paths' hoisted
+    // products (four words) give way to the one word they come from (path b = path a ^ 1),
+    // and its two multiplies are repeated per block.  Cycles per path-step and scheduler,
+    // hoisted / repeated: Heston Euler 63.4 / 67.2, Milstein 69.8 / 69.4, QE 113.2 / 110.7,
+    // Bates Euler 79.3 / 78.3, Milstein 84.4 / 82.5, QE 119.6 / 118.7.
+    constexpr bool kRepeat = !NEG && !(MODEL == kHeston && SCHEME == kEuler);
+    uint32_t xa = gen.path_word(path_a);
+    PhiloxPath ppa = gen.path(path_a), ppb = gen.path(path_b);
     for (int n0 = 0; n0 < n_steps; n0 += kSumChunk) {
         const int n1 = min(n0 + kSumChunk, n_steps);
+        if ((n0 & (kRowSteps - 1)) == 0) gen.fill(n0);
+        const uint4 *row = gen.rows + ((n0 & (kRowSteps - 1)) >> 1);
         float blk_a = 0.0f, blk_b = 0.0f;
         int n = n0;
-        for (; n + 1 < n1; n += 2) {
-            const U4 wa = gen(U4{static_cast<uint32_t>(n >> 1), path_a, stream, 0u});
+        for (; n + 1 < n1; n += 2, ++row) {
+            if constexpr (kRepeat) {
+                asm volatile("" : "+r"(xa));  // not hoisted out of the loop
+                ppa = philox_path_of(xa);
+                ppb = philox_path_of(xa ^ 1u);
+            }
+            const U4 wa = gen.block(row, ppa);
             U4 wb{0u, 0u, 0u, 0u};
-            if constexpr (!NEG) wb = gen(U4{static_cast<uint32_t>(n >> 1), path_b, stream, 0u});
+            if constexpr (!NEG) wb = gen.block(row, ppb);
             const uint32_t qa0 = poisson_hi_f32(wa.x, wa.y), qa1 = poisson_hi_f32(wa.z, wa.w);
             const uint32_t qb0 = poisson_hi_f32(wb.x, wb.y), qb1 = poisson_hi_f32(wb.z, wb.w);
             float2 Z1a, Z2a, Z1b, Z2b;
@@ -426,9 +447,14 @@ __device__ __forceinline__ void simulate_two(const StepConst<float> &p, float S0
             sink(n + 1, a.S, a.v, b.S, b.v);
         }
         if (n < n1) {
-            const U4 wa = gen(U4{static_cast<uint32_t>(n >> 1), path_a, stream, 0u});
+            if constexpr (kRepeat) {
+                asm volatile("" : "+r"(xa));  // not hoisted out of the loop
+                ppa = philox_path_of(xa);
+                ppb = philox_path_of(xa ^ 1u);
+            }
+            const U4 wa = gen.block(row, ppa);
             U4 wb{0u, 0u, 0u, 0u};
-            if constexpr (!NEG) wb = gen(U4{static_cast<uint32_t>(n >> 1), path_b, stream, 0u});
+            if constexpr (!NEG) wb = gen.block(row, ppb);
             float2 Z1, Z2;
             normals_two_f32<NEG>(wa.x, wa.y, wb.x, wb.y, Z1, Z2);
             const uint32_t qa0 = poisson_hi_f32(wa.x, wa.y), qb0 = poisson_hi_f32(wb.x, wb.y);
@@ -469,12 +495,12 @@ __device__ __forceinline__ uint32_t task_kmin(const TaskDev &t) {
 }
 
 template <class R, class Sink>
-__device__ __forceinline__ void simulate_dispatch(const Tab64 *tab, const TaskDev &t, const StepConst<R> &p,
-                                                  uint32_t path, PathState<R> &st, Sink &&sink) {
+__device__ __forceinline__ void simulate_dispatch(const Tab64 *tab, uint4 *rows, const TaskDev &t,
+                                                  const StepConst<R> &p, uint32_t path, PathState<R> &st, Sink &&sink) {
     const R S0 = static_cast<R>(t.S0);
     const R v0 = static_cast<R>(t.v0);
     const uint32_t km = task_kmin<R>(t);
-    const RegKeys g{t.key0, t.key1};
+    const WarpPhilox<philox_rows<R, kBates>(), RegKeys> g{RegKeys{t.key0, t.key1}, rows, t.stream};
     switch (t.model * 3 + t.scheme) {
         case 0: simulate_path<R, kHeston, kEuler>(tab, p, S0, v0, t.n_steps, g, t.key0, t.key1, path, t.stream, km, st, sink); break;
         case 1: simulate_path<R, kHeston, kMilstein>(tab, p, S0, v0, t.n_steps, g, t.key0, t.key1, path, t.stream, km, st, sink); break;
@@ -529,6 +555,8 @@ __global__ void __launch_bounds__(path_block_max<R>(),
     Moments *acc = s_acc[warp];
     __shared__ BlockTables<R> tables;
     tables.fill();
+    constexpr int kRows = philox_rows<R, MODEL>();
+    __shared__ uint4 s_rows[path_block_max<R>() / 32][kRows];
 
     for (;;) {
         long long q = 0;
@@ -559,6 +587,12 @@ __global__ void __launch_bounds__(path_block_max<R>(),
         const int64_t left = n_units - tile_first;
         const int rounds =
             static_cast<int>(min(static_cast<int64_t>(tile_rounds), (left + kWarpTilePaths - 1) / kWarpTilePaths));
+        // Every lane simulates (the generator's rows are the warp's work); a lane beyond the
+        // task's last unit simulates a path that no record counts.
+        const auto with_keys = [&](const auto &simulate) {
+            if constexpr (UK) simulate(WarpPhilox<kRows, ParamKeys>{ParamKeys{rk}, s_rows[warp], stream});
+            else simulate(WarpPhilox<kRows, RegKeys>{RegKeys{k0, k1}, s_rows[warp], stream});
+        };
         for (int j = 0; j < rounds; ++j) {
             const int64_t unit = tile_first + static_cast<int64_t>(j) * kWarpTilePaths + lane;
             const bool active = unit < n_units;
@@ -568,26 +602,18 @@ __global__ void __launch_bounds__(path_block_max<R>(),
                 const uint32_t pb = NEG ? pa : pa + 1u;
                 const bool active_b = NEG ? active : (active && static_cast<int64_t>(pb) < n_paths);
                 PathState<R> sa, sb;
-                if (active) {
-                    const auto simulate = [&](const auto &gen) {
-                        if constexpr (sizeof(R) == 8) {
-                            PathState<double> two[2];
-                            simulate_f64<MODEL, SCHEME, TRK, 2, NEG>(*tables.get(), p, S0, v0, n_steps, gen, k0, k1, pa,
-                                                                     stream, kmin, two, NoSink{});
-                            sa = two[0];
-                            sb = two[1];
-                        } else {
-                            simulate_two<MODEL, SCHEME, NEG, TRK>(p, S0, v0, n_steps, gen, k0, k1, pa, pb, stream, kmin,
-                                                                  sa, sb, NoSink2{},
-                                                                  kSumSlot ? &s_ssum[threadIdx.x] : nullptr);
-                        }
-                    };
-                    if constexpr (UK) simulate(ParamKeys{rk});
-                    else simulate(RegKeys{k0, k1});
-                } else {
-                    sa.S = sa.smax = sa.smin = sb.S = sb.smax = sb.smin = R(0);
-                    sa.ssum = sb.ssum = 0.0;
-                }
+                with_keys([&](const auto &gen) {
+                    if constexpr (sizeof(R) == 8) {
+                        PathState<double> two[2];
+                        simulate_f64<MODEL, SCHEME, TRK, 2, NEG>(*tables.get(), p, S0, v0, n_steps, gen, k0, k1, pa, stream,
+                                                                 kmin, two, NoSink{});
+                        sa = two[0];
+                        sb = two[1];
+                    } else {
+                        simulate_two<MODEL, SCHEME, NEG, TRK>(p, S0, v0, n_steps, gen, k0, k1, pa, pb, stream, kmin, sa, sb,
+                                                              NoSink2{}, kSumSlot ? &s_ssum[threadIdx.x] : nullptr);
+                    }
+                });
                 for (int k = 0; k < np; ++k) {
                     const PayoffSpec ps = t.pay[k];
                     const R xa = active ? final_payoff<R>(ps, sa.S, sa.ssum, sa.smax, sa.smin, n_steps) : R(0);
@@ -604,18 +630,10 @@ __global__ void __launch_bounds__(path_block_max<R>(),
                 }
             } else {
                 PathState<R> st;
-                if (active) {
-                    if constexpr (UK) {
-                        simulate_path<R, MODEL, SCHEME, TRK>(tables.get(), p, S0, v0, n_steps, ParamKeys{rk}, k0, k1,
-                                                        static_cast<uint32_t>(unit), stream, kmin, st, NoSink{});
-                    } else {
-                        simulate_path<R, MODEL, SCHEME, TRK>(tables.get(), p, S0, v0, n_steps, RegKeys{k0, k1}, k0, k1,
-                                                        static_cast<uint32_t>(unit), stream, kmin, st, NoSink{});
-                    }
-                } else {
-                    st.S = st.smax = st.smin = R(0);
-                    st.ssum = 0.0;
-                }
+                with_keys([&](const auto &gen) {
+                    simulate_path<R, MODEL, SCHEME, TRK>(tables.get(), p, S0, v0, n_steps, gen, k0, k1,
+                                                         static_cast<uint32_t>(unit), stream, kmin, st, NoSink{});
+                });
                 for (int k = 0; k < np; ++k) {
                     const PayoffSpec ps = t.pay[k];
                     const R x = active ? final_payoff<R>(ps, st.S, st.ssum, st.smax, st.smin, n_steps) : R(0);
@@ -796,7 +814,7 @@ __global__ void __launch_bounds__(128) merge_task_chunks_kernel(const TaskDev *_
 // Philox round keys in the kernel parameters.  FP64: grid-stride over the paths, so that
 // a block's function tables are filled once.
 template <class R, int MODEL, int SCHEME>
-__global__ void __launch_bounds__(kPathBlock) slab_paths_kernel(const TaskDev *__restrict__ task, int64_t first_path,
+__global__ void __launch_bounds__(kPathBlock, sizeof(R) == 4 ? kPathMinBlocksFp32 : kPathMinBlocksQe64) slab_paths_kernel(const TaskDev *__restrict__ task, int64_t first_path,
                                                                int64_t count, int stride, R *__restrict__ slab_S,
                                                                R *__restrict__ slab_v, int64_t ld,
                                                                const PhiloxRoundKeys rk) {
@@ -804,33 +822,41 @@ __global__ void __launch_bounds__(kPathBlock) slab_paths_kernel(const TaskDev *_
     tables.fill();
     const TaskDev &t = *task;
     const StepConst<R> p = task_const<R>(t);
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < count;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        SlabSink<R> sink{slab_S, slab_v, ld, i, stride, stride};
+    constexpr int kRows = philox_rows<R, MODEL>();
+    __shared__ uint4 s_rows[kPathBlock / 32][kRows];
+    const WarpPhilox<kRows, ParamKeys> gen{ParamKeys{rk}, s_rows[threadIdx.x >> 5], t.stream};
+    // whole warps: a lane beyond the last path simulates without storing
+    const int lane = threadIdx.x & 31;
+    for (int64_t i0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x - lane; i0 < count;
+         i0 += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        const int64_t i = i0 + lane;
+        SlabSink<R> sink{slab_S, slab_v, ld, i, stride, stride, i < count};
         PathState<R> st;
-        simulate_path<R, MODEL, SCHEME, false>(tables.get(), p, static_cast<R>(t.S0), static_cast<R>(t.v0), t.n_steps,
-                                               ParamKeys{rk}, t.key0, t.key1, static_cast<uint32_t>(first_path + i),
-                                               t.stream, task_kmin<R>(t), st, sink);
+        simulate_path<R, MODEL, SCHEME, false>(tables.get(), p, static_cast<R>(t.S0), static_cast<R>(t.v0), t.n_steps, gen,
+                                               t.key0, t.key1, static_cast<uint32_t>(first_path + i), t.stream,
+                                               task_kmin<R>(t), st, sink);
     }
 }
 
 // FP32, two paths per thread (first + 2i and first + 2i + 1), interleaved and stepped as
 // pairs; same values as the one-path kernel.
 template <int MODEL, int SCHEME>
-__global__ void __launch_bounds__(kPathBlock) slab_paths_two_kernel(const TaskDev *__restrict__ task,
+__global__ void __launch_bounds__(kPathBlock, kPathMinBlocksFp32) slab_paths_two_kernel(const TaskDev *__restrict__ task,
                                                                    int64_t first_path, int64_t count, int stride,
                                                                    float *__restrict__ slab_S,
                                                                    float *__restrict__ slab_v, int64_t ld,
                                                                    const PhiloxRoundKeys rk) {
     const int64_t i = 2 * (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x);
-    if (i >= count) return;
+    if (i - 2 * (threadIdx.x & 31) >= count) return;  // whole warps only: the generator's rows are the warp's work
     const TaskDev &t = *task;
     const StepConst<float> p = task_const<float>(t);
-    SlabSink2<float> sink{slab_S, slab_v, ld, i, stride, stride, i + 1 < count};
+    __shared__ uint4 s_rows[kPathBlock / 32][32];
+    const WarpPhilox<32, ParamKeys> gen{ParamKeys{rk}, s_rows[threadIdx.x >> 5], t.stream};
+    SlabSink2<float> sink{slab_S, slab_v, ld, i, stride, stride, i < count, i + 1 < count};
     PathState<float> sa, sb;
     const uint32_t pa = static_cast<uint32_t>(first_path + i);
     simulate_two<MODEL, SCHEME, false, false>(p, static_cast<float>(t.S0), static_cast<float>(t.v0), t.n_steps,
-                                              ParamKeys{rk}, t.key0, t.key1, pa, pa + 1u, t.stream, t.jump_kmin, sa, sb,
+                                              gen, t.key0, t.key1, pa, pa + 1u, t.stream, t.jump_kmin, sa, sb,
                                               sink);
 }
 
@@ -869,11 +895,14 @@ __global__ void __launch_bounds__(kPathBlock) payoff_paths_kernel(const TaskDev 
     tables.fill();
     const TaskDev &t = *task;
     const StepConst<R> p = task_const<R>(t);
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < count;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    __shared__ uint4 s_rows[kPathBlock / 32][philox_rows<R, kBates>()];
+    const int lane = threadIdx.x & 31;
+    for (int64_t i0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x - lane; i0 < count;
+         i0 += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        const int64_t i = i0 + lane;
         PathState<R> st;
-        simulate_dispatch<R>(tables.get(), t, p, static_cast<uint32_t>(first + i), st, NoSink{});
-        out[i] = static_cast<double>(final_payoff<R>(t.pay[0], st.S, st.ssum, st.smax, st.smin, t.n_steps));
+        simulate_dispatch<R>(tables.get(), s_rows[threadIdx.x >> 5], t, p, static_cast<uint32_t>(first + i), st, NoSink{});
+        if (i < count) out[i] = static_cast<double>(final_payoff<R>(t.pay[0], st.S, st.ssum, st.smax, st.smin, t.n_steps));
     }
 }
 

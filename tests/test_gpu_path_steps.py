@@ -48,3 +48,48 @@ def test_fp64_spot_out_of_range_stays_ordered(qk, handle):
     legs = qk.price_plain(k, None, handle)["legs"]
     assert legs[0]["price"] == pytest.approx(100.0 * np.exp(-0.3), rel=1e-3)
     assert np.isfinite(legs[1]["price"])
+
+
+@pytest.mark.parametrize("model", [0, 1])
+def test_qe_with_a_reachable_clamp(qk, handle, oracle, model):
+    """Steps of five years with rho = 0.9: A a can pass 1/2, so min(A, 1/(2a) - eps) matters and
+    no step may take the clamp-free form.  FP64 paths against the oracle; FP32 with one and two
+    paths per lane simulates the same paths (prices to the rounding of the moment merge)."""
+    base = dict(model=model, scheme=qk.ANDERSEN_QE, v0=0.3, theta=0.3, kappa=0.1, sigma=0.5, rho=0.9, T=10.0, n_steps=2,
+                lambda_j=0.1 if model else 0.0, mu_j=-0.05, sigma_j=0.1, seed=9)
+    k = qk.make_contract(n_paths=500, precision=qk.FP64, **base)
+    Sg, _ = qk.paths(k, 0, 500, handle)
+    So, _ = oracle.paths(k, 0, 500)
+    np.testing.assert_allclose(Sg, So, rtol=1e-10)
+    c = qk.make_contract(n_paths=20_001, precision=qk.FP32, payoffs=[qk.payoff(qk.EUROPEAN, qk.PUT, 100.0)], **base)
+    out = []
+    try:
+        for lanes in (1, 2):
+            handle.tune_set(qk.FP32, model, qk.ANDERSEN_QE, 24, False, lanes)
+            out.append(qk.price_batch([c], None, handle)[0]["legs"][0]["price"])
+    finally:
+        handle.tune_reset()
+    assert out[0] == pytest.approx(out[1], rel=1e-12)
+
+
+@pytest.mark.parametrize("n_paths,n_steps", [(1, 1), (31, 63), (33, 64), (65, 65), (129, 130), (1000, 257)])
+@pytest.mark.parametrize("model,scheme", [(0, 0), (1, 0), (1, 2)])
+def test_generator_rows_at_warp_and_block_edges(qk, handle, oracle, model, scheme, n_paths, n_steps):
+    """Path counts around a warp's 32 lanes (one or two paths each) and step counts around the
+    64 steps a warp's generator rows cover: FP64 prices against the oracle's (1e-9, as the other
+    price checks), FP32 with one and two paths per lane alike (to the rounding of the merge)."""
+    base = dict(model=model, scheme=scheme, lambda_j=2.0 if model else 0.0, mu_j=-0.05, sigma_j=0.1, n_paths=n_paths,
+                n_steps=n_steps, seed=(5 << 32) + 7, stream=2 ** 32 - 1,
+                payoffs=[qk.payoff(qk.ASIAN, qk.CALL, 90.0), qk.payoff(qk.LOOKBACK_FLOATING, qk.PUT, 100.0)])
+    k = qk.make_contract(precision=qk.FP64, **base)
+    for got, want in zip(qk.price_batch([k], None, handle)[0]["legs"], oracle.price(k)["legs"]):
+        assert got["price"] == pytest.approx(want["price"], rel=1e-9, abs=1e-12)
+    c = qk.make_contract(precision=qk.FP32, **base)
+    out = []
+    try:
+        for lanes in (1, 2):
+            handle.tune_set(qk.FP32, model, scheme, 24, False, lanes)
+            out.append([leg["price"] for leg in qk.price_batch([c], None, handle)[0]["legs"]])
+    finally:
+        handle.tune_reset()
+    assert out[0] == pytest.approx(out[1], rel=1e-12, abs=1e-15)
