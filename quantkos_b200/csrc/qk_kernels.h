@@ -20,12 +20,12 @@ constexpr int kWarpTilePaths = 32;  // paths per round of a warp tile (one per l
 #endif
 constexpr int kPathMinBlocksFp32 = QK_PATH_MIN_BLOCKS_FP32;  // resident blocks per SM the FP32 path kernel is register-budgeted for
 
-// Resident 256-thread blocks per SM the FP64 path kernels are register-budgeted for: with
-// the one-path Euler kernel 2, 3 and 4 blocks measure 1287, 1291 and 1251 us
-// (1,048,576 x 252), with QE (12 pricings of 100,003 x 126, Asian) 2 and 3 blocks 2147 and
-// 2119 us: a few spilled registers against more warps to hide the FP64 latency.
-constexpr int kPathMinBlocks64 = 4;
-constexpr int kPathMinBlocksQe64 = 3;
+// Resident 256-thread blocks per SM the FP64 path kernels are register-budgeted for.
+// Cycles per path-step and scheduler at 1,048,576 x 252 with budgets for 4 (QE 3), 3 (2)
+// and 2 (4) blocks: Heston Euler European 163 / 164 / 168, Heston QE European 264 / 250 /
+// 265, Bates QE Asian 379 / 371 / 356 (QE in brackets throughout).
+constexpr int kPathMinBlocks64 = 3;
+constexpr int kPathMinBlocksQe64 = 2;
 
 // uniform_key: every task of the launch has Philox key `seed` (round keys go in the
 // kernel parameters); otherwise each task's key is read from its descriptor.

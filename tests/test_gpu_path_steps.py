@@ -93,3 +93,20 @@ def test_generator_rows_at_warp_and_block_edges(qk, handle, oracle, model, schem
     finally:
         handle.tune_reset()
     assert out[0] == pytest.approx(out[1], rel=1e-12, abs=1e-15)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("n_paths", [33, 4096, 150_000, 151_553, 400_000])
+def test_single_wave_launches_keep_the_bits(qk, handle, precision, n_paths):
+    """Path counts on both sides of the line below which every tile gets a resident warp of its
+    own (one-warp-per-scheduler blocks): the block size of persistent launches changes no bit."""
+    c = qk.make_contract(scheme=qk.ANDERSEN_QE, n_paths=n_paths, n_steps=8, seed=3, precision=precision,
+                         payoffs=[qk.payoff(qk.EUROPEAN, qk.CALL, 100.0), qk.payoff(qk.ASIAN, qk.CALL, 100.0)])
+    out = []
+    try:
+        for block in (128, 256):
+            handle.tune_set(precision, qk.HESTON, qk.ANDERSEN_QE, 24, False, 2 if precision else 1, block_size=block)
+            out.append(qk.price_batch([c], None, handle)[0]["legs"])
+    finally:
+        handle.tune_reset()
+    assert out[0] == out[1]
