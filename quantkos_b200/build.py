@@ -37,7 +37,8 @@ NVCC = os.environ.get("NVCC", shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++20", "-Xcompiler", "-fPIC", "-Xcompiler", "-O3",
                      "-Xptxas", "-O3", "--expt-relaxed-constexpr"]
-SOURCES = ["qk_paths.cu", "qk_lsm.cu", "qk_api.cu", "qk_serve.cu", "qk_config.cu", "qk_tune.cu", "qk_noalloc.cu"]
+SOURCES = ["qk_paths.cu", "qk_lsm.cu", "qk_api.cu", "qk_serve.cu", "qk_config.cu", "qk_tune.cu", "qk_noalloc.cu",
+           "qk_select.cu"]
 
 
 def _run(cmd: list[str], cwd: Path | None = None) -> None:

@@ -729,8 +729,10 @@ qk_status assemble_results(qk_handle *h, const Plan &plan, const Moments *task_m
     return QK_OK;
 }
 
-// Leg-0 payoffs (undiscounted, normalised units) of paths first .. first + count - 1.
-qk_status payoffs_range(qk_handle *h, const qk_contract &c, int64_t first, int64_t count, double *out) {
+// Leg-0 payoffs (undiscounted, normalised units) of paths first .. first + count - 1 into
+// the handle's trace arena, after `head` bytes that the caller uses itself.
+static qk_status payoffs_on_device(qk_handle *h, const qk_contract &c, int64_t first, int64_t count, size_t head,
+                                   double **out) {
     qk_status s = validate_contract(c, nullptr);
     if (s != QK_OK) return s;
     if (c.antithetic) return fail(QK_ERR_UNSUPPORTED, "per-path payoffs of antithetic pairs are not dumped");
@@ -739,20 +741,40 @@ qk_status payoffs_range(qk_handle *h, const qk_contract &c, int64_t first, int64
     double scale = 1.0;
     const qk_contract n = normalised(c, &scale);
     const TaskDev t = make_task(n, 1);
-    const size_t head = ((sizeof(TaskDev) + 255) / 256) * 256;
-    if ((s = h->d_trace.ensure(head + static_cast<size_t>(count) * sizeof(double))) != QK_OK) return s;
-    TaskDev *dt = static_cast<TaskDev *>(h->d_trace.ptr);
-    double *dp = reinterpret_cast<double *>(static_cast<char *>(h->d_trace.ptr) + head);
+    const size_t task_bytes = ((sizeof(TaskDev) + 255) / 256) * 256;
+    if ((s = h->d_trace.ensure(head + task_bytes + static_cast<size_t>(count) * sizeof(double))) != QK_OK) return s;
+    char *base = static_cast<char *>(h->d_trace.ptr);
+    TaskDev *dt = reinterpret_cast<TaskDev *>(base + head);
+    *out = reinterpret_cast<double *>(base + head + task_bytes);
     QK_CUDA_TRY(cudaMemcpyAsync(dt, &t, sizeof(TaskDev), cudaMemcpyHostToDevice, h->stream));
-    QK_CUDA_TRY(launch_payoff_paths(c.precision == QK_FP32 ? QK_FP32 : QK_FP64, h->stream, dt, first, count, dp));
+    const bool reads_state = n.payoffs[0].type >= QK_ASIAN && n.payoffs[0].type <= QK_LOOKBACK_FIXED;
+    QK_CUDA_TRY(launch_payoff_paths(c.precision == QK_FP32 ? QK_FP32 : QK_FP64, n.model, n.scheme, reads_state, n.seed,
+                                    h->sm_count, h->stream, dt, first, count, *out));
+    return QK_OK;
+}
+
+qk_status payoffs_range(qk_handle *h, const qk_contract &c, int64_t first, int64_t count, double *out) {
+    double *dp = nullptr;
+    const qk_status s = payoffs_on_device(h, c, first, count, 0, &dp);
+    if (s != QK_OK) return s;
     QK_CUDA_TRY(cudaMemcpyAsync(out, dp, static_cast<size_t>(count) * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     QK_CUDA_TRY(cudaStreamSynchronize(h->stream));
     return QK_OK;
 }
 
-qk_status payoffs_dump(qk_handle *h, const qk_contract &c, std::vector<double> &out) {
-    out.resize(static_cast<size_t>(c.n_paths));
-    return payoffs_range(h, c, 0, c.n_paths, out.data());
+qk_status payoff_order_statistics(qk_handle *h, const qk_contract &c, const SelectRanks &ranks, int n_ranks,
+                                  double *out) {
+    const size_t scratch = select_scratch_bytes();
+    const size_t head = scratch + 256;  // the selection's state, then its results
+    double *dp = nullptr;
+    const qk_status s = payoffs_on_device(h, c, 0, c.n_paths, head, &dp);
+    if (s != QK_OK) return s;
+    char *base = static_cast<char *>(h->d_trace.ptr);
+    double *dr = reinterpret_cast<double *>(base + scratch);
+    QK_CUDA_TRY(launch_select(h->stream, h->sm_count, dp, c.n_paths, ranks, n_ranks, base, dr));
+    QK_CUDA_TRY(cudaMemcpyAsync(out, dr, static_cast<size_t>(n_ranks) * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    QK_CUDA_TRY(cudaStreamSynchronize(h->stream));
+    return QK_OK;
 }
 
 qk_status finish_timing(qk_handle *h, double path_steps) {
@@ -831,6 +853,7 @@ qk_status qk_create(int32_t device, qk_handle **out) {
         if (device < 64 && !loaded[device]) {
             cudaError_t e = preload_path_kernels();
             if (e == cudaSuccess) e = preload_lsm_kernels();
+            if (e == cudaSuccess) e = preload_select_kernels();
             if (e != cudaSuccess) return fail(QK_ERR_CUDA, std::string("loading the kernels: ") + cudaGetErrorString(e));
             loaded[device] = true;
         }

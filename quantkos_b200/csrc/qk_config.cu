@@ -530,17 +530,16 @@ qk_status qk_run_config(qk_handle *h, const qk_config *cfg, qk_result *out, doub
         if (st != QK_OK) return st;
     }
     if (c.analyze_distribution && pct && k.payoffs[0].type != QK_AMERICAN) {
-        // OptionPricer::analyze_risk_neutral_discounted_payoff_distribution: sort all payoffs,
-        // read 15 order statistics, apply discount and scale.
-        std::vector<double> pay;
-        QK_TRY(qk::payoffs_dump(h, k, pay));
-        std::sort(pay.begin(), pay.end());
-        const double N = static_cast<double>(pay.size());
+        // OptionPricer::analyze_risk_neutral_discounted_payoff_distribution: 15 order statistics
+        // of all payoffs, discount and scale applied.
+        const double N = static_cast<double>(k.n_paths);
         const double eff = std::exp(-k.r * k.T) * ((k.payoffs[0].type == QK_BINARY_CASH) ? 1.0 : scale);
         const double fr[13] = {0.01, 0.05, 0.10, 0.20, 0.30, 0.40, 0.50, 0.60, 0.70, 0.80, 0.90, 0.95, 0.99};
-        pct[0] = pay.front() * eff;
-        for (int i = 0; i < 13; ++i) pct[i + 1] = pay[static_cast<size_t>(N * fr[i])] * eff;
-        pct[14] = pay.back() * eff;
+        qk::SelectRanks ranks = {};
+        for (int i = 0; i < 13; ++i) ranks.r[i + 1] = static_cast<size_t>(N * fr[i]);
+        ranks.r[14] = static_cast<size_t>(k.n_paths) - 1;
+        QK_TRY(qk::payoff_order_statistics(h, k, ranks, 15, pct));
+        for (int i = 0; i < 15; ++i) pct[i] *= eff;
     }
     return QK_OK;
 }

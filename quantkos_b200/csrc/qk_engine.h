@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "qk_internal.h"
+#include "qk_kernels.h"
 
 namespace qk {
 
@@ -147,8 +148,9 @@ qk_status pool_reserve(int device, cudaStream_t s, size_t bytes);
 void pool_release(int device, size_t bytes);
 void pool_trim(int device);
 
-// Every path's leg-0 payoff (undiscounted, normalised) of a contract, on the host.
-qk_status payoffs_dump(qk_handle *h, const qk_contract &c, std::vector<double> &out);
+// Order statistics of a contract's leg-0 payoffs (undiscounted, normalised) over its
+// paths: the values of n_ranks ascending ranks, selected on the device.
+qk_status payoff_order_statistics(qk_handle *h, const qk_contract &c, const SelectRanks &ranks, int n_ranks, double *out);
 qk_status payoffs_range(qk_handle *h, const qk_contract &c, int64_t first, int64_t count, double *out);
 
 // Longstaff-Schwartz for the American contracts of a plan (qk_lsm.cu).

@@ -53,8 +53,19 @@ cudaError_t launch_slab_paths(int precision, int model, int scheme, uint64_t see
 cudaError_t launch_step_trace(int precision, cudaStream_t s, const TaskDev *task, const double *z, const double *u,
                               int umax, int n, double *S_out, double *v_out, int *status);
 // Leg-0 payoffs of paths first .. first + count - 1 of the task (undiscounted, normalised).
-cudaError_t launch_payoff_paths(int precision, cudaStream_t s, const TaskDev *task, int64_t first, int64_t count,
-                                double *out);
+// track: the leg reads the path state.
+cudaError_t launch_payoff_paths(int precision, int model, int scheme, bool track, uint64_t seed, int sm_count,
+                                cudaStream_t s, const TaskDev *task, int64_t first, int64_t count, double *out);
+// Order statistics: the values of ascending ranks r[0..n_ranks-1] (0 = smallest) of x[0..n-1],
+// n < 2^32, into out[n_ranks] (device); scratch holds select_scratch_bytes().
+constexpr int kSelectRanks = 16;
+struct SelectRanks {
+    unsigned long long r[kSelectRanks];
+};
+size_t select_scratch_bytes();
+cudaError_t launch_select(cudaStream_t s, int sm_count, const double *x, int64_t n, const SelectRanks &ranks, int n_ranks,
+                          void *scratch, double *out);
+cudaError_t preload_select_kernels();
 // One leg's payoff on the fed spot sequence S[0..n-1] starting from S0 (one thread).
 cudaError_t launch_payoff_trace(int precision, cudaStream_t s, const PayoffSpec &ps, const double *S, int n, double S0,
                                 double *out);

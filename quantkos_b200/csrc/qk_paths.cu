@@ -4,6 +4,8 @@
 // the path dump, and the fed-draw parity trace.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "qk_device.cuh"
 #include "qk_kernels.h"
 
@@ -99,6 +101,8 @@ struct SlabSink2 {
 // Steps are taken in chunks of kSumChunk; the Asian running sum is accumulated in
 // the working precision inside a chunk and folded into the FP64 sum after it.
 constexpr int kSumChunk = 16;
+
+constexpr int kPayoffBlock = 128;  // threads per block of the per-path payoff kernel
 
 template <class R>
 __device__ __forceinline__ void track(PathState<R> &st, R &blk) {
@@ -494,23 +498,6 @@ __device__ __forceinline__ uint32_t task_kmin(const TaskDev &t) {
     return sizeof(R) == 4 ? t.jump_kmin : t.jump_kmin64;
 }
 
-template <class R, class Sink>
-__device__ __forceinline__ void simulate_dispatch(const Tab64 *tab, uint4 *rows, const TaskDev &t,
-                                                  const StepConst<R> &p, uint32_t path, PathState<R> &st, Sink &&sink) {
-    const R S0 = static_cast<R>(t.S0);
-    const R v0 = static_cast<R>(t.v0);
-    const uint32_t km = task_kmin<R>(t);
-    const WarpPhilox<philox_rows<R, kBates>(), RegKeys> g{RegKeys{t.key0, t.key1}, rows, t.stream};
-    switch (t.model * 3 + t.scheme) {
-        case 0: simulate_path<R, kHeston, kEuler>(tab, p, S0, v0, t.n_steps, g, t.key0, t.key1, path, t.stream, km, st, sink); break;
-        case 1: simulate_path<R, kHeston, kMilstein>(tab, p, S0, v0, t.n_steps, g, t.key0, t.key1, path, t.stream, km, st, sink); break;
-        case 2: simulate_path<R, kHeston, kQE>(tab, p, S0, v0, t.n_steps, g, t.key0, t.key1, path, t.stream, km, st, sink); break;
-        case 3: simulate_path<R, kBates, kEuler>(tab, p, S0, v0, t.n_steps, g, t.key0, t.key1, path, t.stream, km, st, sink); break;
-        case 4: simulate_path<R, kBates, kMilstein>(tab, p, S0, v0, t.n_steps, g, t.key0, t.key1, path, t.stream, km, st, sink); break;
-        default: simulate_path<R, kBates, kQE>(tab, p, S0, v0, t.n_steps, g, t.key0, t.key1, path, t.stream, km, st, sink); break;
-    }
-}
-
 // ----------------------------------------------------------------------------
 // Fused pricing kernel.  Persistent: each warp pops queue slots from a device
 // cursor; slot q belongs to the task whose tile range [tile_begin, tile_begin +
@@ -888,21 +875,46 @@ SlabKernel<R> slab_kernel_for(int model, int scheme) {
 
 // Per-path payoff of leg 0 (undiscounted, normalised units), for the payoff
 // distribution analysis (OptionPricer.hpp:340-360 sorts every path's payoff).
-template <class R>
-__global__ void __launch_bounds__(kPathBlock) payoff_paths_kernel(const TaskDev *__restrict__ task, int64_t first,
-                                                                 int64_t count, double *__restrict__ out) {
+template <class R, int MODEL, int SCHEME, bool TRK>
+__global__ void __launch_bounds__(kPayoffBlock, 2 * (sizeof(R) == 4 ? kPathMinBlocksFp32
+                                                     : SCHEME == kQE ? kPathMinBlocksQe64 : kPathMinBlocks64))
+    payoff_paths_kernel(const TaskDev *__restrict__ task, int64_t first, int64_t count, double *__restrict__ out,
+                        const PhiloxRoundKeys rk) {
     __shared__ BlockTables<R> tables;
     tables.fill();
     const TaskDev &t = *task;
     const StepConst<R> p = task_const<R>(t);
-    __shared__ uint4 s_rows[kPathBlock / 32][philox_rows<R, kBates>()];
+    constexpr int kRows = philox_rows<R, MODEL>();
+    __shared__ uint4 s_rows[kPayoffBlock / 32][kRows];
+    const WarpPhilox<kRows, ParamKeys> gen{ParamKeys{rk}, s_rows[threadIdx.x >> 5], t.stream};
     const int lane = threadIdx.x & 31;
     for (int64_t i0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x - lane; i0 < count;
          i0 += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         const int64_t i = i0 + lane;
+        const uint32_t path = static_cast<uint32_t>(first + i);
         PathState<R> st;
-        simulate_dispatch<R>(tables.get(), s_rows[threadIdx.x >> 5], t, p, static_cast<uint32_t>(first + i), st, NoSink{});
+        if constexpr (sizeof(R) == 8)
+            simulate_path<R, MODEL, SCHEME, TRK>(tables.get(), p, t.S0, t.v0, t.n_steps, gen, t.key0, t.key1, path, t.stream,
+                                                 t.jump_kmin64, st, NoSink{});
+        else
+            simulate_path<R, MODEL, SCHEME, TRK>(tables.get(), p, static_cast<R>(t.S0), static_cast<R>(t.v0), t.n_steps, gen,
+                                                 t.key0, t.key1, path, t.stream, t.jump_kmin, st, NoSink{});
         if (i < count) out[i] = static_cast<double>(final_payoff<R>(t.pay[0], st.S, st.ssum, st.smax, st.smin, t.n_steps));
+    }
+}
+
+template <class R>
+using PayoffKernel = void (*)(const TaskDev *, int64_t, int64_t, double *, const PhiloxRoundKeys);
+
+template <class R, bool TRK>
+PayoffKernel<R> payoff_kernel_for(int model, int scheme) {
+    switch (model * 3 + scheme) {
+        case 0: return payoff_paths_kernel<R, kHeston, kEuler, TRK>;
+        case 1: return payoff_paths_kernel<R, kHeston, kMilstein, TRK>;
+        case 2: return payoff_paths_kernel<R, kHeston, kQE, TRK>;
+        case 3: return payoff_paths_kernel<R, kBates, kEuler, TRK>;
+        case 4: return payoff_paths_kernel<R, kBates, kMilstein, TRK>;
+        default: return payoff_paths_kernel<R, kBates, kQE, TRK>;
     }
 }
 
@@ -1037,13 +1049,15 @@ cudaError_t launch_step_trace(int precision, cudaStream_t s, const TaskDev *task
     return cudaGetLastError();
 }
 
-cudaError_t launch_payoff_paths(int precision, cudaStream_t s, const TaskDev *task, int64_t first, int64_t count,
-                                double *out) {
-    const int64_t blocks = (count + kPathBlock - 1) / kPathBlock;
-    if (precision == QK_FP32)
-        payoff_paths_kernel<float><<<static_cast<unsigned>(blocks), kPathBlock, 0, s>>>(task, first, count, out);
-    else
-        payoff_paths_kernel<double><<<static_cast<unsigned>(blocks), kPathBlock, 0, s>>>(task, first, count, out);
+cudaError_t launch_payoff_paths(int precision, int model, int scheme, bool track, uint64_t seed, int sm_count,
+                                cudaStream_t s, const TaskDev *task, int64_t first, int64_t count, double *out) {
+    const PhiloxRoundKeys rk = philox_round_keys(static_cast<uint32_t>(seed & 0xFFFFFFFFull),
+                                                 static_cast<uint32_t>(seed >> 32));
+    const int64_t blocks = (count + kPayoffBlock - 1) / kPayoffBlock;
+    const unsigned grid = static_cast<unsigned>(std::min<int64_t>(blocks, static_cast<int64_t>(sm_count) * 8));
+    const auto launch = [&](auto kernel) { kernel<<<grid, kPayoffBlock, 0, s>>>(task, first, count, out, rk); };
+    if (precision == QK_FP32) launch(track ? payoff_kernel_for<float, true>(model, scheme) : payoff_kernel_for<float, false>(model, scheme));
+    else launch(track ? payoff_kernel_for<double, true>(model, scheme) : payoff_kernel_for<double, false>(model, scheme));
     return cudaGetLastError();
 }
 
@@ -1099,8 +1113,9 @@ static cudaError_t preload_path_kernels_of() {
                         e = cudaFuncGetAttributes(&fa, price_kernel_for<R>(model, scheme, uk != 0, lane, trk != 0));
             if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, slab_kernel_for<R>(model, scheme));
             if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, slab_two_kernel_for(model, scheme));
+            if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, payoff_kernel_for<R, true>(model, scheme));
+            if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, payoff_kernel_for<R, false>(model, scheme));
         }
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, payoff_paths_kernel<R>);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, payoff_trace_kernel<R>);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, step_trace_kernel<R>);
     return e;
