@@ -204,6 +204,27 @@ static bool needs_path_state(const qk_contract &c) {
     return false;
 }
 
+// The floats 1 - 2 A a can take on a QE step in the plain form of the quadratic regime:
+// a = h / (m + G) with h / m a mediant of two fixed ratios (see make_step_const) and G
+// between m sqrt(1 - psi_c / 2) and m, so between two bounds that do not depend on the
+// variance, with eight floats of room on each side for rounding (a term outside takes the
+// step's general code, so the bounds decide speed, not results).  A daily step leaves a few
+// thousand; none where there are more than kTermTableMax.
+static uint32_t term_range_lo(const StepConst<float> &c) {
+    if (!(c.h_psi_plain > 0.0f)) return 0;
+    const double r1 = static_cast<double>(c.h_f1) / c.exp_mkdt;
+    const double r2 = c.theta_m > 0.0f ? static_cast<double>(c.h_f2) / c.theta_m : r1;
+    const double a_lo = 0.5 * std::min(r1, r2);
+    const double a_hi = std::max(r1, r2) / (1.0 + std::sqrt(std::max(0.0, 1.0 - 0.5 * c.psi_c)));
+    const float t0 = static_cast<float>(1.0 - c.two_A * a_lo), t1 = static_cast<float>(1.0 - c.two_A * a_hi);
+    const float f0 = std::min(t0, t1), f1 = std::max(t0, t1);
+    if (!(f0 > 1e-3f && f1 < 1e3f)) return 0;
+    uint32_t b0, b1;
+    std::memcpy(&b0, &f0, 4);
+    std::memcpy(&b1, &f1, 4);
+    return b1 - b0 + 17u <= kTermTableMax ? b0 - 8u : 0;
+}
+
 TaskDev make_task(const qk_contract &b, int ppt, int lane_mode) {
     TaskDev t;
     std::memset(&t, 0, sizeof(t));
@@ -226,6 +247,7 @@ TaskDev make_task(const qk_contract &b, int ppt, int lane_mode) {
     const float Lf = t.cf.exp_m_lambda_dt;
     const double kd = std::ceil(static_cast<double>(Lf) * 8388608.0 - 0.5);
     t.jump_kmin = static_cast<uint32_t>(std::min(std::max(kd, 0.0), 8388608.0));
+    if (b.scheme == QK_ANDERSEN_QE) t.term_lo = term_range_lo(t.cf);
     // FP64: (w + 1/2) 2^-32 >= L  <=>  w >= ceil(L 2^32 - 1/2) (both exact); capped, so that at
     // L = 1 the largest word still reaches the exact test
     t.jump_kmin64 = static_cast<uint32_t>(
@@ -285,15 +307,17 @@ static double step_cost(const TaskDev &t) {
 // of 512 threads, 64 us with blocks of 128).
 struct LaunchShape {
     int grid, block;
+    bool table;  // a persistent launch of one FP32 QE task: its SFU results from a table (TermTable)
 };
-static LaunchShape launch_shape(const qk_handle *h, const TaskDev &t, int64_t slots, int block) {
+static LaunchShape launch_shape(const qk_handle *h, const TaskDev &t, size_t n_tasks, int64_t slots, int block) {
     const int single = 128;
     const int64_t per_sm =
         price_tiles_max_blocks_per_sm(t.precision, t.model, t.scheme, t.lane_mode, t.track != 0, single);
     if (slots <= h->sm_count * per_sm * (single / 32))
-        return LaunchShape{static_cast<int>((slots + single / 32 - 1) / (single / 32)), single};
+        return LaunchShape{static_cast<int>((slots + single / 32 - 1) / (single / 32)), single, false};
     const int n = price_tiles_max_blocks_per_sm(t.precision, t.model, t.scheme, t.lane_mode, t.track != 0, block);
-    return LaunchShape{static_cast<int>(std::min<int64_t>(slots, static_cast<int64_t>(h->sm_count) * n)), block};
+    const bool table = n_tasks == 1 && price_tiles_takes_table(t, block);
+    return LaunchShape{static_cast<int>(std::min<int64_t>(slots, static_cast<int64_t>(h->sm_count) * n)), block, table};
 }
 
 // The plain method's launch shape (one task per launch; not tuned).
@@ -550,7 +574,7 @@ static qk_status enqueue_plan(qk_handle *h, const Plan &plan, bool capture) {
         // a bump's launch fills the SMs the one before it leaves idle at its end
         for (size_t i = 0; i < nt; ++i) {
             const TaskDev &t = plan.tasks[i];
-            const LaunchShape shape = launch_shape(h, t, t.n_tiles, kPathBlock);
+            const LaunchShape shape = launch_shape(h, t, 1, t.n_tiles, kPathBlock);
             // one task: its own queue cursor, its own tile range (prefix of one task = itself)
             const uint64_t seed = static_cast<uint64_t>(t.key0) | (static_cast<uint64_t>(t.key1) << 32);
             QK_CUDA_TRY(launch_price_tiles(t.precision, t.model, t.scheme, shape.grid,
@@ -571,7 +595,7 @@ static qk_status enqueue_plan(qk_handle *h, const Plan &plan, bool capture) {
                 ++e;
             const int64_t slots_end = plan.tasks[e - 1].tile_begin + plan.tasks[e - 1].n_tiles;
             const int64_t slots = slots_end - tb.tile_begin;
-            const LaunchShape shape = launch_shape(h, tb, slots, h->tune_block[tb.precision][tb.model][tb.scheme]);
+            const LaunchShape shape = launch_shape(h, tb, e - b, slots, h->tune_block[tb.precision][tb.model][tb.scheme]);
             bool uniform_key = true;
             for (size_t i = b; i < e; ++i)
                 uniform_key &= plan.tasks[i].key0 == tb.key0 && plan.tasks[i].key1 == tb.key1;
@@ -579,7 +603,7 @@ static qk_status enqueue_plan(qk_handle *h, const Plan &plan, bool capture) {
             cudaStream_t ks = n_streams > 1 ? h->kind_stream[kind % n_streams] : h->stream;
             QK_CUDA_TRY(launch_price_tiles(tb.precision, tb.model, tb.scheme, shape.grid, ks, dt + b, dp + b,
                                            static_cast<int32_t>(e - b), tb.tile_begin, slots_end, dc + b, dpart,
-                                           uniform_key, seed, tb.lane_mode, tb.track, shape.block));
+                                           uniform_key, seed, tb.lane_mode, tb.track, shape.block, shape.table));
             h->launches++;
             ++kind;
             b = e;
@@ -1100,7 +1124,8 @@ qk_status qk_paths_dump(qk_handle *h, const qk_contract *c, int64_t first, int64
     char *dS = base + ((sizeof(TaskDev) + 255) / 256) * 256;
     char *dv = dS + cells * esz;
     QK_CUDA_TRY(cudaMemcpyAsync(dt, &t, sizeof(TaskDev), cudaMemcpyHostToDevice, h->stream));
-    QK_CUDA_TRY(launch_slab_paths(prec, n.model, n.scheme, n.seed, h->stream, dt, first, count, 1, dS, dv, count));
+    QK_CUDA_TRY(launch_slab_paths(prec, n.model, n.scheme, n.seed, h->stream, dt, first, count, 1, dS, dv, count,
+                                  h->sm_count));
     std::vector<char> hS(cells * esz), hv(cells * esz);
     QK_CUDA_TRY(cudaMemcpyAsync(hS.data(), dS, cells * esz, cudaMemcpyDeviceToHost, h->stream));
     QK_CUDA_TRY(cudaMemcpyAsync(hv.data(), dv, cells * esz, cudaMemcpyDeviceToHost, h->stream));

@@ -424,16 +424,40 @@ __device__ __forceinline__ float2 lg2_2(float2 x) { return make_float2(ptx_lg2(x
 __device__ __forceinline__ float2 ex2_2(float2 x) { return make_float2(ptx_ex2(x.x), ptx_ex2(x.y)); }
 __device__ __forceinline__ float2 max0_2(float2 a) { return make_float2(fmaxf(a.x, 0.0f), fmaxf(a.y, 0.0f)); }
 
+// Where the paired QE step takes 1 / term and log2 term from, term = 1 - 2 A a: the SFU, or
+// a shared-memory table of the SFU's results for every float of the task's range
+// [lo, lo + n) of bit patterns (term moves by a few hundred millionths, so at daily steps
+// that is a few thousand floats).  The same bits for two of the step's twelve SFU
+// operations less, on the unit that bounds QE: five-payoff Bates QE, 16,777,216 x 252,
+// 14.00 -> 13.41 ms; Heston QE Asian, 5,000,000 x 365, 5.62 -> 5.33 ms.
+struct TermSfu {
+    static constexpr bool kTable = false;
+};
+struct TermTable {
+    static constexpr bool kTable = true;
+    const float2 *tab;  // kTermTableMax + 1 entries; the last one stands for all terms beyond
+    uint32_t lo;
+    __device__ __forceinline__ static TermTable fill(float2 *tab, uint32_t lo) {
+        for (uint32_t i = threadIdx.x; i <= kTermTableMax; i += blockDim.x) {
+            const float x = __uint_as_float(lo + i);
+            tab[i] = make_float2(ptx_rcp(x), ptx_lg2(x));
+        }
+        __syncthreads();
+        return TermTable{tab, lo};
+    }
+};
+
 // QE step of two paths (spot S, variance v as pairs): paired when both take the
 // quadratic branch (the common case), otherwise each path through step_qe_f32.
-__device__ __forceinline__ void step_qe_two_f32(const StepConst<float> &p, float2 &S, float2 &v, float2 Zv,
-                                                float2 Zind) {
+template <class Term>
+__device__ __forceinline__ void step_qe_two_f32(const Term &tt, const StepConst<float> &p, float2 &S, float2 &v,
+                                                float2 Zv, float2 Zind) {
     const float2 m = __ffma2_rn(v, f2(p.exp_mkdt), f2(p.theta_m));
     const float2 h = __ffma2_rn(v, f2(p.h_f1), f2(p.h_f2));  // s^2 / 2
     const float2 m2 = __fmul2_rn(m, m);
     const float2 em2 = __fmul2_rn(f2(p.h_eps), m2);
     const float2 pm2 = __fmul2_rn(f2(p.h_psi_plain), m2);
-    const bool quad = m.x > p.eps && m.y > p.eps && h.x > em2.x && h.y > em2.y && h.x <= pm2.x && h.y <= pm2.y;
+    bool quad = m.x > p.eps && m.y > p.eps && h.x > em2.x && h.y > em2.y && h.x <= pm2.x && h.y <= pm2.y;
     // the quadratic form for both paths first (no branch before the long SFU chain);
     // a pair not both in the quadratic regime is redone per path below
     const float2 S_old = S, v_old = v;
@@ -447,8 +471,18 @@ __device__ __forceinline__ void step_qe_two_f32(const StepConst<float> &p, float
     const float2 vn = __fmul2_rn(__fmul2_rn(a, bz), bz);
     const float2 Aa = __fmul2_rn(f2(p.A), a);
     const float2 term = __ffma2_rn(f2(-2.0f), Aa, f2(1.0f));
-    const float2 logM = __ffma2_rn(__fmul2_rn(Aa, b2), rcp2(term),
-                                   __fmul2_rn(f2(-0.5f * Math<float>::kLn2), lg2_2(term)));
+    float2 rterm, lterm;
+    if constexpr (Term::kTable) {
+        const uint32_t ia = __float_as_uint(term.x) - tt.lo, ib = __float_as_uint(term.y) - tt.lo;
+        quad = quad && ia < kTermTableMax && ib < kTermTableMax;
+        const float2 ta = tt.tab[min(ia, kTermTableMax)], tb = tt.tab[min(ib, kTermTableMax)];
+        rterm = make_float2(ta.x, tb.x);
+        lterm = make_float2(ta.y, tb.y);
+    } else {
+        rterm = rcp2(term);
+        lterm = lg2_2(term);
+    }
+    const float2 logM = __ffma2_rn(__fmul2_rn(Aa, b2), rterm, __fmul2_rn(f2(-0.5f * Math<float>::kLn2), lterm));
     // qe_spot_f32, paired
     const float2 K0n = __ffma2_rn(f2(p.K1_half_K3), v, logM);
     const float2 isig = __ffma2_rn(f2(p.K3), v, __fmul2_rn(f2(p.K4), vn));

@@ -36,6 +36,11 @@ enum : int {
 };
 enum : int { kCall = 0, kPut = 1 };
 
+// Floats a term table of the FP32 QE kernels covers (TaskDev::term_lo): 48 KB, so that two
+// resident 512-thread blocks of the pricing kernel or four 256-thread blocks of the slab
+// kernel fit an SM.
+constexpr uint32_t kTermTableMax = 6144;
+
 // Bound on Knuth's Poisson loop per step (the reference loops without bound);
 // validation rejects lambda*dt > kMaxLambdaDt so the bound is never reached in practice.
 constexpr int kMaxJumpsPerStep = 4096;
@@ -81,6 +86,7 @@ struct TaskDev {
     uint32_t key0, key1;   // Philox key = seed
     uint32_t stream;       // Philox counter word 2 (common random numbers across bumps)
     uint32_t jump_kmin;    // FP32 jump test: a step jumps iff (first Poisson word >> 9) >= jump_kmin
+    uint32_t term_lo;      // FP32 QE: least float (bit pattern) that 1 - 2 A a can take; 0: too many for a table
     uint32_t jump_kmin64;  // FP64: a first Poisson word below this cannot jump (exact test beyond it)
     int64_t n_paths;
     int64_t tile_begin;    // first queue slot of the task (tiles of a task are consecutive)

@@ -35,7 +35,10 @@ constexpr int kPathMinBlocksQe64 = 2;
 cudaError_t launch_price_tiles(int precision, int model, int scheme, int grid, cudaStream_t s, const TaskDev *tasks,
                                const int64_t *prefix, int32_t n_tasks, int64_t slot_begin, int64_t slot_end,
                                unsigned long long *cursor, Moments *partials, bool uniform_key, uint64_t seed,
-                               int lane_mode = kLaneOne, bool track = true, int block = kPathBlock);
+                               int lane_mode = kLaneOne, bool track = true, int block = kPathBlock,
+                               bool table = false);
+// Whether a launch of this one task in blocks of `block` threads may use its term table.
+bool price_tiles_takes_table(const TaskDev &t, int block);
 // max_tiles: the largest n_tiles among the tasks (sets the block width).
 cudaError_t launch_merge_tasks(int n_tasks, cudaStream_t s, const TaskDev *tasks, const Moments *partials,
                                TaskMoments *out, int64_t max_tiles = 0);
@@ -47,9 +50,10 @@ constexpr int kMergeChunkTiles = 512;
 cudaError_t launch_merge_two_level(int n_tasks, int64_t n_chunks, cudaStream_t s, const TaskDev *tasks,
                                    const Moments *partials, Moments *chunks, TaskMoments *out);
 // paths_per_thread 2: each thread simulates two consecutive paths (same values).
+// has_table: the task has a term table (TaskDev::term_lo; two paths per thread only).
 cudaError_t launch_slab_paths(int precision, int model, int scheme, uint64_t seed, cudaStream_t s, const TaskDev *task,
                               int64_t first_path, int64_t count, int stride, void *slab_S, void *slab_v, int64_t ld,
-                              int paths_per_thread = 1);
+                              int sm_count, int paths_per_thread = 1, bool has_table = false);
 cudaError_t launch_step_trace(int precision, cudaStream_t s, const TaskDev *task, const double *z, const double *u,
                               int umax, int n, double *S_out, double *v_out, int *status);
 // Leg-0 payoffs of paths first .. first + count - 1 of the task (undiscounted, normalised).

@@ -1240,7 +1240,8 @@ qk_status run_lsm_contracts(qk_handle *h, Plan &plan, bool plain, std::vector<Mo
         // FP32: two paths per thread, stepped as pairs
         QK_CUDA_LSM(launch_slab_paths(prec, b.model, b.scheme, b.seed, s,
                                       static_cast<const TaskDev *>(h->lsm_task.ptr) + k, 0, b.n_paths, stride,
-                                      L.slab_S.ptr, use_v ? L.slab_v.ptr : nullptr, ld, prec == QK_FP32 ? 2 : 1));
+                                      L.slab_S.ptr, use_v ? L.slab_v.ptr : nullptr, ld, h->sm_count,
+                                      prec == QK_FP32 ? 2 : 1, tasks[k].term_lo != 0));
         h->lsm_launches++;
         QK_CUDA_LSM(cudaEventRecord(h->lsm_events[3 * k + 1], s));
         LsmArgs a;

@@ -53,17 +53,14 @@ struct SlabSink {
     int64_t pos;    // slab index of this path's next stored date: row * ld + column
     int stride;     // steps between stored dates
     int left;       // steps until the next stored date
-    bool has;       // the path exists (a warp's lanes beyond the last path store nothing)
     // Called once per step, in order: every stride-th step is stored.
     template <class Spot>
     __device__ __forceinline__ void operator()(int, Spot spot, R v) {
         if (--left == 0) {
             left = stride;
-            if (has) {
-                if constexpr (sizeof(R) == 8) slab_S[pos] = spot();
-                else slab_S[pos] = spot;
-                if (slab_v) slab_v[pos] = v;
-            }
+            if constexpr (sizeof(R) == 8) slab_S[pos] = spot();
+            else slab_S[pos] = spot;
+            if (slab_v) slab_v[pos] = v;
             pos += ld;
         }
     }
@@ -83,14 +80,14 @@ struct SlabSink2 {
     int64_t pos;   // slab index of path a's next stored date; path b is the next column
     int stride;
     int left;
-    bool has_a, has_b;
+    bool has_b;
     __device__ __forceinline__ void operator()(int, R Sa, R va, R Sb, R vb) {
         if (--left == 0) {
             left = stride;
-            if (has_a) slab_S[pos] = Sa;
+            slab_S[pos] = Sa;
             if (has_b) slab_S[pos + 1] = Sb;
             if (slab_v) {
-                if (has_a) slab_v[pos] = va;
+                slab_v[pos] = va;
                 if (has_b) slab_v[pos + 1] = vb;
             }
             pos += ld;
@@ -378,13 +375,13 @@ __device__ __forceinline__ void jumps_two(const StepConst<float> &p, PathState<f
 
 // One FP32 step of a lane's two paths from their normals (the paired scheme step, then
 // the jumps).
-template <int MODEL, int SCHEME, bool NEG>
-__device__ __forceinline__ void step_two_z_f32(const StepConst<float> &p, PathState<float> &a, PathState<float> &b,
-                                               float2 Z1, float2 Z2, uint32_t pois_a, uint32_t pois_b, uint32_t kmin,
-                                               uint32_t k0, uint32_t k1, uint32_t path_a, uint32_t path_b,
-                                               uint32_t stream, int n) {
+template <int MODEL, int SCHEME, bool NEG, class Term>
+__device__ __forceinline__ void step_two_z_f32(const Term &tt, const StepConst<float> &p, PathState<float> &a,
+                                               PathState<float> &b, float2 Z1, float2 Z2, uint32_t pois_a,
+                                               uint32_t pois_b, uint32_t kmin, uint32_t k0, uint32_t k1,
+                                               uint32_t path_a, uint32_t path_b, uint32_t stream, int n) {
     float2 S2 = make_float2(a.S, b.S), v2 = make_float2(a.v, b.v);
-    if constexpr (SCHEME == kQE) step_qe_two_f32(p, S2, v2, Z1, Z2);
+    if constexpr (SCHEME == kQE) step_qe_two_f32(tt, p, S2, v2, Z1, Z2);
     else if constexpr (SCHEME == kMilstein) step_milstein_two_f32(p, S2, v2, Z1, Z2);
     else step_euler_two_f32(p, S2, v2, Z1, Z2);
     a.S = S2.x;
@@ -398,8 +395,8 @@ __device__ __forceinline__ void step_two_z_f32(const StepConst<float> &p, PathSt
 // between the 16-step blocks that add to them: this thread's shared-memory slot (two
 // FP64 sums read and written once per block, four registers fewer in the step loop),
 // or nullptr for a.ssum and b.ssum.
-template <int MODEL, int SCHEME, bool NEG, bool TRK = true, class Gen, class Sink2>
-__device__ __forceinline__ void simulate_two(const StepConst<float> &p, float S0, float v0, int n_steps, const Gen &gen,
+template <int MODEL, int SCHEME, bool NEG, bool TRK = true, class Term, class Gen, class Sink2>
+__device__ __forceinline__ void simulate_two(const Term &tt, const StepConst<float> &p, float S0, float v0, int n_steps, const Gen &gen,
                                              uint32_t k0, uint32_t k1, uint32_t path_a, uint32_t path_b,
                                              uint32_t stream, uint32_t kmin, PathState<float> &a, PathState<float> &b,
                                              Sink2 &&sink, double2 *ssum_slot = nullptr) {
@@ -440,12 +437,12 @@ __device__ __forceinline__ void simulate_two(const StepConst<float> &p, float S0
             // Box-Muller (independent of the first step) overlaps the first step's work
             // (QE, whose step holds more live values, measures faster without it)
             if constexpr (SCHEME != kQE) normals_two_f32<NEG>(wa.z, wa.w, wb.z, wb.w, Z1b, Z2b);
-            step_two_z_f32<MODEL, SCHEME, NEG>(p, a, b, Z1a, Z2a, qa0, qb0, kmin, k0, k1, path_a, path_b, stream, n);
+            step_two_z_f32<MODEL, SCHEME, NEG>(tt, p, a, b, Z1a, Z2a, qa0, qb0, kmin, k0, k1, path_a, path_b, stream, n);
             if constexpr (TRK) track(a, blk_a);
             if constexpr (TRK) track(b, blk_b);
             sink(n, a.S, a.v, b.S, b.v);
             if constexpr (SCHEME == kQE) normals_two_f32<NEG>(wa.z, wa.w, wb.z, wb.w, Z1b, Z2b);
-            step_two_z_f32<MODEL, SCHEME, NEG>(p, a, b, Z1b, Z2b, qa1, qb1, kmin, k0, k1, path_a, path_b, stream, n + 1);
+            step_two_z_f32<MODEL, SCHEME, NEG>(tt, p, a, b, Z1b, Z2b, qa1, qb1, kmin, k0, k1, path_a, path_b, stream, n + 1);
             if constexpr (TRK) track(a, blk_a);
             if constexpr (TRK) track(b, blk_b);
             sink(n + 1, a.S, a.v, b.S, b.v);
@@ -462,7 +459,7 @@ __device__ __forceinline__ void simulate_two(const StepConst<float> &p, float S0
             float2 Z1, Z2;
             normals_two_f32<NEG>(wa.x, wa.y, wb.x, wb.y, Z1, Z2);
             const uint32_t qa0 = poisson_hi_f32(wa.x, wa.y), qb0 = poisson_hi_f32(wb.x, wb.y);
-            step_two_z_f32<MODEL, SCHEME, NEG>(p, a, b, Z1, Z2, qa0, qb0, kmin, k0, k1, path_a, path_b, stream, n);
+            step_two_z_f32<MODEL, SCHEME, NEG>(tt, p, a, b, Z1, Z2, qa0, qb0, kmin, k0, k1, path_a, path_b, stream, n);
             if constexpr (TRK) track(a, blk_a);
             if constexpr (TRK) track(b, blk_b);
             sink(n, a.S, a.v, b.S, b.v);
@@ -521,7 +518,8 @@ __device__ __forceinline__ int find_task(const int64_t *__restrict__ prefix, int
 // kLaneTwo (two independent paths 2u and 2u+1).
 // Blocks of 128, 256 or 512 threads (FP32; up to 256 in FP64): the register budget is
 // set for kPathMinBlocksFp32 resident 256-thread blocks per SM (64 registers a thread).
-template <class R, int MODEL, int SCHEME, bool UK, int LANE, bool TRK>
+// TAB: one FP32 QE task, its term table in dynamic shared memory.
+template <class R, int MODEL, int SCHEME, bool UK, int LANE, bool TRK, bool TAB = false>
 __global__ void __launch_bounds__(path_block_max<R>(),
                                   sizeof(R) == 4 ? kPathMinBlocksFp32 * kPathBlock / path_block_max<R>()
                                                  : (SCHEME == kQE ? kPathMinBlocksQe64 : kPathMinBlocks64))
@@ -544,6 +542,11 @@ __global__ void __launch_bounds__(path_block_max<R>(),
     tables.fill();
     constexpr int kRows = philox_rows<R, MODEL>();
     __shared__ uint4 s_rows[path_block_max<R>() / 32][kRows];
+    extern __shared__ float2 s_term[];
+    const auto tt = [&] {
+        if constexpr (TAB) return TermTable::fill(s_term, tasks[0].term_lo);
+        else return TermSfu{};
+    }();
 
     for (;;) {
         long long q = 0;
@@ -597,7 +600,7 @@ __global__ void __launch_bounds__(path_block_max<R>(),
                         sa = two[0];
                         sb = two[1];
                     } else {
-                        simulate_two<MODEL, SCHEME, NEG, TRK>(p, S0, v0, n_steps, gen, k0, k1, pa, pb, stream, kmin, sa, sb,
+                        simulate_two<MODEL, SCHEME, NEG, TRK>(tt, p, S0, v0, n_steps, gen, k0, k1, pa, pb, stream, kmin, sa, sb,
                                                               NoSink2{}, kSumSlot ? &s_ssum[threadIdx.x] : nullptr);
                     }
                 });
@@ -649,6 +652,15 @@ __host__ PriceKernel<R> price_kernel_for_keys(int model, int scheme) {
         case 4: return price_tiles_kernel<R, kBates, kMilstein, UK, LANE, TRK>;
         default: return price_tiles_kernel<R, kBates, kQE, UK, LANE, TRK>;
     }
+}
+
+// The kernel with a term table: FP32 QE, parameter keys, two paths per lane.
+PriceKernel<float> price_table_kernel_for(int model, bool track) {
+    if (model == kHeston)
+        return track ? price_tiles_kernel<float, kHeston, kQE, true, kLaneTwo, true, true>
+                     : price_tiles_kernel<float, kHeston, kQE, true, kLaneTwo, false, true>;
+    return track ? price_tiles_kernel<float, kBates, kQE, true, kLaneTwo, true, true>
+                 : price_tiles_kernel<float, kBates, kQE, true, kLaneTwo, false, true>;
 }
 
 template <class R, int LANE>
@@ -812,12 +824,13 @@ __global__ void __launch_bounds__(kPathBlock, sizeof(R) == 4 ? kPathMinBlocksFp3
     constexpr int kRows = philox_rows<R, MODEL>();
     __shared__ uint4 s_rows[kPathBlock / 32][kRows];
     const WarpPhilox<kRows, ParamKeys> gen{ParamKeys{rk}, s_rows[threadIdx.x >> 5], t.stream};
-    // whole warps: a lane beyond the last path simulates without storing
+    // whole warps (the generator's rows are the warp's work): a lane beyond the last path
+    // repeats that path and stores its values again
     const int lane = threadIdx.x & 31;
     for (int64_t i0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x - lane; i0 < count;
          i0 += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int64_t i = i0 + lane;
-        SlabSink<R> sink{slab_S, slab_v, ld, i, stride, stride, i < count};
+        const int64_t i = std::min(i0 + lane, count - 1);
+        SlabSink<R> sink{slab_S, slab_v, ld, i, stride, stride};
         PathState<R> st;
         simulate_path<R, MODEL, SCHEME, false>(tables.get(), p, static_cast<R>(t.S0), static_cast<R>(t.v0), t.n_steps, gen,
                                                t.key0, t.key1, static_cast<uint32_t>(first_path + i), t.stream,
@@ -826,38 +839,44 @@ __global__ void __launch_bounds__(kPathBlock, sizeof(R) == 4 ? kPathMinBlocksFp3
 }
 
 // FP32, two paths per thread (first + 2i and first + 2i + 1), interleaved and stepped as
-// pairs; same values as the one-path kernel.
-template <int MODEL, int SCHEME>
-__global__ void __launch_bounds__(kPathBlock, kPathMinBlocksFp32) slab_paths_two_kernel(const TaskDev *__restrict__ task,
-                                                                   int64_t first_path, int64_t count, int stride,
-                                                                   float *__restrict__ slab_S,
-                                                                   float *__restrict__ slab_v, int64_t ld,
-                                                                   const PhiloxRoundKeys rk) {
-    const int64_t i = 2 * (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x);
-    if (i - 2 * (threadIdx.x & 31) >= count) return;  // whole warps only: the generator's rows are the warp's work
+// pairs; same values as the one-path kernel.  One pair per thread and blocks of 256: the
+// hardware's dealing of 8,192 blocks measures 6% faster than four resident blocks per SM
+// striding over the pairs, also with a term table (TAB) to fill in every block.
+template <int MODEL, int SCHEME, bool TAB>
+__global__ void __launch_bounds__(kPathBlock, kPathMinBlocksFp32)
+    slab_paths_two_kernel(const TaskDev *__restrict__ task, int64_t first_path, int64_t count, int stride,
+                          float *__restrict__ slab_S, float *__restrict__ slab_v, int64_t ld, const PhiloxRoundKeys rk) {
     const TaskDev &t = *task;
     const StepConst<float> p = task_const<float>(t);
     __shared__ uint4 s_rows[kPathBlock / 32][32];
+    extern __shared__ float2 s_term[];
+    const auto tt = [&] {
+        if constexpr (TAB) return TermTable::fill(s_term, t.term_lo);
+        else return TermSfu{};
+    }();
     const WarpPhilox<32, ParamKeys> gen{ParamKeys{rk}, s_rows[threadIdx.x >> 5], t.stream};
-    SlabSink2<float> sink{slab_S, slab_v, ld, i, stride, stride, i < count, i + 1 < count};
+    // whole warps: a lane beyond the last path repeats the last pair and stores its values again
+    const int64_t i0 = 2 * (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x);
+    if (i0 - 2 * static_cast<int64_t>(threadIdx.x & 31) >= count) return;
+    const int64_t i = std::min(i0, (count - 1) & ~int64_t(1));
+    SlabSink2<float> sink{slab_S, slab_v, ld, i, stride, stride, i + 1 < count};
     PathState<float> sa, sb;
     const uint32_t pa = static_cast<uint32_t>(first_path + i);
-    simulate_two<MODEL, SCHEME, false, false>(p, static_cast<float>(t.S0), static_cast<float>(t.v0), t.n_steps,
-                                              gen, t.key0, t.key1, pa, pa + 1u, t.stream, t.jump_kmin, sa, sb,
-                                              sink);
+    simulate_two<MODEL, SCHEME, false, false>(tt, p, static_cast<float>(t.S0), static_cast<float>(t.v0), t.n_steps, gen,
+                                              t.key0, t.key1, pa, pa + 1u, t.stream, t.jump_kmin, sa, sb, sink);
 }
 
 template <class R>
 using SlabKernel = void (*)(const TaskDev *, int64_t, int64_t, int, R *, R *, int64_t, const PhiloxRoundKeys);
 
-SlabKernel<float> slab_two_kernel_for(int model, int scheme) {
+SlabKernel<float> slab_two_kernel_for(int model, int scheme, bool table) {
     switch (model * 3 + scheme) {
-        case 0: return slab_paths_two_kernel<kHeston, kEuler>;
-        case 1: return slab_paths_two_kernel<kHeston, kMilstein>;
-        case 2: return slab_paths_two_kernel<kHeston, kQE>;
-        case 3: return slab_paths_two_kernel<kBates, kEuler>;
-        case 4: return slab_paths_two_kernel<kBates, kMilstein>;
-        default: return slab_paths_two_kernel<kBates, kQE>;
+        case 0: return slab_paths_two_kernel<kHeston, kEuler, false>;
+        case 1: return slab_paths_two_kernel<kHeston, kMilstein, false>;
+        case 2: return table ? slab_paths_two_kernel<kHeston, kQE, true> : slab_paths_two_kernel<kHeston, kQE, false>;
+        case 3: return slab_paths_two_kernel<kBates, kEuler, false>;
+        case 4: return slab_paths_two_kernel<kBates, kMilstein, false>;
+        default: return table ? slab_paths_two_kernel<kBates, kQE, true> : slab_paths_two_kernel<kBates, kQE, false>;
     }
 }
 
@@ -982,17 +1001,27 @@ __global__ void step_trace_kernel(const TaskDev *__restrict__ task, const double
 cudaError_t launch_price_tiles(int precision, int model, int scheme, int grid, cudaStream_t s, const TaskDev *tasks,
                                const int64_t *prefix, int32_t n_tasks, int64_t slot_begin, int64_t slot_end,
                                unsigned long long *cursor, Moments *partials, bool uniform_key, uint64_t seed,
-                               int lane_mode, bool track, int block) {
+                               int lane_mode, bool track, int block, bool table) {
     if (!price_tiles_block_ok(precision, block)) return cudaErrorInvalidConfiguration;
     const PhiloxRoundKeys rk = philox_round_keys(static_cast<uint32_t>(seed & 0xFFFFFFFFull),
                                                  static_cast<uint32_t>(seed >> 32));
-    if (precision == QK_FP32)
+    if (table)
+        price_table_kernel_for(model, track)<<<grid, block, (kTermTableMax + 1) * sizeof(float2), s>>>(
+            tasks, prefix, n_tasks, slot_begin, slot_end, cursor, partials, rk);
+    else if (precision == QK_FP32)
         price_kernel_for<float>(model, scheme, uniform_key, lane_mode, track)<<<grid, block, 0, s>>>(
             tasks, prefix, n_tasks, slot_begin, slot_end, cursor, partials, rk);
     else
         price_kernel_for<double>(model, scheme, uniform_key, lane_mode, track)<<<grid, block, 0, s>>>(
             tasks, prefix, n_tasks, slot_begin, slot_end, cursor, partials, rk);
     return cudaGetLastError();
+}
+
+// One block of 512 threads fills the table for 16 warps; smaller blocks would hold more
+// copies of it per SM than fit beside their other shared memory.
+bool price_tiles_takes_table(const TaskDev &t, int block) {
+    return t.precision == QK_FP32 && t.scheme == kQE && t.lane_mode == kLaneTwo && t.term_lo > 0 &&
+           block == path_block_max<float>();
 }
 
 bool price_tiles_block_ok(int precision, int block) {
@@ -1019,14 +1048,18 @@ cudaError_t launch_merge_two_level(int n_tasks, int64_t n_chunks, cudaStream_t s
 
 cudaError_t launch_slab_paths(int precision, int model, int scheme, uint64_t seed, cudaStream_t s, const TaskDev *task,
                               int64_t first_path, int64_t count, int stride, void *slab_S, void *slab_v, int64_t ld,
-                              int paths_per_thread) {
+                              int sm_count, int paths_per_thread, bool has_table) {
     const PhiloxRoundKeys rk = philox_round_keys(static_cast<uint32_t>(seed & 0xFFFFFFFFull),
                                                  static_cast<uint32_t>(seed >> 32));
     if (paths_per_thread == 2) {
         if (precision != QK_FP32) return cudaErrorInvalidValue;
         const int64_t threads = (count + 1) / 2;
-        const unsigned blocks2 = static_cast<unsigned>((threads + kPathBlock - 1) / kPathBlock);
-        slab_two_kernel_for(model, scheme)<<<blocks2, kPathBlock, 0, s>>>(
+        const int64_t blocks2 = (threads + kPathBlock - 1) / kPathBlock;
+        const int64_t resident = static_cast<int64_t>(sm_count) * kPathMinBlocksFp32;
+        // a block's table (a 1/200 of its steps at 250) where the GPU is filled several times over
+        const bool table = scheme == kQE && has_table && blocks2 > resident;
+        slab_two_kernel_for(model, scheme, table)<<<static_cast<unsigned>(blocks2), kPathBlock,
+                                                    table ? (kTermTableMax + 1) * sizeof(float2) : 0, s>>>(
             task, first_path, count, stride, static_cast<float *>(slab_S), static_cast<float *>(slab_v), ld, rk);
         return cudaGetLastError();
     }
@@ -1112,7 +1145,8 @@ static cudaError_t preload_path_kernels_of() {
                     for (int trk = 0; trk < 2 && e == cudaSuccess; ++trk)
                         e = cudaFuncGetAttributes(&fa, price_kernel_for<R>(model, scheme, uk != 0, lane, trk != 0));
             if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, slab_kernel_for<R>(model, scheme));
-            if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, slab_two_kernel_for(model, scheme));
+            for (int tab = 0; tab < 2 && e == cudaSuccess; ++tab)
+                e = cudaFuncGetAttributes(&fa, slab_two_kernel_for(model, scheme, tab != 0));
             if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, payoff_kernel_for<R, true>(model, scheme));
             if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, payoff_kernel_for<R, false>(model, scheme));
         }
@@ -1124,6 +1158,16 @@ static cudaError_t preload_path_kernels_of() {
 cudaError_t preload_path_kernels() {
     cudaFuncAttributes fa;
     cudaError_t e = preload_path_kernels_of<float>();
+    // the term tables need more dynamic shared memory than the default limit
+    const int table_bytes = (kTermTableMax + 1) * static_cast<int>(sizeof(float2));
+    for (int model = 0; model < 2 && e == cudaSuccess; ++model) {
+        for (int trk = 0; trk < 2 && e == cudaSuccess; ++trk)
+            e = cudaFuncSetAttribute(price_table_kernel_for(model, trk != 0), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     table_bytes);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(slab_two_kernel_for(model, kQE, true), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     table_bytes);
+    }
     if (e == cudaSuccess) e = preload_path_kernels_of<double>();
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, merge_tasks_kernel);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, merge_chunks_kernel);

@@ -110,3 +110,49 @@ def test_single_wave_launches_keep_the_bits(qk, handle, precision, n_paths):
     finally:
         handle.tune_reset()
     assert out[0] == out[1]
+
+
+@pytest.mark.parametrize("model", [0, 1])
+@pytest.mark.parametrize("params", [
+    dict(sigma=0.3, rho=-0.7, T=0.1, n_steps=25),                         # term above 1, a few thousand floats
+    dict(sigma=0.3, rho=0.6, T=0.1, n_steps=25),                          # term below 1
+    dict(sigma=0.9, rho=-0.7, v0=0.01, theta=0.01, kappa=0.5, T=0.1, n_steps=25),  # many steps outside the plain regime
+    dict(sigma=0.3, rho=0.0, T=0.1, n_steps=25),                          # term next to 1
+    dict(sigma=0.3, rho=-0.7, theta=0.0, kappa=0.0, T=0.1, n_steps=25),   # no mean reversion
+    dict(sigma=0.5, rho=-0.9, T=4.0, n_steps=9),                          # too many floats for a table
+])
+def test_term_table_keeps_the_bits(qk, handle, model, params):
+    """A persistent launch of one FP32 QE contract in 512-thread blocks takes two SFU results per
+    step from a table; blocks of 256 threads take none.  The same bits, also next to and outside
+    the table's range."""
+    c = qk.make_contract(model=model, scheme=qk.ANDERSEN_QE, lambda_j=0.4 if model else 0.0, mu_j=-0.05, sigma_j=0.1,
+                         n_paths=1_000_003, seed=31, precision=qk.FP32,
+                         payoffs=[qk.payoff(qk.EUROPEAN, qk.CALL, 100.0), qk.payoff(qk.ASIAN, qk.PUT, 100.0)], **params)
+    out = []
+    try:
+        for block in (256, 512):
+            handle.tune_set(qk.FP32, model, qk.ANDERSEN_QE, 24, False, 2, block_size=block)
+            out.append(qk.price_batch([c], None, handle)[0]["legs"])
+    finally:
+        handle.tune_reset()
+    assert out[0] == out[1]
+
+
+@pytest.mark.parametrize("model", [0, 1])
+def test_slab_term_table_keeps_the_bits(qk, handle, model):
+    """American forward slabs of one FP32 QE contract: path counts below and above the line from
+    which the slab kernel uses the table price like the FP64 engine (0.25 SE, as the other FP32
+    American checks), and a contract equals itself priced in one call with another."""
+    for n_paths in (100_001, 400_003):
+        c = qk.make_contract(model=model, scheme=qk.ANDERSEN_QE, lambda_j=0.2 if model else 0.0, mu_j=-0.05, sigma_j=0.1,
+                             n_paths=n_paths, n_steps=50, T=0.2, seed=8, precision=qk.FP32, lsm_basis=qk.LSM_POLY_SV,
+                             lsm_dates=10, payoffs=[qk.payoff(qk.AMERICAN, qk.PUT, 100.0)])
+        alone = qk.price_batch([c], None, handle)[0]["legs"][0]
+        both = qk.price_batch([c, c], None, handle)
+        assert both[0]["legs"][0] == both[1]["legs"][0] == alone
+        if model == 0:  # Bates draws its jumps from other bits in FP64
+            c64 = qk.make_contract(**{**dict(scheme=qk.ANDERSEN_QE, n_paths=n_paths, n_steps=50, T=0.2, seed=8,
+                                             precision=qk.FP64, lsm_basis=qk.LSM_POLY_SV, lsm_dates=10),
+                                      "payoffs": [qk.payoff(qk.AMERICAN, qk.PUT, 100.0)]})
+            want = qk.price_plain(c64, None, handle)["legs"][0]
+            assert abs(alone["price"] - want["price"]) < 0.25 * want["std_error"]
