@@ -900,7 +900,7 @@ qk_status qk_create(int32_t device, qk_handle **out) {
     // used by the LSM streams only after they fork from it); the device's memory pool
     // keeps freed blocks for reuse instead of returning them at every synchronization
     for (qk::DevArena *a : {&h->d_tasks, &h->d_prefix, &h->d_partials, &h->d_moments, &h->d_cursor, &h->d_trace,
-                            &h->d_chunks, &h->d_lsm_moments, &h->lsm_task, &h->lsm_centre})
+                            &h->d_chunks, &h->d_lsm_moments, &h->lsm_task})
         a->stream = h->stream;
     for (int l = 0; l < kLsmLanes; ++l)
         for (qk::DevArena *a : {&h->lsm[l].slab_S, &h->lsm[l].slab_v, &h->lsm[l].cashflow, &h->lsm[l].block_sums,

@@ -98,10 +98,10 @@ struct qk_handle {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev_start = nullptr, ev_paths0 = nullptr, ev_paths1 = nullptr, ev_end = nullptr;
     qk::DevArena d_tasks, d_prefix, d_partials, d_moments, d_cursor, d_trace, d_chunks;
-    qk::HostArena h_tasks, h_moments, h_lsm;
+    qk::HostArena h_tasks, h_moments, h_lsm, h_lsm_up;
     qk::DevArena d_lsm_moments;
     qk::LsmArena lsm[qk::kLsmLanes];
-    qk::DevArena lsm_task, lsm_centre;    // descriptors and centring shifts of all jobs of a call
+    qk::DevArena lsm_task;                // descriptors and centring shifts of all jobs of a call
     cudaStream_t lsm_stream[qk::kLsmLanes] = {};
     cudaStream_t kind_stream[qk::kKindStreams] = {};
     cudaEvent_t kind_fork = nullptr, kind_join[qk::kKindStreams] = {};

@@ -1114,7 +1114,7 @@ void lsm_release(qk_handle *h) {
     if (h->lsm_fork) cudaEventDestroy(h->lsm_fork);
     h->lsm_fork = nullptr;
     h->lsm_task.release();
-    h->lsm_centre.release();
+    h->h_lsm_up.release();
     h->h_lsm.release();
     h->d_lsm_moments.release();
 }
@@ -1195,13 +1195,22 @@ qk_status run_lsm_contracts(qk_handle *h, Plan &plan, bool plain, std::vector<Mo
         if ((st = L.status.ensure(static_cast<size_t>(lane_dates[l]) * sizeof(int) + 256)) != QK_OK) return st;
     }
     if ((st = lsm_events_ensure(h, 3 * nj)) != QK_OK) return st;
-    if ((st = h->lsm_task.ensure(nj * sizeof(TaskDev))) != QK_OK) return st;
     if ((st = h->d_lsm_moments.ensure(nj * grid * sizeof(Moments))) != QK_OK) return st;
     if ((st = h->h_lsm.ensure(nj * grid * sizeof(Moments))) != QK_OK) return st;
-    // descriptors and per-date centring constants of all jobs (one upload, blocking)
-    std::vector<TaskDev> tasks(nj);
-    std::vector<double> centres;
+    // Descriptors, then per-date centring constants, of all jobs: one copy from pinned memory
+    // on the handle's stream, which the lanes fork from.  (A blocking copy from pageable
+    // memory may return before its last part has reached the device, and the lanes' streams
+    // do not wait for the default stream it goes through.)
+    size_t n_centres = 0;
+    for (const Job &j : jobs) n_centres += 2 * static_cast<size_t>(dates_of(j.b));
+    const size_t task_bytes = (nj * sizeof(TaskDev) + 255) / 256 * 256;
+    const size_t up_bytes = task_bytes + n_centres * sizeof(double);
+    if ((st = h->lsm_task.ensure(up_bytes)) != QK_OK) return st;
+    if ((st = h->h_lsm_up.ensure(up_bytes)) != QK_OK) return st;
+    TaskDev *tasks = static_cast<TaskDev *>(h->h_lsm_up.ptr);
+    double *centres = reinterpret_cast<double *>(static_cast<char *>(h->h_lsm_up.ptr) + task_bytes);
     std::vector<size_t> centre_off(nj);
+    size_t at = 0;
     for (size_t k = 0; k < nj; ++k) {
         const qk_contract &b = jobs[k].b;
         tasks[k] = make_task(b, 1);
@@ -1209,19 +1218,16 @@ qk_status run_lsm_contracts(qk_handle *h, Plan &plan, bool plain, std::vector<Mo
         const int stride = b.n_steps / D;
         const double dt = b.T / b.n_steps;
         const double K = b.payoffs[0].strike;
-        centre_off[k] = centres.size();
+        centre_off[k] = at;
         for (int d = 0; d < D; ++d) {
             const double t = (d + 1) * stride * dt;
             // forward level of S/K and the mean of v_t: shifts that centre the regression basis
-            centres.push_back(b.S0 / K * std::exp((b.r - b.q) * t));
-            centres.push_back(b.theta + (b.v0 - b.theta) * std::exp(-b.kappa * t));
+            centres[at++] = b.S0 / K * std::exp((b.r - b.q) * t);
+            centres[at++] = b.theta + (b.v0 - b.theta) * std::exp(-b.kappa * t);
         }
     }
-    if ((st = h->lsm_centre.ensure(std::max<size_t>(centres.size(), 1) * sizeof(double))) != QK_OK) return st;
-    const double *d_centre = static_cast<const double *>(h->lsm_centre.ptr);
-    QK_CUDA_LSM(cudaMemcpy(h->lsm_task.ptr, tasks.data(), nj * sizeof(TaskDev), cudaMemcpyHostToDevice));
-    QK_CUDA_LSM(cudaMemcpy(h->lsm_centre.ptr, centres.data(), centres.size() * sizeof(double),
-                           cudaMemcpyHostToDevice));
+    const double *d_centre = reinterpret_cast<const double *>(static_cast<const char *>(h->lsm_task.ptr) + task_bytes);
+    QK_CUDA_LSM(cudaMemcpyAsync(h->lsm_task.ptr, h->h_lsm_up.ptr, up_bytes, cudaMemcpyHostToDevice, h->stream));
     // fork: the lanes start after the work already queued on the handle's stream
     QK_CUDA_LSM(cudaEventRecord(h->lsm_fork, h->stream));
     for (int l = 0; l < lanes; ++l) QK_CUDA_LSM(cudaStreamWaitEvent(h->lsm_stream[l], h->lsm_fork, 0));
