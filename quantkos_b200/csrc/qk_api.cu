@@ -517,44 +517,52 @@ qk_status build_plan(qk_handle *h, const qk_contract *cs, int32_t n, const qk_gr
     return QK_OK;
 }
 
-// Device arenas for the plan and the copy of its task descriptors and tile
-// prefix to the device.
+// The plan on the device, one buffer and one copy: task descriptors, the tile prefix, then
+// the queue cursors (zero; the merge clears them again after each run).
+static size_t plan_prefix_at(size_t nt) { return nt * sizeof(TaskDev); }
+static size_t plan_cursor_at(size_t nt) { return plan_prefix_at(nt) + nt * sizeof(int64_t); }
+static size_t plan_bytes(size_t nt) { return plan_cursor_at(nt) + nt * sizeof(unsigned long long); }
+static_assert(sizeof(TaskDev) % 8 == 0, "the prefix follows the descriptors");
+
+// Device arenas for the plan and its upload.
 static qk_status upload_plan(qk_handle *h, const Plan &plan) {
     const size_t nt = plan.tasks.size();
     qk_status s;
-    if ((s = h->d_tasks.ensure(nt * sizeof(TaskDev))) != QK_OK) return s;
-    if ((s = h->d_prefix.ensure(nt * sizeof(int64_t))) != QK_OK) return s;
+    if ((s = h->d_tasks.ensure(plan_bytes(nt))) != QK_OK) return s;
     if ((s = h->d_partials.ensure(static_cast<size_t>(plan.total_records) * sizeof(Moments))) != QK_OK) return s;
     if ((s = h->d_moments.ensure(nt * QK_MAX_PAYOFFS * sizeof(Moments))) != QK_OK) return s;
     if ((s = h->d_chunks.ensure(static_cast<size_t>(plan.total_chunks) * QK_MAX_PAYOFFS * sizeof(Moments))) != QK_OK)
         return s;
-    if ((s = h->d_cursor.ensure(nt * sizeof(unsigned long long))) != QK_OK) return s;
-    if ((s = h->h_tasks.ensure(nt * sizeof(TaskDev) + nt * sizeof(int64_t))) != QK_OK) return s;
+    if ((s = h->h_tasks.ensure(plan_bytes(nt))) != QK_OK) return s;
     if ((s = h->h_moments.ensure(nt * QK_MAX_PAYOFFS * sizeof(Moments))) != QK_OK) return s;
-    TaskDev *ht = static_cast<TaskDev *>(h->h_tasks.ptr);
-    int64_t *hp = reinterpret_cast<int64_t *>(ht + nt);
-    std::memcpy(ht, plan.tasks.data(), nt * sizeof(TaskDev));
+    char *base = static_cast<char *>(h->h_tasks.ptr);
+    std::memcpy(base, plan.tasks.data(), nt * sizeof(TaskDev));
+    int64_t *hp = reinterpret_cast<int64_t *>(base + plan_prefix_at(nt));
     for (size_t i = 0; i < nt; ++i) hp[i] = plan.tasks[i].tile_begin;
-    QK_CUDA_TRY(cudaMemcpyAsync(h->d_tasks.ptr, ht, nt * sizeof(TaskDev), cudaMemcpyHostToDevice, h->stream));
-    QK_CUDA_TRY(cudaMemcpyAsync(h->d_prefix.ptr, hp, nt * sizeof(int64_t), cudaMemcpyHostToDevice, h->stream));
+    std::memset(base + plan_cursor_at(nt), 0, nt * sizeof(unsigned long long));
+    QK_CUDA_TRY(cudaMemcpyAsync(h->d_tasks.ptr, base, plan_bytes(nt), cudaMemcpyHostToDevice, h->stream));
     return QK_OK;
 }
 
-// The steady part of a run: clear the queue cursors, launch the path kernels
-// (one persistent launch per kernel kind for the batched engine, one launch per
-// task for the plain method), merge the tile moments and copy them to the host.
+// Up to this many tasks the merge writes the results straight into the pinned host buffer
+// (256 bytes a task over PCIe as posted writes); more go by one copy.
+constexpr size_t kDirectResultTasks = 64;
+
+// The steady part of a run: launch the path kernels (one persistent launch per kernel kind
+// for the batched engine, one launch per task for the plain method), merge the tile
+// moments (and clear the queue cursors) and bring the results to the host.
 // `capture`: the stream is being captured into a graph, so the timing events
 // are recorded as external event nodes of that graph.
 static qk_status enqueue_plan(qk_handle *h, const Plan &plan, bool capture) {
     const size_t nt = plan.tasks.size();
     const unsigned ev_flags = capture ? cudaEventRecordExternal : cudaEventRecordDefault;
-    QK_CUDA_TRY(cudaMemsetAsync(h->d_cursor.ptr, 0, nt * sizeof(unsigned long long), h->stream));
     QK_CUDA_TRY(cudaEventRecordWithFlags(h->ev_paths0, h->stream, ev_flags));
-    const TaskDev *dt = static_cast<const TaskDev *>(h->d_tasks.ptr);
-    const int64_t *dp = static_cast<const int64_t *>(h->d_prefix.ptr);
-    unsigned long long *dc = static_cast<unsigned long long *>(h->d_cursor.ptr);
+    char *plan_base = static_cast<char *>(h->d_tasks.ptr);
+    const TaskDev *dt = reinterpret_cast<const TaskDev *>(plan_base);
+    const int64_t *dp = reinterpret_cast<const int64_t *>(plan_base + plan_prefix_at(nt));
+    unsigned long long *dc = reinterpret_cast<unsigned long long *>(plan_base + plan_cursor_at(nt));
     Moments *dpart = static_cast<Moments *>(h->d_partials.ptr);
-    // launches on forked streams: every launch waits for the cursor reset and the start
+    // launches on forked streams: every launch waits for the plan's upload and the start
     // event; the handle's stream waits for all of them before the merge
     int n_launches = static_cast<int>(nt);  // the plain method: one per task
     if (!plan.plain) {
@@ -616,12 +624,13 @@ static qk_status enqueue_plan(qk_handle *h, const Plan &plan, bool capture) {
         }
     }
     QK_CUDA_TRY(cudaEventRecordWithFlags(h->ev_paths1, h->stream, ev_flags));
-    QK_CUDA_TRY(launch_merge_two_level(static_cast<int>(nt), plan.total_chunks, h->stream, dt, dpart,
-                                       static_cast<Moments *>(h->d_chunks.ptr),
-                                       static_cast<Moments *>(h->d_moments.ptr)));
-    h->launches += 2;
-    QK_CUDA_TRY(cudaMemcpyAsync(h->h_moments.ptr, h->d_moments.ptr, nt * QK_MAX_PAYOFFS * sizeof(Moments),
-                                cudaMemcpyDeviceToHost, h->stream));
+    const bool direct = nt <= kDirectResultTasks;
+    Moments *results = static_cast<Moments *>(direct ? h->h_moments.ptr : h->d_moments.ptr);
+    QK_CUDA_TRY(launch_merge(static_cast<int>(nt), plan.total_chunks, h->stream, dt, dpart,
+                             static_cast<Moments *>(h->d_chunks.ptr), results, dc, &h->launches));
+    if (!direct)
+        QK_CUDA_TRY(cudaMemcpyAsync(h->h_moments.ptr, h->d_moments.ptr, nt * QK_MAX_PAYOFFS * sizeof(Moments),
+                                    cudaMemcpyDeviceToHost, h->stream));
     return QK_OK;
 }
 
@@ -629,7 +638,7 @@ static qk_status enqueue_plan(qk_handle *h, const Plan &plan, bool capture) {
 qk_status run_plan(qk_handle *h, Plan &plan) {
     const size_t nt = plan.tasks.size();
     h->launches = 0;
-    h->h2d_bytes = static_cast<int64_t>(nt * (sizeof(TaskDev) + sizeof(int64_t)));
+    h->h2d_bytes = static_cast<int64_t>(plan_bytes(nt));
     h->d2h_bytes = static_cast<int64_t>(nt * QK_MAX_PAYOFFS * sizeof(Moments));
     QK_CUDA_TRY(cudaEventRecord(h->ev_start, h->stream));
     if (nt > 0) {
@@ -899,7 +908,7 @@ qk_status qk_create(int32_t device, qk_handle **out) {
     // device arenas grow stream-ordered on the handle's stream (the LSM working sets are
     // used by the LSM streams only after they fork from it); the device's memory pool
     // keeps freed blocks for reuse instead of returning them at every synchronization
-    for (qk::DevArena *a : {&h->d_tasks, &h->d_prefix, &h->d_partials, &h->d_moments, &h->d_cursor, &h->d_trace,
+    for (qk::DevArena *a : {&h->d_tasks, &h->d_partials, &h->d_moments, &h->d_trace,
                             &h->d_chunks, &h->d_lsm_moments, &h->lsm_task})
         a->stream = h->stream;
     for (int l = 0; l < kLsmLanes; ++l)
@@ -922,11 +931,9 @@ qk_status qk_destroy(qk_handle *h) {
     release_prepared(h);
     lsm_release(h);
     h->d_tasks.release();
-    h->d_prefix.release();
     h->d_partials.release();
     h->d_moments.release();
     h->d_chunks.release();
-    h->d_cursor.release();
     h->d_trace.release();
     h->h_tasks.release();
     h->h_moments.release();

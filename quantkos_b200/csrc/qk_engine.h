@@ -97,7 +97,7 @@ struct qk_handle {
     int sm_count = 148;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev_start = nullptr, ev_paths0 = nullptr, ev_paths1 = nullptr, ev_end = nullptr;
-    qk::DevArena d_tasks, d_prefix, d_partials, d_moments, d_cursor, d_trace, d_chunks;
+    qk::DevArena d_tasks, d_partials, d_moments, d_trace, d_chunks;  // d_tasks: descriptors, prefix, cursors
     qk::HostArena h_tasks, h_moments, h_lsm, h_lsm_up;
     qk::DevArena d_lsm_moments;
     qk::LsmArena lsm[qk::kLsmLanes];

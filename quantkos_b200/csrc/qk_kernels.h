@@ -44,12 +44,13 @@ cudaError_t launch_merge_tasks(int n_tasks, cudaStream_t s, const TaskDev *tasks
                                TaskMoments *out, int64_t max_tiles = 0);
 // Tile records per level-1 merge chunk.
 constexpr int kMergeChunkTiles = 512;
-// Two-level merge: level 1 reduces chunks of kMergeChunkTiles tile records
-// (n_chunks = sum of the tasks' n_chunks) into chunks[n_chunks][QK_MAX_PAYOFFS],
-// level 2 reduces each task's chunk records into out[task][QK_MAX_PAYOFFS].
-cudaError_t launch_merge_two_level(int n_tasks, int64_t n_chunks, cudaStream_t s, const TaskDev *tasks,
-                                   const Moments *partials, Moments *chunks, TaskMoments *out);
-// paths_per_thread 2: each thread simulates two consecutive paths (same values).
+// Merge of the tile records: level 1 reduces chunks of kMergeChunkTiles records (n_chunks =
+// sum of the tasks' n_chunks) into chunks[n_chunks][QK_MAX_PAYOFFS], level 2 each task's
+// chunk records into out[task][QK_MAX_PAYOFFS]; where every task has one chunk, level 1
+// writes out itself.  Clears the tasks' queue cursors.  out: device or pinned host memory.
+// *launches is increased by the kernels launched.
+cudaError_t launch_merge(int n_tasks, int64_t n_chunks, cudaStream_t s, const TaskDev *tasks, const Moments *partials,
+                         Moments *chunks, TaskMoments *out, unsigned long long *cursors, int64_t *launches);
 // has_table: the task has a term table (TaskDev::term_lo; two paths per thread only).
 cudaError_t launch_slab_paths(int precision, int model, int scheme, uint64_t seed, cudaStream_t s, const TaskDev *task,
                               int64_t first_path, int64_t count, int stride, void *slab_S, void *slab_v, int64_t ld,

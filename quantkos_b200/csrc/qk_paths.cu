@@ -775,9 +775,13 @@ __global__ void __launch_bounds__(1024) merge_tasks_kernel(const TaskDev *__rest
 // over the tasks' chunk_base (ascending, every task has at least one chunk).
 __global__ void __launch_bounds__(256) merge_chunks_kernel(const TaskDev *__restrict__ tasks, int32_t n_tasks,
                                                            const Moments *__restrict__ partials,
-                                                           Moments *__restrict__ chunks) {
+                                                           Moments *__restrict__ chunks,
+                                                           unsigned long long *__restrict__ cursors) {
     __shared__ double red[4][32];
     const int64_t b = blockIdx.x;
+    // the path kernels are done with the queue: ready for the next run
+    if (b == 0)
+        for (int i = threadIdx.x; i < n_tasks; i += blockDim.x) cursors[i] = 0ull;
     int lo = 0, hi = n_tasks - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
@@ -1037,12 +1041,16 @@ cudaError_t launch_merge_tasks(int n_tasks, cudaStream_t s, const TaskDev *tasks
     return cudaGetLastError();
 }
 
-cudaError_t launch_merge_two_level(int n_tasks, int64_t n_chunks, cudaStream_t s, const TaskDev *tasks,
-                                   const Moments *partials, Moments *chunks, TaskMoments *out) {
-    merge_chunks_kernel<<<static_cast<unsigned>(n_chunks), 256, 0, s>>>(tasks, n_tasks, partials, chunks);
+cudaError_t launch_merge(int n_tasks, int64_t n_chunks, cudaStream_t s, const TaskDev *tasks, const Moments *partials,
+                         Moments *chunks, TaskMoments *out, unsigned long long *cursors, int64_t *launches) {
+    const bool one_level = n_chunks == n_tasks;  // every task has at least one chunk
+    merge_chunks_kernel<<<static_cast<unsigned>(n_chunks), 256, 0, s>>>(tasks, n_tasks, partials,
+                                                                       one_level ? out : chunks, cursors);
+    ++*launches;
     cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess || one_level) return e;
     merge_task_chunks_kernel<<<n_tasks, 128, 0, s>>>(tasks, chunks, out);
+    ++*launches;
     return cudaGetLastError();
 }
 

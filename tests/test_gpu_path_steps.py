@@ -156,3 +156,21 @@ def test_slab_term_table_keeps_the_bits(qk, handle, model):
                                       "payoffs": [qk.payoff(qk.AMERICAN, qk.PUT, 100.0)]})
             want = qk.price_plain(c64, None, handle)["legs"][0]
             assert abs(alone["price"] - want["price"]) < 0.25 * want["std_error"]
+
+
+@pytest.mark.parametrize("n_contracts", [1, 5, 6, 30])
+def test_results_on_both_sides_of_the_direct_write(qk, handle, n_contracts):
+    """12 pricing tasks per contract: up to 64 tasks the merge writes the results to the host
+    itself, beyond that they are copied; one-chunk and many-chunk tasks mixed.  A prepared set
+    replayed (its queue cursors cleared by the run before) gives the one-shot call's results."""
+    cs = [qk.make_contract(n_paths=3_000 + 40_000 * (i % 3), n_steps=6 + i % 5, seed=50 + i, scheme=i % 3,
+                           precision=(qk.FP64, qk.FP32)[i % 2]) for i in range(n_contracts)]
+    g = qk.make_greeks(qk.GREEK_ALL, bump_S_rel=0.01, bump_vol=0.02)
+    want = qk.price_batch(cs, g, handle)
+    for c, w in zip(cs, want):
+        assert qk.price_batch([c], g, handle)[0]["legs"][0]["price"] == pytest.approx(w["legs"][0]["price"], rel=1e-13)
+    prep = qk.PreparedBatch(cs, g, handle)
+    for _ in range(3):
+        prep.run()
+        prep.run()
+        assert [r["legs"] for r in prep.fetch()] == [r["legs"] for r in want]
