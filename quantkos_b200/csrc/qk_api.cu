@@ -196,12 +196,15 @@ std::vector<int> roles_for(const qk_greeks *g, double T) {
     return roles;
 }
 
-// Asian, barrier and lookback legs read the running sum, max or min of the path;
-// European, binary and American legs only its final spot.
-static bool needs_path_state(const qk_contract &c) {
-    for (int k = 0; k < c.n_payoffs; ++k)
-        if (c.payoffs[k].type >= QK_ASIAN && c.payoffs[k].type <= QK_LOOKBACK_FIXED) return true;
-    return false;
+// The path state a contract's legs read (European, binary and American legs: only the
+// final spot), as its precision's kernels keep it.
+static int path_state(const qk_contract &c, int precision) {
+    int t = kTrackNone;
+    for (int k = 0; k < c.n_payoffs; ++k) {
+        if (c.payoffs[k].type == QK_ASIAN) t |= kTrackSum;
+        else if (c.payoffs[k].type > QK_ASIAN && c.payoffs[k].type <= QK_LOOKBACK_FIXED) t |= kTrackRange;
+    }
+    return precision == QK_FP32 && t != kTrackNone ? static_cast<int>(kTrackAll) : t;
 }
 
 // The floats 1 - 2 A a can take on a QE step in the plain form of the quadratic regime:
@@ -253,7 +256,7 @@ TaskDev make_task(const qk_contract &b, int ppt, int lane_mode) {
     t.jump_kmin64 = static_cast<uint32_t>(
         std::min(std::max(std::ceil(t.cd.exp_m_lambda_dt * 4294967296.0 - 0.5), 0.0), 4294967295.0));
     t.lane_mode = b.antithetic ? kLanePair : lane_mode;
-    t.track = needs_path_state(b) ? 1 : 0;
+    t.track = path_state(b, b.precision);
     const int64_t units = lane_units(b.n_paths, t.lane_mode);
     const int64_t tile_units = static_cast<int64_t>(kWarpTilePaths) * ppt;
     t.n_tiles = static_cast<int32_t>((units + tile_units - 1) / tile_units);
@@ -312,10 +315,10 @@ struct LaunchShape {
 static LaunchShape launch_shape(const qk_handle *h, const TaskDev &t, size_t n_tasks, int64_t slots, int block) {
     const int single = 128;
     const int64_t per_sm =
-        price_tiles_max_blocks_per_sm(t.precision, t.model, t.scheme, t.lane_mode, t.track != 0, single);
+        price_tiles_max_blocks_per_sm(t.precision, t.model, t.scheme, t.lane_mode, t.track, single);
     if (slots <= h->sm_count * per_sm * (single / 32))
         return LaunchShape{static_cast<int>((slots + single / 32 - 1) / (single / 32)), single, false};
-    const int n = price_tiles_max_blocks_per_sm(t.precision, t.model, t.scheme, t.lane_mode, t.track != 0, block);
+    const int n = price_tiles_max_blocks_per_sm(t.precision, t.model, t.scheme, t.lane_mode, t.track, block);
     const bool table = n_tasks == 1 && price_tiles_takes_table(t, block);
     return LaunchShape{static_cast<int>(std::min<int64_t>(slots, static_cast<int64_t>(h->sm_count) * n)), block, table};
 }
@@ -432,7 +435,7 @@ qk_status build_plan(qk_handle *h, const qk_contract *cs, int32_t n, const qk_gr
     plan.status.assign(n, QK_OK);
     plan.task_of.assign(static_cast<size_t>(n) * kNumRoles, -1);
     // paths per kernel kind (precision, model, scheme): each kind is one launch
-    int64_t kind_paths[2][2][3][3][2] = {};  // [precision][model][scheme][lane mode][track]: lane units per launch
+    int64_t kind_paths[2][2][3][3][4] = {};  // [precision][model][scheme][lane mode][track]: lane units per launch
     auto lane_mode_of = [&](const qk_contract &c, int pr) {
         if (c.antithetic) return static_cast<int>(kLanePair);
         if (plain) return static_cast<int>(kLaneOne);
@@ -450,7 +453,7 @@ qk_status build_plan(qk_handle *h, const qk_contract *cs, int32_t n, const qk_gr
         }
         const int pr = plain ? QK_FP64 : cs[i].precision;
         const int lm = lane_mode_of(cs[i], pr);
-        kind_paths[pr][cs[i].model][cs[i].scheme][lm][needs_path_state(cs[i])] +=
+        kind_paths[pr][cs[i].model][cs[i].scheme][lm][path_state(cs[i], pr)] +=
             lane_units(cs[i].n_paths, lm) * static_cast<int64_t>(roles_for(g, cs[i].T).size());
     }
     struct Item {
@@ -464,7 +467,7 @@ qk_status build_plan(qk_handle *h, const qk_contract *cs, int32_t n, const qk_gr
         const int pr = plain ? QK_FP64 : cs[i].precision;
         const int lm = lane_mode_of(cs[i], pr);
         const int64_t units = lane_units(cs[i].n_paths, lm);
-        const bool trk = needs_path_state(cs[i]);
+        const int trk = path_state(cs[i], pr);
         const int64_t launch_units = plain ? units : kind_paths[pr][cs[i].model][cs[i].scheme][lm][trk];
         const int ppt = choose_ppt(units, launch_units, h->sm_count,
                                    plain ? kPlainTilesPerWarp : h->tune_tpw[pr][cs[i].model][cs[i].scheme]);
@@ -780,8 +783,10 @@ static qk_status payoffs_on_device(qk_handle *h, const qk_contract &c, int64_t f
     TaskDev *dt = reinterpret_cast<TaskDev *>(base + head);
     *out = reinterpret_cast<double *>(base + head + task_bytes);
     QK_CUDA_TRY(cudaMemcpyAsync(dt, &t, sizeof(TaskDev), cudaMemcpyHostToDevice, h->stream));
-    const bool reads_state = n.payoffs[0].type >= QK_ASIAN && n.payoffs[0].type <= QK_LOOKBACK_FIXED;
-    QK_CUDA_TRY(launch_payoff_paths(c.precision == QK_FP32 ? QK_FP32 : QK_FP64, n.model, n.scheme, reads_state, n.seed,
+    qk_contract leg0 = n;
+    leg0.n_payoffs = 1;
+    QK_CUDA_TRY(launch_payoff_paths(c.precision == QK_FP32 ? QK_FP32 : QK_FP64, n.model, n.scheme,
+                                    path_state(leg0, c.precision == QK_FP32 ? QK_FP32 : QK_FP64), n.seed,
                                     h->sm_count, h->stream, dt, first, count, *out));
     return QK_OK;
 }

@@ -73,6 +73,12 @@ struct PayoffSpec {
 // consecutive paths 2u and 2u+1 (instruction-level parallelism).
 enum : int { kLaneOne = 0, kLanePair = 1, kLaneTwo = 2 };
 
+// Path state a kernel keeps: the running sum (Asian legs), the running maximum and minimum
+// (barrier and lookback legs).  In FP64, where a state's cost is an exponential and two
+// comparisons a step, each combination has its kernel; in FP32 (a few operations) a launch
+// keeps all or none.
+enum : int { kTrackNone = 0, kTrackSum = 1, kTrackRange = 2, kTrackAll = 3 };
+
 __host__ __device__ inline int64_t lane_units(int64_t n_paths, int lane_mode) {
     return lane_mode == kLaneOne ? n_paths : (lane_mode == kLanePair ? n_paths / 2 : (n_paths + 1) / 2);
 }
@@ -98,7 +104,7 @@ struct TaskDev {
     int64_t chunk_base;    // first merge chunk of the task (two-level merge of the tile records)
     int32_t n_chunks;      // merge chunks of the task: ceil(n_tiles / kMergeChunkTiles)
     int32_t lane_mode;     // kLaneOne / kLanePair / kLaneTwo: what a lane simulates; tiles count lane units
-    int32_t track;         // 1 if a leg reads the path state (Asian sum, running max / min)
+    int32_t track;         // path state that some leg reads (kTrack*)
     PayoffSpec pay[QK_MAX_PAYOFFS];
 };
 

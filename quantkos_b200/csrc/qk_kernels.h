@@ -30,12 +30,11 @@ constexpr int kPathMinBlocksQe64 = 2;
 // uniform_key: every task of the launch has Philox key `seed` (round keys go in the
 // kernel parameters); otherwise each task's key is read from its descriptor.
 // lane_mode: what a lane simulates for every task of the launch (TaskDev::lane_mode).
-// track: some task of the launch has a leg that reads the path state (TaskDev::track);
-// false selects the kernel that keeps none.
+// track: the path state that some task's legs read (TaskDev::track, kTrack*).
 cudaError_t launch_price_tiles(int precision, int model, int scheme, int grid, cudaStream_t s, const TaskDev *tasks,
                                const int64_t *prefix, int32_t n_tasks, int64_t slot_begin, int64_t slot_end,
                                unsigned long long *cursor, Moments *partials, bool uniform_key, uint64_t seed,
-                               int lane_mode = kLaneOne, bool track = true, int block = kPathBlock,
+                               int lane_mode = kLaneOne, int track = kTrackAll, int block = kPathBlock,
                                bool table = false);
 // Whether a launch of this one task in blocks of `block` threads may use its term table.
 bool price_tiles_takes_table(const TaskDev &t, int block);
@@ -58,8 +57,8 @@ cudaError_t launch_slab_paths(int precision, int model, int scheme, uint64_t see
 cudaError_t launch_step_trace(int precision, cudaStream_t s, const TaskDev *task, const double *z, const double *u,
                               int umax, int n, double *S_out, double *v_out, int *status);
 // Leg-0 payoffs of paths first .. first + count - 1 of the task (undiscounted, normalised).
-// track: the leg reads the path state.
-cudaError_t launch_payoff_paths(int precision, int model, int scheme, bool track, uint64_t seed, int sm_count,
+// track: the path state that leg reads (kTrack*).
+cudaError_t launch_payoff_paths(int precision, int model, int scheme, int track, uint64_t seed, int sm_count,
                                 cudaStream_t s, const TaskDev *task, int64_t first, int64_t count, double *out);
 // Order statistics: the values of ascending ranks r[0..n_ranks-1] (0 = smallest) of x[0..n-1],
 // n < 2^32, into out[n_ranks] (device); scratch holds select_scratch_bytes().
@@ -75,7 +74,7 @@ cudaError_t preload_select_kernels();
 cudaError_t launch_payoff_trace(int precision, cudaStream_t s, const PayoffSpec &ps, const double *S, int n, double S0,
                                 double *out);
 int price_tiles_max_blocks_per_sm(int precision, int model, int scheme, int lane_mode = kLaneOne,
-                                  bool track = true, int block = kPathBlock);
+                                  int track = kTrackAll, int block = kPathBlock);
 // Whether `block` threads per block is a valid launch of the pricing kernel in `precision`.
 bool price_tiles_block_ok(int precision, int block);
 // Loads the device code of every one-path-per-lane pricing kernel (both precisions,

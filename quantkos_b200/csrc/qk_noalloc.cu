@@ -125,7 +125,7 @@ extern "C" qk_status qk_price_noalloc(const qk_contract *c, void *stream, qk_res
     cudaGetDevice(&dev);
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int per_sm = qk::price_tiles_max_blocks_per_sm(t.precision, t.model, t.scheme, t.lane_mode, t.track != 0);
+    const int per_sm = qk::price_tiles_max_blocks_per_sm(t.precision, t.model, t.scheme, t.lane_mode, t.track);
     const int grid = static_cast<int>(std::min<int64_t>((t.n_tiles + 7) / 8, static_cast<int64_t>(sms) * per_sm));
     qk::Moments m[QK_MAX_PAYOFFS];
     cudaError_t e = cudaMemcpyAsync(d_task, &t, sizeof(t), cudaMemcpyHostToDevice, st);
@@ -133,7 +133,7 @@ extern "C" qk_status qk_price_noalloc(const qk_contract *c, void *stream, qk_res
     if (e == cudaSuccess) e = cudaMemsetAsync(d_cursor, 0, sizeof(unsigned long long), st);  // queue starts empty
     if (e == cudaSuccess)
         e = qk::launch_price_tiles(t.precision, t.model, t.scheme, std::max(grid, 1), st, d_task, d_prefix, 1, 0,
-                                   t.n_tiles, d_cursor, d_partials, true, c->seed, t.lane_mode, t.track != 0);
+                                   t.n_tiles, d_cursor, d_partials, true, c->seed, t.lane_mode, t.track);
     if (e == cudaSuccess) e = qk::launch_merge_tasks(1, st, d_task, d_partials, d_moments);
     if (e == cudaSuccess) e = cudaMemcpyAsync(m, d_moments, sizeof(m), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);

@@ -175,16 +175,20 @@ __device__ __noinline__ double2 jump_log2_f64(uint32_t word, double L, double mu
 // FP64 paths: NP paths of one lane (1; 2: an antithetic pair, NEG, or two independent
 // paths), stepped on the logarithm of the spot (step64).  Sums, maxima and minima are
 // those of S / S0; st holds the spot's on return.
-template <int MODEL, int SCHEME, bool TRK, int NP, bool NEG, class Gen, class Sink>
+template <int MODEL, int SCHEME, int TRK, int NP, bool NEG, class Gen, class Sink>
 __device__ __forceinline__ void simulate_f64(const Tab64 &tab, const StepConst<double> &p, double S0, double v0,
                                              int n_steps, const Gen &gen, uint32_t k0, uint32_t k1, uint32_t path,
                                              uint32_t stream, uint32_t kmin, PathState<double> (&st)[NP], Sink &&sink) {
+    // the running maximum and minimum: of x itself where x is the whole logarithm (no
+    // exponential a step), of the relative spot with QE, whose martingale product is apart
+    constexpr bool kLogRange = SCHEME != kQE;
+    constexpr bool kSpot = (TRK & kTrackSum) || ((TRK & kTrackRange) && !kLogRange);
     Path64 s[NP];
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
         s[i] = Path64{0.0, 1.0, v0};
         st[i].ssum = 0.0;
-        st[i].smax = st[i].smin = 1.0;
+        st[i].smax = st[i].smin = kLogRange ? 0.0 : 1.0;
     }
     constexpr int ND = NEG ? 1 : NP;  // draw sequences
     PhiloxPath pp[ND];
@@ -227,9 +231,11 @@ __device__ __forceinline__ void simulate_f64(const Tab64 &tab, const StepConst<d
             }
 #pragma unroll
             for (int i = 0; i < NP; ++i) {
-                if constexpr (TRK) {
-                    const double r = rel_spot64<SCHEME>(tab, s[i]);
-                    blk[i] += r;
+                double r = s[i].x;
+                if constexpr (kSpot) r = rel_spot64<SCHEME>(tab, s[i]);
+                if constexpr (TRK & kTrackSum) blk[i] += r;
+                if constexpr (TRK & kTrackRange) {
+                    if constexpr (kLogRange) r = s[i].x;
                     st[i].smax = r > st[i].smax ? r : st[i].smax;
                     st[i].smin = r < st[i].smin ? r : st[i].smin;
                 }
@@ -250,7 +256,7 @@ __device__ __forceinline__ void simulate_f64(const Tab64 &tab, const StepConst<d
         }
 #pragma unroll
         for (int i = 0; i < NP; ++i) {
-            if constexpr (TRK) st[i].ssum += blk[i];
+            if constexpr (TRK & kTrackSum) st[i].ssum += blk[i];
             fold64<SCHEME>(tab, s[i]);
         }
     }
@@ -258,19 +264,16 @@ __device__ __forceinline__ void simulate_f64(const Tab64 &tab, const StepConst<d
     for (int i = 0; i < NP; ++i) {
         st[i].S = S0 * exp2_64(tab, s[i].x);
         st[i].v = s[i].v;
-        if constexpr (TRK) {
-            st[i].ssum *= S0;
-            st[i].smax *= S0;
-            st[i].smin *= S0;
-        } else {
-            st[i].smax = st[i].smin = st[i].S;
+        if constexpr (TRK & kTrackSum) st[i].ssum *= S0;
+        if constexpr (TRK & kTrackRange) {
+            st[i].smax = S0 * (kLogRange ? exp2_64(tab, st[i].smax) : st[i].smax);
+            st[i].smin = S0 * (kLogRange ? exp2_64(tab, st[i].smin) : st[i].smin);
         }
     }
 }
 
-// TRK: keep the path state that Asian, barrier and lookback legs read (running sum,
-// max, min); false for launches whose legs read only the final spot.
-template <class R, int MODEL, int SCHEME, bool TRK = true, class Gen, class Sink>
+// TRK: the path state to keep (kTrack*).
+template <class R, int MODEL, int SCHEME, int TRK = kTrackAll, class Gen, class Sink>
 __device__ __forceinline__ void simulate_path(const Tab64 *tab, const StepConst<R> &p, R S0, R v0, int n_steps,
                                               const Gen &gen, uint32_t k0, uint32_t k1, uint32_t path, uint32_t stream,
                                               uint32_t kmin, PathState<R> &st, Sink &&sink) {
@@ -395,7 +398,7 @@ __device__ __forceinline__ void step_two_z_f32(const Term &tt, const StepConst<f
 // between the 16-step blocks that add to them: this thread's shared-memory slot (two
 // FP64 sums read and written once per block, four registers fewer in the step loop),
 // or nullptr for a.ssum and b.ssum.
-template <int MODEL, int SCHEME, bool NEG, bool TRK = true, class Term, class Gen, class Sink2>
+template <int MODEL, int SCHEME, bool NEG, int TRK = kTrackAll, class Term, class Gen, class Sink2>
 __device__ __forceinline__ void simulate_two(const Term &tt, const StepConst<float> &p, float S0, float v0, int n_steps, const Gen &gen,
                                              uint32_t k0, uint32_t k1, uint32_t path_a, uint32_t path_b,
                                              uint32_t stream, uint32_t kmin, PathState<float> &a, PathState<float> &b,
@@ -519,7 +522,7 @@ __device__ __forceinline__ int find_task(const int64_t *__restrict__ prefix, int
 // Blocks of 128, 256 or 512 threads (FP32; up to 256 in FP64): the register budget is
 // set for kPathMinBlocksFp32 resident 256-thread blocks per SM (64 registers a thread).
 // TAB: one FP32 QE task, its term table in dynamic shared memory.
-template <class R, int MODEL, int SCHEME, bool UK, int LANE, bool TRK, bool TAB = false>
+template <class R, int MODEL, int SCHEME, bool UK, int LANE, int TRK, bool TAB = false>
 __global__ void __launch_bounds__(path_block_max<R>(),
                                   sizeof(R) == 4 ? kPathMinBlocksFp32 * kPathBlock / path_block_max<R>()
                                                  : (SCHEME == kQE ? kPathMinBlocksQe64 : kPathMinBlocks64))
@@ -532,7 +535,7 @@ __global__ void __launch_bounds__(path_block_max<R>(),
     __shared__ Moments s_acc[path_block_max<R>() / 32][QK_MAX_PAYOFFS];
     // the Asian running sums of a lane's two independent paths (simulate_two); one slot per
     // thread (antithetic pairs keep theirs in registers, which measures faster there)
-    constexpr bool kSumSlot = sizeof(R) == 4 && LANE == kLaneTwo && TRK;
+    constexpr bool kSumSlot = sizeof(R) == 4 && LANE == kLaneTwo && TRK != kTrackNone;
     __shared__ double2 s_ssum[kSumSlot ? path_block_max<R>() : 1];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -642,7 +645,7 @@ template <class R>
 using PriceKernel = void (*)(const TaskDev *, const int64_t *, int32_t, int64_t, int64_t, unsigned long long *,
                              Moments *, const PhiloxRoundKeys);
 
-template <class R, bool UK, int LANE, bool TRK>
+template <class R, bool UK, int LANE, int TRK>
 __host__ PriceKernel<R> price_kernel_for_keys(int model, int scheme) {
     switch (model * 3 + scheme) {
         case 0: return price_tiles_kernel<R, kHeston, kEuler, UK, LANE, TRK>;
@@ -655,26 +658,33 @@ __host__ PriceKernel<R> price_kernel_for_keys(int model, int scheme) {
 }
 
 // The kernel with a term table: FP32 QE, parameter keys, two paths per lane.
-PriceKernel<float> price_table_kernel_for(int model, bool track) {
+PriceKernel<float> price_table_kernel_for(int model, int track) {
     if (model == kHeston)
-        return track ? price_tiles_kernel<float, kHeston, kQE, true, kLaneTwo, true, true>
-                     : price_tiles_kernel<float, kHeston, kQE, true, kLaneTwo, false, true>;
-    return track ? price_tiles_kernel<float, kBates, kQE, true, kLaneTwo, true, true>
-                 : price_tiles_kernel<float, kBates, kQE, true, kLaneTwo, false, true>;
+        return track ? price_tiles_kernel<float, kHeston, kQE, true, kLaneTwo, kTrackAll, true>
+                     : price_tiles_kernel<float, kHeston, kQE, true, kLaneTwo, kTrackNone, true>;
+    return track ? price_tiles_kernel<float, kBates, kQE, true, kLaneTwo, kTrackAll, true>
+                 : price_tiles_kernel<float, kBates, kQE, true, kLaneTwo, kTrackNone, true>;
+}
+
+template <class R, bool UK, int LANE>
+__host__ PriceKernel<R> price_kernel_for_state(int model, int scheme, int track) {
+    if (track == kTrackNone) return price_kernel_for_keys<R, UK, LANE, kTrackNone>(model, scheme);
+    if constexpr (sizeof(R) == 8) {
+        if (track == kTrackSum) return price_kernel_for_keys<R, UK, LANE, kTrackSum>(model, scheme);
+        if (track == kTrackRange) return price_kernel_for_keys<R, UK, LANE, kTrackRange>(model, scheme);
+    }
+    return price_kernel_for_keys<R, UK, LANE, kTrackAll>(model, scheme);
 }
 
 template <class R, int LANE>
-__host__ PriceKernel<R> price_kernel_for_lane(int model, int scheme, bool uniform_key, bool track) {
-    if (track)
-        return uniform_key ? price_kernel_for_keys<R, true, LANE, true>(model, scheme)
-                           : price_kernel_for_keys<R, false, LANE, true>(model, scheme);
-    return uniform_key ? price_kernel_for_keys<R, true, LANE, false>(model, scheme)
-                       : price_kernel_for_keys<R, false, LANE, false>(model, scheme);
+__host__ PriceKernel<R> price_kernel_for_lane(int model, int scheme, bool uniform_key, int track) {
+    return uniform_key ? price_kernel_for_state<R, true, LANE>(model, scheme, track)
+                       : price_kernel_for_state<R, false, LANE>(model, scheme, track);
 }
 
 template <class R>
 __host__ PriceKernel<R> price_kernel_for(int model, int scheme, bool uniform_key = true, int lane_mode = kLaneOne,
-                                         bool track = true) {
+                                         int track = kTrackAll) {
     switch (lane_mode) {
         case kLanePair: return price_kernel_for_lane<R, kLanePair>(model, scheme, uniform_key, track);
         case kLaneTwo: return price_kernel_for_lane<R, kLaneTwo>(model, scheme, uniform_key, track);
@@ -836,7 +846,7 @@ __global__ void __launch_bounds__(kPathBlock, sizeof(R) == 4 ? kPathMinBlocksFp3
         const int64_t i = std::min(i0 + lane, count - 1);
         SlabSink<R> sink{slab_S, slab_v, ld, i, stride, stride};
         PathState<R> st;
-        simulate_path<R, MODEL, SCHEME, false>(tables.get(), p, static_cast<R>(t.S0), static_cast<R>(t.v0), t.n_steps, gen,
+        simulate_path<R, MODEL, SCHEME, kTrackNone>(tables.get(), p, static_cast<R>(t.S0), static_cast<R>(t.v0), t.n_steps, gen,
                                                t.key0, t.key1, static_cast<uint32_t>(first_path + i), t.stream,
                                                task_kmin<R>(t), st, sink);
     }
@@ -866,7 +876,7 @@ __global__ void __launch_bounds__(kPathBlock, kPathMinBlocksFp32)
     SlabSink2<float> sink{slab_S, slab_v, ld, i, stride, stride, i + 1 < count};
     PathState<float> sa, sb;
     const uint32_t pa = static_cast<uint32_t>(first_path + i);
-    simulate_two<MODEL, SCHEME, false, false>(tt, p, static_cast<float>(t.S0), static_cast<float>(t.v0), t.n_steps, gen,
+    simulate_two<MODEL, SCHEME, false, kTrackNone>(tt, p, static_cast<float>(t.S0), static_cast<float>(t.v0), t.n_steps, gen,
                                               t.key0, t.key1, pa, pa + 1u, t.stream, t.jump_kmin, sa, sb, sink);
 }
 
@@ -898,7 +908,7 @@ SlabKernel<R> slab_kernel_for(int model, int scheme) {
 
 // Per-path payoff of leg 0 (undiscounted, normalised units), for the payoff
 // distribution analysis (OptionPricer.hpp:340-360 sorts every path's payoff).
-template <class R, int MODEL, int SCHEME, bool TRK>
+template <class R, int MODEL, int SCHEME, int TRK>
 __global__ void __launch_bounds__(kPayoffBlock, 2 * (sizeof(R) == 4 ? kPathMinBlocksFp32
                                                      : SCHEME == kQE ? kPathMinBlocksQe64 : kPathMinBlocks64))
     payoff_paths_kernel(const TaskDev *__restrict__ task, int64_t first, int64_t count, double *__restrict__ out,
@@ -929,8 +939,8 @@ __global__ void __launch_bounds__(kPayoffBlock, 2 * (sizeof(R) == 4 ? kPathMinBl
 template <class R>
 using PayoffKernel = void (*)(const TaskDev *, int64_t, int64_t, double *, const PhiloxRoundKeys);
 
-template <class R, bool TRK>
-PayoffKernel<R> payoff_kernel_for(int model, int scheme) {
+template <class R, int TRK>
+PayoffKernel<R> payoff_kernel_for_state(int model, int scheme) {
     switch (model * 3 + scheme) {
         case 0: return payoff_paths_kernel<R, kHeston, kEuler, TRK>;
         case 1: return payoff_paths_kernel<R, kHeston, kMilstein, TRK>;
@@ -939,6 +949,15 @@ PayoffKernel<R> payoff_kernel_for(int model, int scheme) {
         case 4: return payoff_paths_kernel<R, kBates, kMilstein, TRK>;
         default: return payoff_paths_kernel<R, kBates, kQE, TRK>;
     }
+}
+template <class R>
+PayoffKernel<R> payoff_kernel_for(int model, int scheme, int track) {
+    if (track == kTrackNone) return payoff_kernel_for_state<R, kTrackNone>(model, scheme);
+    if constexpr (sizeof(R) == 8) {
+        if (track == kTrackSum) return payoff_kernel_for_state<R, kTrackSum>(model, scheme);
+        if (track == kTrackRange) return payoff_kernel_for_state<R, kTrackRange>(model, scheme);
+    }
+    return payoff_kernel_for_state<R, kTrackAll>(model, scheme);
 }
 
 // Payoff of one leg on a fed spot sequence S_1..S_n (one thread): the path kernel's
@@ -1005,7 +1024,7 @@ __global__ void step_trace_kernel(const TaskDev *__restrict__ task, const double
 cudaError_t launch_price_tiles(int precision, int model, int scheme, int grid, cudaStream_t s, const TaskDev *tasks,
                                const int64_t *prefix, int32_t n_tasks, int64_t slot_begin, int64_t slot_end,
                                unsigned long long *cursor, Moments *partials, bool uniform_key, uint64_t seed,
-                               int lane_mode, bool track, int block, bool table) {
+                               int lane_mode, int track, int block, bool table) {
     if (!price_tiles_block_ok(precision, block)) return cudaErrorInvalidConfiguration;
     const PhiloxRoundKeys rk = philox_round_keys(static_cast<uint32_t>(seed & 0xFFFFFFFFull),
                                                  static_cast<uint32_t>(seed >> 32));
@@ -1090,15 +1109,15 @@ cudaError_t launch_step_trace(int precision, cudaStream_t s, const TaskDev *task
     return cudaGetLastError();
 }
 
-cudaError_t launch_payoff_paths(int precision, int model, int scheme, bool track, uint64_t seed, int sm_count,
+cudaError_t launch_payoff_paths(int precision, int model, int scheme, int track, uint64_t seed, int sm_count,
                                 cudaStream_t s, const TaskDev *task, int64_t first, int64_t count, double *out) {
     const PhiloxRoundKeys rk = philox_round_keys(static_cast<uint32_t>(seed & 0xFFFFFFFFull),
                                                  static_cast<uint32_t>(seed >> 32));
     const int64_t blocks = (count + kPayoffBlock - 1) / kPayoffBlock;
     const unsigned grid = static_cast<unsigned>(std::min<int64_t>(blocks, static_cast<int64_t>(sm_count) * 8));
     const auto launch = [&](auto kernel) { kernel<<<grid, kPayoffBlock, 0, s>>>(task, first, count, out, rk); };
-    if (precision == QK_FP32) launch(track ? payoff_kernel_for<float, true>(model, scheme) : payoff_kernel_for<float, false>(model, scheme));
-    else launch(track ? payoff_kernel_for<double, true>(model, scheme) : payoff_kernel_for<double, false>(model, scheme));
+    if (precision == QK_FP32) launch(payoff_kernel_for<float>(model, scheme, track));
+    else launch(payoff_kernel_for<double>(model, scheme, track));
     return cudaGetLastError();
 }
 
@@ -1150,13 +1169,13 @@ static cudaError_t preload_path_kernels_of() {
         for (int scheme = 0; scheme < 3 && e == cudaSuccess; ++scheme) {
             for (int uk = 0; uk < 2 && e == cudaSuccess; ++uk)
                 for (int lane = 0; lane < 3 && e == cudaSuccess; ++lane)
-                    for (int trk = 0; trk < 2 && e == cudaSuccess; ++trk)
-                        e = cudaFuncGetAttributes(&fa, price_kernel_for<R>(model, scheme, uk != 0, lane, trk != 0));
+                    for (int trk = 0; trk < 4 && e == cudaSuccess; ++trk)
+                        e = cudaFuncGetAttributes(&fa, price_kernel_for<R>(model, scheme, uk != 0, lane, trk));
             if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, slab_kernel_for<R>(model, scheme));
             for (int tab = 0; tab < 2 && e == cudaSuccess; ++tab)
                 e = cudaFuncGetAttributes(&fa, slab_two_kernel_for(model, scheme, tab != 0));
-            if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, payoff_kernel_for<R, true>(model, scheme));
-            if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, payoff_kernel_for<R, false>(model, scheme));
+            for (int trk = 0; trk < 4 && e == cudaSuccess; ++trk)
+                e = cudaFuncGetAttributes(&fa, payoff_kernel_for<R>(model, scheme, trk));
         }
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, payoff_trace_kernel<R>);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, step_trace_kernel<R>);
@@ -1170,7 +1189,7 @@ cudaError_t preload_path_kernels() {
     const int table_bytes = (kTermTableMax + 1) * static_cast<int>(sizeof(float2));
     for (int model = 0; model < 2 && e == cudaSuccess; ++model) {
         for (int trk = 0; trk < 2 && e == cudaSuccess; ++trk)
-            e = cudaFuncSetAttribute(price_table_kernel_for(model, trk != 0), cudaFuncAttributeMaxDynamicSharedMemorySize,
+            e = cudaFuncSetAttribute(price_table_kernel_for(model, trk), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      table_bytes);
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(slab_two_kernel_for(model, kQE, true), cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1189,25 +1208,25 @@ cudaError_t preload_noalloc_kernels() {
     cudaError_t e = cudaFuncGetAttributes(&fa, merge_tasks_kernel);
     for (int model = 0; model < 2 && e == cudaSuccess; ++model)
         for (int scheme = 0; scheme < 3 && e == cudaSuccess; ++scheme)
-            for (int trk = 0; trk < 2 && e == cudaSuccess; ++trk) {
-                e = cudaFuncGetAttributes(&fa, price_kernel_for<float>(model, scheme, true, kLaneOne, trk != 0));
+            for (int trk = 0; trk < 4 && e == cudaSuccess; ++trk) {
+                e = cudaFuncGetAttributes(&fa, price_kernel_for<float>(model, scheme, true, kLaneOne, trk));
                 if (e == cudaSuccess)
-                    e = cudaFuncGetAttributes(&fa, price_kernel_for<double>(model, scheme, true, kLaneOne, trk != 0));
+                    e = cudaFuncGetAttributes(&fa, price_kernel_for<double>(model, scheme, true, kLaneOne, trk));
             }
     return e;
 }
 
-int price_tiles_max_blocks_per_sm(int precision, int model, int scheme, int lane_mode, bool track, int block) {
+int price_tiles_max_blocks_per_sm(int precision, int model, int scheme, int lane_mode, int track, int block) {
     // answered once per device, kernel variant and block size on each host thread
     // (planning asks for every contract of every call)
-    constexpr int kDevs = 16, kVariants = 2 * 2 * 3 * 3 * 2 * 3;
+    constexpr int kDevs = 16, kVariants = 2 * 2 * 3 * 3 * 4 * 3;
     static thread_local int cache[kDevs][kVariants] = {};
     int dev = 0;
     const int bidx = block == 128 ? 0 : (block == 256 ? 1 : (block == 512 ? 2 : -1));
     int *slot = nullptr;
     if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kDevs && bidx >= 0 && precision >= 0 &&
         precision < 2 && model >= 0 && model < 2 && scheme >= 0 && scheme < 3 && lane_mode >= 0 && lane_mode < 3) {
-        slot = &cache[dev][((((precision * 2 + model) * 3 + scheme) * 3 + lane_mode) * 2 + (track ? 1 : 0)) * 3 + bidx];
+        slot = &cache[dev][((((precision * 2 + model) * 3 + scheme) * 3 + lane_mode) * 4 + (track & 3)) * 3 + bidx];
         if (*slot > 0) return *slot;
     }
     int nb = 0;
