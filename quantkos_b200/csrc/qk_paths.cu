@@ -155,13 +155,13 @@ __device__ __forceinline__ void one_step_z(const StepConst<float> &p, PathState<
 
 // FP64 jumps: log2 of the jump factor of a step whose first Poisson word reached the
 // threshold, with the jump normal as drawn (x) and negated (y, antithetic pairs); 0 if the
-// exact test finds no jump.  Arguments by value: nothing of the caller's state has to live
-// in memory for this rare call.
-__device__ __noinline__ double2 jump_log2_f64(uint32_t word, double L, double mu_j, double sigma_j, uint32_t k0,
-                                              uint32_t k1, uint32_t path, uint32_t stream, uint32_t n) {
+// exact test finds no jump.  What only this rare call needs it reads from the task's
+// descriptor, so that none of it takes registers in the path loop.
+__device__ __noinline__ double2 jump_log2_f64(const TaskDev &t, uint32_t word, uint32_t path, uint32_t n) {
+    const double L = t.cd.exp_m_lambda_dt, mu_j = t.cd.mu_j, sigma_j = t.cd.sigma_j;
     double prod = Math<double>::u01(word);
     if (!(prod >= L)) return make_double2(0.0, 0.0);
-    PhiloxJumpDraws<double> d{k0, k1, path, stream, n, prod, 1, 0, U4{0, 0, 0, 0}};
+    PhiloxJumpDraws<double> d{t.key0, t.key1, path, t.stream, n, prod, 1, 0, U4{0, 0, 0, 0}};
     int N = 0;
     do {
         ++N;
@@ -176,9 +176,11 @@ __device__ __noinline__ double2 jump_log2_f64(uint32_t word, double L, double mu
 // paths), stepped on the logarithm of the spot (step64).  Sums, maxima and minima are
 // those of S / S0; st holds the spot's on return.
 template <int MODEL, int SCHEME, int TRK, int NP, bool NEG, class Gen, class Sink>
-__device__ __forceinline__ void simulate_f64(const Tab64 &tab, const StepConst<double> &p, double S0, double v0,
-                                             int n_steps, const Gen &gen, uint32_t k0, uint32_t k1, uint32_t path,
-                                             uint32_t stream, uint32_t kmin, PathState<double> (&st)[NP], Sink &&sink) {
+__device__ __forceinline__ void simulate_f64(const Tab64 &tab, const StepConst<double> &p, const TaskDev &t,
+                                             const Gen &gen, uint32_t path, PathState<double> (&st)[NP], Sink &&sink) {
+    const double S0 = t.S0, v0 = t.v0;
+    const int n_steps = t.n_steps;
+    const uint32_t kmin = t.jump_kmin64;
     // the running maximum and minimum: of x itself where x is the whole logarithm (no
     // exponential a step), of the relative spot with QE, whose martingale product is apart
     constexpr bool kLogRange = SCHEME != kQE;
@@ -222,8 +224,7 @@ __device__ __forceinline__ void simulate_f64(const Tab64 &tab, const StepConst<d
                     // word n mod 4 of the domain-2 block
                     const uint32_t word = (n & 2) ? (odd ? wp[i].w : wp[i].z) : (odd ? wp[i].y : wp[i].x);
                     if (word >= kmin) {
-                        const double2 j = jump_log2_f64(word, p.exp_m_lambda_dt, p.mu_j, p.sigma_j, k0, k1, path + i,
-                                                        stream, static_cast<uint32_t>(n));
+                        const double2 j = jump_log2_f64(t, word, path + i, static_cast<uint32_t>(n));
                         s[i].x += j.x;
                         if constexpr (NEG) s[1].x += j.y;
                     }
@@ -274,14 +275,16 @@ __device__ __forceinline__ void simulate_f64(const Tab64 &tab, const StepConst<d
 
 // TRK: the path state to keep (kTrack*).
 template <class R, int MODEL, int SCHEME, int TRK = kTrackAll, class Gen, class Sink>
-__device__ __forceinline__ void simulate_path(const Tab64 *tab, const StepConst<R> &p, R S0, R v0, int n_steps,
-                                              const Gen &gen, uint32_t k0, uint32_t k1, uint32_t path, uint32_t stream,
-                                              uint32_t kmin, PathState<R> &st, Sink &&sink) {
+__device__ __forceinline__ void simulate_path(const Tab64 *tab, const StepConst<R> &p, const TaskDev &t, const Gen &gen,
+                                              uint32_t path, PathState<R> &st, Sink &&sink) {
     if constexpr (sizeof(R) == 8) {
         PathState<double> one[1];
-        simulate_f64<MODEL, SCHEME, TRK, 1, false>(*tab, p, S0, v0, n_steps, gen, k0, k1, path, stream, kmin, one, sink);
+        simulate_f64<MODEL, SCHEME, TRK, 1, false>(*tab, p, t, gen, path, one, sink);
         st = one[0];
     } else {
+        const float S0 = static_cast<float>(t.S0), v0 = static_cast<float>(t.v0);
+        const int n_steps = t.n_steps;
+        const uint32_t k0 = t.key0, k1 = t.key1, stream = t.stream, kmin = t.jump_kmin;
         st.S = S0;
         st.v = v0;
         st.ssum = 0.0;
@@ -598,8 +601,7 @@ __global__ void __launch_bounds__(path_block_max<R>(),
                 with_keys([&](const auto &gen) {
                     if constexpr (sizeof(R) == 8) {
                         PathState<double> two[2];
-                        simulate_f64<MODEL, SCHEME, TRK, 2, NEG>(*tables.get(), p, S0, v0, n_steps, gen, k0, k1, pa, stream,
-                                                                 kmin, two, NoSink{});
+                        simulate_f64<MODEL, SCHEME, TRK, 2, NEG>(*tables.get(), p, t, gen, pa, two, NoSink{});
                         sa = two[0];
                         sb = two[1];
                     } else {
@@ -624,8 +626,7 @@ __global__ void __launch_bounds__(path_block_max<R>(),
             } else {
                 PathState<R> st;
                 with_keys([&](const auto &gen) {
-                    simulate_path<R, MODEL, SCHEME, TRK>(tables.get(), p, S0, v0, n_steps, gen, k0, k1,
-                                                         static_cast<uint32_t>(unit), stream, kmin, st, NoSink{});
+                    simulate_path<R, MODEL, SCHEME, TRK>(tables.get(), p, t, gen, static_cast<uint32_t>(unit), st, NoSink{});
                 });
                 for (int k = 0; k < np; ++k) {
                     const PayoffSpec ps = t.pay[k];
@@ -846,9 +847,7 @@ __global__ void __launch_bounds__(kPathBlock, sizeof(R) == 4 ? kPathMinBlocksFp3
         const int64_t i = std::min(i0 + lane, count - 1);
         SlabSink<R> sink{slab_S, slab_v, ld, i, stride, stride};
         PathState<R> st;
-        simulate_path<R, MODEL, SCHEME, kTrackNone>(tables.get(), p, static_cast<R>(t.S0), static_cast<R>(t.v0), t.n_steps, gen,
-                                               t.key0, t.key1, static_cast<uint32_t>(first_path + i), t.stream,
-                                               task_kmin<R>(t), st, sink);
+        simulate_path<R, MODEL, SCHEME, kTrackNone>(tables.get(), p, t, gen, static_cast<uint32_t>(first_path + i), st, sink);
     }
 }
 
@@ -926,12 +925,7 @@ __global__ void __launch_bounds__(kPayoffBlock, 2 * (sizeof(R) == 4 ? kPathMinBl
         const int64_t i = i0 + lane;
         const uint32_t path = static_cast<uint32_t>(first + i);
         PathState<R> st;
-        if constexpr (sizeof(R) == 8)
-            simulate_path<R, MODEL, SCHEME, TRK>(tables.get(), p, t.S0, t.v0, t.n_steps, gen, t.key0, t.key1, path, t.stream,
-                                                 t.jump_kmin64, st, NoSink{});
-        else
-            simulate_path<R, MODEL, SCHEME, TRK>(tables.get(), p, static_cast<R>(t.S0), static_cast<R>(t.v0), t.n_steps, gen,
-                                                 t.key0, t.key1, path, t.stream, t.jump_kmin, st, NoSink{});
+        simulate_path<R, MODEL, SCHEME, TRK>(tables.get(), p, t, gen, path, st, NoSink{});
         if (i < count) out[i] = static_cast<double>(final_payoff<R>(t.pay[0], st.S, st.ssum, st.smax, st.smin, t.n_steps));
     }
 }
