@@ -654,6 +654,34 @@ qk_status run_plan(qk_handle *h, Plan &plan) {
     return QK_OK;
 }
 
+// A plan of one task, its paths' payoffs stored (`payoffs`, n_paths values) and its tile
+// records formed from them: one simulation where the payoff distribution is wanted beside
+// the price.  FP64 Heston QE Asian, 100,000 x 128, with percentiles: 468 us with a second
+// simulation for the payoffs, 326 us.
+static qk_status run_plan_storing_payoffs(qk_handle *h, const Plan &plan, double *payoffs) {
+    const TaskDev &t = plan.tasks[0];
+    h->launches = 0;
+    h->h2d_bytes = static_cast<int64_t>(plan_bytes(1));
+    h->d2h_bytes = static_cast<int64_t>(QK_MAX_PAYOFFS * sizeof(Moments));
+    QK_CUDA_TRY(cudaEventRecord(h->ev_start, h->stream));
+    const qk_status s = upload_plan(h, plan);
+    if (s != QK_OK) return s;
+    char *plan_base = static_cast<char *>(h->d_tasks.ptr);
+    const TaskDev *dt = reinterpret_cast<const TaskDev *>(plan_base);
+    Moments *dpart = static_cast<Moments *>(h->d_partials.ptr);
+    const uint64_t seed = static_cast<uint64_t>(t.key0) | (static_cast<uint64_t>(t.key1) << 32);
+    QK_CUDA_TRY(cudaEventRecord(h->ev_paths0, h->stream));
+    QK_CUDA_TRY(launch_payoff_paths(t.precision, t.model, t.scheme, t.track, seed, h->sm_count, h->stream, dt, 0,
+                                    t.n_paths, payoffs));
+    QK_CUDA_TRY(launch_payoff_moments(t.precision, h->stream, dt, t.n_tiles, payoffs, dpart));
+    h->launches += 2;
+    QK_CUDA_TRY(cudaEventRecord(h->ev_paths1, h->stream));
+    QK_CUDA_TRY(launch_merge(1, plan.total_chunks, h->stream, dt, dpart, static_cast<Moments *>(h->d_chunks.ptr),
+                             static_cast<Moments *>(h->h_moments.ptr),
+                             reinterpret_cast<unsigned long long *>(plan_base + plan_cursor_at(1)), &h->launches));
+    return QK_OK;
+}
+
 void release_prepared(qk_handle *h) {
     if (h->graph) cudaGraphExecDestroy(h->graph);
     h->graph = nullptr;
@@ -836,7 +864,7 @@ qk_status finish_timing(qk_handle *h, double path_steps) {
 }
 
 qk_status price_contracts(qk_handle *h, const qk_contract *c, int32_t n, const qk_greeks *gs, qk_result *out,
-                              bool plain) {
+                          bool plain, PayoffRanks *dist) {
     if (!h || !c || !out || n < 0) return fail(QK_ERR_INVALID_ARG, "NULL argument or negative count");
     QK_CUDA_TRY(cudaSetDevice(h->device));
     release_prepared(h);  // the plan and arenas are about to change
@@ -845,12 +873,35 @@ qk_status price_contracts(qk_handle *h, const qk_contract *c, int32_t n, const q
     h->lsm_ms = h->lsm_paths_ms = 0.0;
     h->lsm_launches = 0;
     h->lsm_jobs = 0;
-    if ((s = run_plan(h, h->plan)) != QK_OK) return s;
+    // antithetic tasks keep no payoffs per path; a plan in another precision than the
+    // contract's (the plain method on an FP32 contract) simulates other payoffs
+    const bool with_payoffs = dist && h->plan.tasks.size() == 1 && h->plan.american.empty() &&
+                              h->plan.tasks[0].lane_mode != kLanePair && h->plan.tasks[0].precision == c->precision;
+    double *payoffs = nullptr;
+    const size_t select_bytes = select_scratch_bytes(), head = select_bytes + 256;  // its state, then its results
+    if (with_payoffs) {
+        if ((s = h->d_trace.ensure(head + static_cast<size_t>(h->plan.tasks[0].n_paths) * sizeof(double))) != QK_OK)
+            return s;
+        payoffs = reinterpret_cast<double *>(static_cast<char *>(h->d_trace.ptr) + head);
+        s = run_plan_storing_payoffs(h, h->plan, payoffs);
+    } else {
+        s = run_plan(h, h->plan);
+    }
+    if (s != QK_OK) return s;
     std::vector<Moments> lsm_moments;
     if (!h->plan.american.empty()) {
         if ((s = run_lsm_contracts(h, h->plan, plain, lsm_moments)) != QK_OK) return s;
     }
     QK_CUDA_TRY(cudaEventRecord(h->ev_end, h->stream));
+    if (with_payoffs) {
+        char *base = static_cast<char *>(h->d_trace.ptr);
+        double *dr = reinterpret_cast<double *>(base + select_bytes);
+        QK_CUDA_TRY(launch_select(h->stream, h->sm_count, payoffs, h->plan.tasks[0].n_paths, dist->ranks, dist->n_ranks,
+                                  base, dr));
+        QK_CUDA_TRY(cudaMemcpyAsync(dist->out, dr, static_cast<size_t>(dist->n_ranks) * sizeof(double),
+                                    cudaMemcpyDeviceToHost, h->stream));
+        dist->done = true;
+    }
     QK_CUDA_TRY(cudaStreamSynchronize(h->stream));
     if ((s = assemble_results(h, h->plan, static_cast<const Moments *>(h->h_moments.ptr), out)) != QK_OK) return s;
     if (!h->plan.american.empty()) assemble_lsm_results(h, h->plan, lsm_moments, out);

@@ -513,11 +513,21 @@ qk_status qk_run_config(qk_handle *h, const qk_config *cfg, qk_result *out, doub
     qk_contract k;
     qk_greeks g;
     QK_TRY(qk_config_to_contract(&c, &k, &g));
-    if (c.engine == 0) {
-        QK_TRY(qk_price_plain(h, &k, g.mask ? &g : nullptr, out));
-    } else {
-        QK_TRY(qk_price_batch(h, &k, 1, g.mask ? &g : nullptr, out));
+    if (!g.mask) std::memset(&g, 0, sizeof(g));
+    // OptionPricer::analyze_risk_neutral_discounted_payoff_distribution: 15 order statistics
+    // of all payoffs.  Without Greeks they come from the pricing's own paths.
+    const bool distribution = c.analyze_distribution && pct && k.payoffs[0].type != QK_AMERICAN;
+    double order[15];
+    qk::PayoffRanks dist;
+    if (distribution) {
+        const double N = static_cast<double>(k.n_paths);
+        const double fr[13] = {0.01, 0.05, 0.10, 0.20, 0.30, 0.40, 0.50, 0.60, 0.70, 0.80, 0.90, 0.95, 0.99};
+        for (int i = 0; i < 13; ++i) dist.ranks.r[i + 1] = static_cast<size_t>(N * fr[i]);
+        dist.ranks.r[14] = static_cast<size_t>(k.n_paths) - 1;
+        dist.n_ranks = 15;
+        dist.out = order;
     }
+    QK_TRY(qk::price_contracts(h, &k, 1, &g, out, c.engine == 0, distribution && !g.mask ? &dist : nullptr));
     const double scale = k.normalize ? k.S0 : 1.0;
     if (c.paths_file[0] != '\0') {
         const std::string path = (std::filesystem::path(c.out_dir) / c.paths_file).string();
@@ -529,17 +539,10 @@ qk_status qk_run_config(qk_handle *h, const qk_config *cfg, qk_result *out, doub
         h->timing = keep;
         if (st != QK_OK) return st;
     }
-    if (c.analyze_distribution && pct && k.payoffs[0].type != QK_AMERICAN) {
-        // OptionPricer::analyze_risk_neutral_discounted_payoff_distribution: 15 order statistics
-        // of all payoffs, discount and scale applied.
-        const double N = static_cast<double>(k.n_paths);
+    if (distribution) {
+        if (!dist.done) QK_TRY(qk::payoff_order_statistics(h, k, dist.ranks, dist.n_ranks, order));
         const double eff = std::exp(-k.r * k.T) * ((k.payoffs[0].type == QK_BINARY_CASH) ? 1.0 : scale);
-        const double fr[13] = {0.01, 0.05, 0.10, 0.20, 0.30, 0.40, 0.50, 0.60, 0.70, 0.80, 0.90, 0.95, 0.99};
-        qk::SelectRanks ranks = {};
-        for (int i = 0; i < 13; ++i) ranks.r[i + 1] = static_cast<size_t>(N * fr[i]);
-        ranks.r[14] = static_cast<size_t>(k.n_paths) - 1;
-        QK_TRY(qk::payoff_order_statistics(h, k, ranks, 15, pct));
-        for (int i = 0; i < 15; ++i) pct[i] *= eff;
+        for (int i = 0; i < 15; ++i) pct[i] = order[i] * eff;
     }
     return QK_OK;
 }

@@ -134,9 +134,21 @@ qk_contract normalised(const qk_contract &c, double *scale);
 qk_contract bumped(const qk_contract &n, const qk_greeks *g, int role);
 std::vector<int> roles_for(const qk_greeks *g, double T);
 
+// Order statistics of a one-leg contract's payoffs (undiscounted, normalised) wanted
+// beside its price: the values of n_ranks ascending ranks.
+struct PayoffRanks {
+    SelectRanks ranks = {};
+    int n_ranks = 0;
+    double *out = nullptr;
+    bool done = false;  // set by price_contracts when it answered them
+};
+
 // Plan, run and assemble a set of contracts; `gs` holds one Greeks request per
-// contract (or NULL).  Used by qk_price_* and by the serving lanes.
-qk_status price_contracts(qk_handle *h, const qk_contract *c, int32_t n, const qk_greeks *gs, qk_result *out, bool plain);
+// contract (or NULL).  Used by qk_price_* and by the serving lanes.  `dist` (one contract
+// of one leg): answered from the pricing's own paths where the plan is one task in the
+// contract's precision.
+qk_status price_contracts(qk_handle *h, const qk_contract *c, int32_t n, const qk_greeks *gs, qk_result *out, bool plain,
+                          PayoffRanks *dist = nullptr);
 
 // Memory held in a device's default pool (whose release threshold the handles raise so
 // that it keeps what it has mapped): pool_reserve maps `bytes` into it once (allocate and

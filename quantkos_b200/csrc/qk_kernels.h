@@ -60,6 +60,10 @@ cudaError_t launch_step_trace(int precision, cudaStream_t s, const TaskDev *task
 // track: the path state that leg reads (kTrack*).
 cudaError_t launch_payoff_paths(int precision, int model, int scheme, int track, uint64_t seed, int sm_count,
                                 cudaStream_t s, const TaskDev *task, int64_t first, int64_t count, double *out);
+// The pricing kernel's tile records of a one-leg task (one path or two independent paths
+// per lane) from the payoffs of all its paths.
+cudaError_t launch_payoff_moments(int precision, cudaStream_t s, const TaskDev *task, int32_t n_tiles,
+                                  const double *payoffs, Moments *partials);
 // Order statistics: the values of ascending ranks r[0..n_ranks-1] (0 = smallest) of x[0..n-1],
 // n < 2^32, into out[n_ranks] (device); scratch holds select_scratch_bytes().
 constexpr int kSelectRanks = 16;

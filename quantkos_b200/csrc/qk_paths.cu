@@ -954,6 +954,38 @@ PayoffKernel<R> payoff_kernel_for(int model, int scheme, int track) {
     return payoff_kernel_for_state<R, kTrackAll>(model, scheme);
 }
 
+// Tile records of a one-leg task from its paths' payoffs, a warp per tile: the pricing
+// kernel's records, in its order of operations (same bits), so that a run that needs every
+// payoff simulates once.  Reads 8 B per path: bound by launch latency below some ten million.
+__global__ void __launch_bounds__(256) payoff_moments_kernel(const TaskDev *__restrict__ task, double eps_payoff,
+                                                             const double *__restrict__ payoffs,
+                                                             Moments *__restrict__ partials) {
+    const TaskDev &t = *task;
+    const int lane = threadIdx.x & 31;
+    const int64_t tile = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (tile >= t.n_tiles) return;
+    const int64_t n_paths = t.n_paths, n_units = lane_units(n_paths, t.lane_mode);
+    const bool big = tile < t.n_big, two = t.lane_mode == kLaneTwo;
+    const int64_t first_round = big ? tile * t.ppt : static_cast<int64_t>(t.n_big) * t.ppt + (tile - t.n_big) * t.ppt_tail;
+    const int64_t last_round = std::min<int64_t>(first_round + (big ? t.ppt : t.ppt_tail),
+                                                 (n_units + kWarpTilePaths - 1) / kWarpTilePaths);
+    Moments acc{0.0, 0.0, 0.0, 0.0};
+    for (int64_t j = first_round; j < last_round; ++j) {
+        const int64_t unit = j * kWarpTilePaths + lane;
+        const int64_t a = two ? 2 * unit : unit;
+        const bool active = a < n_paths;
+        const double x = active ? payoffs[a] : 0.0;
+        Moments wm = warp_moments(x, active, x > eps_payoff);
+        if (two) {
+            const bool active_b = a + 1 < n_paths;
+            const double xb = active_b ? payoffs[a + 1] : 0.0;
+            wm = chan_merge(wm, warp_moments(xb, active_b, xb > eps_payoff));
+        }
+        acc = chan_merge(acc, wm);
+    }
+    if (lane == 0) partials[t.partial_base + tile] = acc;
+}
+
 // Payoff of one leg on a fed spot sequence S_1..S_n (one thread): the path kernel's
 // tracking (running max / min, the Asian sum in blocks of kSumChunk steps in the working
 // precision folded into FP64) and final_payoff, on the given values instead of simulated
@@ -1115,6 +1147,14 @@ cudaError_t launch_payoff_paths(int precision, int model, int scheme, int track,
     return cudaGetLastError();
 }
 
+cudaError_t launch_payoff_moments(int precision, cudaStream_t s, const TaskDev *task, int32_t n_tiles,
+                                  const double *payoffs, Moments *partials) {
+    // OptionPricer.hpp:316, in the payoffs' precision
+    const double eps = precision == QK_FP32 ? static_cast<double>(1e-6f) : 1e-12;
+    payoff_moments_kernel<<<(n_tiles + 7) / 8, 256, 0, s>>>(task, eps, payoffs, partials);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_payoff_trace(int precision, cudaStream_t s, const PayoffSpec &ps, const double *S, int n, double S0,
                                 double *out) {
     if (precision == QK_FP32)
@@ -1191,6 +1231,7 @@ cudaError_t preload_path_kernels() {
     }
     if (e == cudaSuccess) e = preload_path_kernels_of<double>();
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, merge_tasks_kernel);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, payoff_moments_kernel);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, merge_chunks_kernel);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, merge_task_chunks_kernel);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, sfu_probe_kernel);
