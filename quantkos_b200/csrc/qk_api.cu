@@ -215,6 +215,7 @@ static int path_state(const qk_contract &c, int precision) {
 // thousand; none where there are more than kTermTableMax.
 static uint32_t term_range_lo(const StepConst<float> &c) {
     if (!(c.h_psi_plain > 0.0f)) return 0;
+    if (!(c.theta_m > c.eps)) return 0;  // the kernels with a table take m = v e^{-k dt} + theta_m > eps as given
     const double r1 = static_cast<double>(c.h_f1) / c.exp_mkdt;
     const double r2 = c.theta_m > 0.0f ? static_cast<double>(c.h_f2) / c.theta_m : r1;
     const double a_lo = 0.5 * std::min(r1, r2);

@@ -101,6 +101,13 @@ inline StepConst<R> make_step_const(const qk_contract &c, double dt, double eps)
     const double a_max = std::max(d.h_f1 / d.exp_mkdt, d.theta_m > 0.0 ? d.h_f2 / d.theta_m : 0.0);
     const bool plain = 2.0 * (d.A + eps) * a_max <= 1.0 - 1.0 / 1024.0 && std::fabs(d.two_A) * a_max < 1e12;
     d.h_psi_plain = plain ? 0.5 * d.psi_c : -1.0;
+    // The paired FP32 step knows 2 / psi to 2^-21 (a reciprocal good to one unit in the last
+    // place, two roundings): within these bounds, 2^-18 inside the regime's, the one-path
+    // step's comparisons of s^2 give the quadratic regime too, and a step between the two
+    // takes the one-path step.  An infinite lower bound: no step takes the plain form.
+    constexpr double kInside = 1.0 / 262144.0;
+    d.ip_lo = plain && d.psi_c > 0.0 ? 2.0 / d.psi_c * (1.0 + kInside) : HUGE_VAL;
+    d.ip_hi = 2.0 / eps * (1.0 - kInside);
     if constexpr (sizeof(R) == sizeof(double)) {
         return d;
     } else {

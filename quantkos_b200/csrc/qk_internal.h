@@ -60,6 +60,7 @@ struct StepConst {
     R l_K2, l_A, l_c1, l_sqrt_K3;                  // QE: K2, A, -K3 / 2 (the coefficient of v), sqrt(K3) (K3 = K4)
     R h_f1, h_f2, h_eps, two_A;                    // QE: s^2 / 2 = v h_f1 + h_f2, eps / 2, 2 A
     R h_psi_plain;                                 // psi_c / 2, or -1 where A a could reach its clamp (make_step_const)
+    R ip_lo, ip_hi;                                // FP32 QE: bounds of 2 / psi in the plain quadratic regime
 };
 
 struct PayoffSpec {

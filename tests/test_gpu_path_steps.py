@@ -7,6 +7,8 @@ oracle; 1e-12 is asserted, as for the other FP64 path checks.  Next to zero vari
 (b + Z)^2 loses relative accuracy where b + Z cancels (b >= 0.7, so at most about 1e-12 of
 a variance that small moves the spot by far less); 1e-10 on the spot there.
 """
+import math
+
 import numpy as np
 import pytest
 
@@ -174,3 +176,32 @@ def test_results_on_both_sides_of_the_direct_write(qk, handle, n_contracts):
         prep.run()
         prep.run()
         assert [r["legs"] for r in prep.fetch()] == [r["legs"] for r in want]
+
+
+@pytest.mark.parametrize("psi,v0,theta", [(1.5, 1e-3, 1e-3), (1.5 * (1 - 2.0**-19), 1e-3, 1e-3), (1.5 * (1 + 2.0**-19), 1e-3, 1e-3),
+                                          (1e-6, 0.04, 0.04), (1e-6 * (1 + 2.0**-19), 0.04, 0.04), (0.5, 2e-6, 1e-7)])
+@pytest.mark.parametrize("n_paths", [65, 1_000_003])
+def test_qe_regime_bounds_keep_the_bits(qk, handle, n_paths, psi, v0, theta):
+    """Paths that start with psi next to psi_c = 3/2, next to eps = 1e-6, and with a mean next to
+    eps: two paths per lane (the regime from 2 / psi, with and without a term table) against the
+    one-path step's comparisons.  The same paths bit for bit, so prices differ by the order of the
+    FP64 merge alone."""
+    kappa, dt = 2.0, 0.004
+    e = math.exp(-kappa * dt)
+    m = v0 * e + theta * (1 - e)
+    s2 = v0 * e * (1 - e) / kappa + theta * (1 - e) ** 2 / (2 * kappa)  # over sigma^2
+    c = qk.make_contract(scheme=qk.ANDERSEN_QE, v0=v0, theta=theta, kappa=kappa, sigma=math.sqrt(psi * m * m / s2), rho=-0.5,
+                         n_steps=6, T=6 * dt, n_paths=n_paths, seed=77, precision=qk.FP32,
+                         payoffs=[qk.payoff(qk.EUROPEAN, qk.CALL, 100.0), qk.payoff(qk.LOOKBACK_FLOATING, qk.PUT, 100.0)])
+    out = []
+    try:
+        for lanes, block in ((1, 256), (2, 256), (2, 512)):
+            handle.tune_set(qk.FP32, qk.HESTON, qk.ANDERSEN_QE, 24, False, lanes, block_size=block)
+            out.append(qk.price_batch([c], None, handle)[0]["legs"])
+    finally:
+        handle.tune_reset()
+    for legs in out[1:]:
+        for a, b in zip(out[0], legs):
+            assert a["prob_itm"] == b["prob_itm"]
+            assert math.isclose(a["price"], b["price"], rel_tol=1e-11)
+            assert math.isclose(a["std_error"], b["std_error"], rel_tol=1e-11)
