@@ -50,7 +50,8 @@ METRIC = "path-steps/s"
 # sqrt(x(x-1)), rcp(1+b2), sqrt(b2), rcp(term), lg2(term); spot update
 # sqrt(K3 v + K4 v'), ex2.  The SFU pipe (16 lanes/clk/SM) then bounds the kernel
 # at (measured SFU op rate) / 12 path-steps/s; the FP32/integer work (Philox, the
-# QE algebra) fits under that bound on the 128-lane issue.
+# QE algebra) fits under that bound on the 128-lane issue.  A launch of one contract
+# reads two of the twelve (rcp(term), lg2(term)) from a table of the SFU's own results.
 SFU_PER_STEP = 12.0
 # Algorithmic scalar lane operations per path-step of the FP32 kinds (from the formulas
 # as implemented; one-path-per-lane count), for the issue-slot bound (every operation,
