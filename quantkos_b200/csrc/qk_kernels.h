@@ -65,7 +65,7 @@ cudaError_t launch_payoff_paths(int precision, int model, int scheme, int track,
 cudaError_t launch_payoff_moments(int precision, cudaStream_t s, const TaskDev *task, int32_t n_tiles,
                                   const double *payoffs, Moments *partials);
 // Order statistics: the values of ascending ranks r[0..n_ranks-1] (0 = smallest) of x[0..n-1],
-// n < 2^32, into out[n_ranks] (device); scratch holds select_scratch_bytes().
+// n < 2^32, into out[n_ranks] (device or pinned host memory); scratch holds select_scratch_bytes().
 constexpr int kSelectRanks = 16;
 struct SelectRanks {
     unsigned long long r[kSelectRanks];

@@ -22,7 +22,7 @@
 // its radius.  The tables (14 KB) live in shared memory, filled at the start of a kernel by
 // the block's threads with the CUDA functions: about 0.5 us, no table in global memory to
 // load.  Plain FP64 Heston Euler European, 1,048,576 x 252: 286 warp instructions per 32
-// path-steps and 2.77 ms with the library's functions on the spot, 109 and 1.25 ms with
+// path-steps and 2.77 ms with the library's functions on the spot, 106 and 1.21 ms with
 // these on its logarithm (FP64 pipe 53% busy in both, 52% now at less than half the work:
 // FP64 and the generator's wide multiplies share issue and register ports).
 #pragma once

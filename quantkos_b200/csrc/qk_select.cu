@@ -7,8 +7,8 @@
 // digit.  Exact: the selected values are elements of the array.  Bound by launch latency
 // for small arrays (nine launches) and by eight reads of the array for large ones.  A
 // configuration's run with percentiles (FP64 Asian, 100,000 x 128): 4.57 ms when every
-// payoff was copied to the host and sorted there, 0.49 ms (0.33 ms with the payoffs taken
-// from the pricing's own paths).
+// payoff was copied to the host and sorted there, 0.49 ms with a first form of these passes,
+// 0.27 ms now, with the payoffs taken from the pricing's own paths.
 #include <cuda_runtime.h>
 
 #include "qk_kernels.h"
@@ -38,18 +38,20 @@ constexpr int kSelectBlock = 256;
 __global__ void __launch_bounds__(kSelectBlock) select_pass_kernel(const double *__restrict__ x, int64_t n, int n_ranks,
                                                                    int pass, SelectState *st, double *__restrict__ out) {
     __shared__ unsigned int s_hist[kSelectRanks][256];
-    __shared__ unsigned long long s_prefix[kSelectRanks];
-    __shared__ int s_group[kSelectRanks + 1];  // first rank of each group; [n_groups] ends the list
+    __shared__ unsigned long long s_prefix[kSelectRanks];  // by group
+    __shared__ int s_group[kSelectRanks];                  // by rank
     __shared__ int s_n_groups;
     __shared__ bool s_last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) {
-        int g = 0;
-        for (int r = 0; r < n_ranks; ++r) {
-            s_prefix[r] = st->prefix[r];
-            if (r == 0 || s_prefix[r] != s_prefix[r - 1]) s_group[g++] = r;
-        }
-        s_n_groups = g;
+    if (warp == 0) {  // a lane per rank: one load latency
+        const unsigned long long p = lane < n_ranks ? st->prefix[lane] : 0ull;
+        const unsigned long long before = __shfl_up_sync(0xffffffffu, p, 1);
+        const bool first = lane < n_ranks && (lane == 0 || p != before);
+        const unsigned heads = __ballot_sync(0xffffffffu, first);
+        const int g = __popc(heads & (0xffffffffu >> (31 - lane))) - 1;
+        if (first) s_prefix[g] = p;
+        if (lane < n_ranks) s_group[lane] = g;
+        if (lane == 0) s_n_groups = __popc(heads);
     }
     for (int i = threadIdx.x; i < kSelectRanks * 256; i += kSelectBlock) (&s_hist[0][0])[i] = 0u;
     __syncthreads();
@@ -63,7 +65,7 @@ __global__ void __launch_bounds__(kSelectBlock) select_pass_kernel(const double 
         const unsigned long long head = pass == 0 ? 0ull : k >> (shift + 8);
         int bin = -1;
         for (int g = 0; g < groups; ++g)
-            if (have && head == s_prefix[s_group[g]]) bin = g * 256 + static_cast<int>((k >> shift) & 255u);
+            if (have && head == s_prefix[g]) bin = g * 256 + static_cast<int>((k >> shift) & 255u);
         const unsigned same = __match_any_sync(0xffffffffu, bin);
         if (bin >= 0 && lane == __ffs(same) - 1) atomicAdd(&s_hist[0][0] + bin, static_cast<unsigned>(__popc(same)));
     }
@@ -80,8 +82,7 @@ __global__ void __launch_bounds__(kSelectBlock) select_pass_kernel(const double 
     // last block: rank r's digit, a warp per rank, eight bins per lane
     __threadfence();
     for (int r = warp; r < n_ranks; r += kSelectBlock / 32) {
-        int g = 0;
-        while (g + 1 < groups && s_group[g + 1] <= r) ++g;
+        const int g = s_group[r];
         unsigned c[8], sum = 0;
         for (int j = 0; j < 8; ++j) sum += c[j] = __ldcg(&st->hist[g][8 * lane + j]);
         unsigned before = sum;  // inclusive, then exclusive, sum over the lanes
@@ -95,7 +96,7 @@ __global__ void __launch_bounds__(kSelectBlock) select_pass_kernel(const double 
             unsigned long long left = want - before;
             int j = 0;
             while (left >= c[j]) left -= c[j++];
-            const unsigned long long prefix = (pass == 0 ? 0ull : s_prefix[r] << 8) | static_cast<unsigned>(8 * lane + j);
+            const unsigned long long prefix = (pass == 0 ? 0ull : s_prefix[g] << 8) | static_cast<unsigned>(8 * lane + j);
             st->prefix[r] = prefix;
             st->rank[r] = left;
             if (pass == 7) out[r] = from_ordered_bits(prefix);
@@ -123,9 +124,12 @@ cudaError_t launch_select(cudaStream_t s, int sm_count, const double *x, int64_t
                           void *scratch, double *out) {
     SelectState *st = static_cast<SelectState *>(scratch);
     select_init_kernel<<<1, 256, 0, s>>>(st, ranks);
-    // eight values per thread at least, at most two blocks per SM
-    const int64_t blocks = (n + 8 * kSelectBlock - 1) / (8 * kSelectBlock);
-    const int grid = static_cast<int>(blocks < 2 * sm_count ? (blocks < 1 ? 1 : blocks) : 2 * sm_count);
+    // a value per thread where that is at most four blocks per SM: a pass over few values is a
+    // chain of latencies, and each value a thread takes adds one (100,000 values, eight passes:
+    // 147 us with eight values a thread, the prefixes read one after another and the results
+    // copied from the device; 90 us)
+    const int64_t blocks = (n + kSelectBlock - 1) / kSelectBlock;
+    const int grid = static_cast<int>(blocks < 4 * sm_count ? (blocks < 1 ? 1 : blocks) : 4 * sm_count);
     for (int pass = 0; pass < 8; ++pass)
         select_pass_kernel<<<grid, kSelectBlock, 0, s>>>(x, n, n_ranks, pass, st, out);
     return cudaGetLastError();
