@@ -648,6 +648,78 @@ __device__ __forceinline__ double rel_spot64(const Tab64 &t, const Path64 &s) {
     else return exp2_64(t, s.x);
 }
 
+// ----------------------------------------------------------------------------
+// FP64 steps on the spot itself with the CUDA library's functions: the paths of the
+// exercise-date slabs and of the path dump.  An American price hangs on exercise decisions,
+// and in the reference's mode those come from unscaled normal equations whose smallest pivot
+// is 1e-7 beside sums of 1e5: last bits of the spots reach the fit, one flipped decision
+// spreads to a thousand at earlier dates, and the price moves by 1e-4 of itself (4e-4 for
+// Bates QE, 300,001 x 100, with step64's paths, on one of 84 contracts tried).  These steps
+// keep the spots, and with them those prices, bit for bit.  Heston Milstein in the
+// reference's mode, 300,001 x 100: 1,154 us with step64's paths, 1,283 us with these.
+// ----------------------------------------------------------------------------
+template <int SCHEME>
+__device__ __forceinline__ void step_spot64(const StepConst<double> &p, double &S, double &v, double Z1, double Z2) {
+    if constexpr (SCHEME != kQE) {
+        const double ZS = p.rho * Z1 + p.rho_c * Z2;
+        const double sqv = ::sqrt(v);
+        const double ex = p.r_minus_q_dt - v * p.half_dt + (sqv * p.sqrt_dt) * ZS;
+        const double Sn = S * ::exp(ex);
+        double vn;
+        if constexpr (SCHEME == kEuler) {
+            vn = v * p.one_minus_k_dt + p.k_theta_dt + (p.sigma_sqrt_dt * sqv) * Z1;
+        } else {
+            const double corr = p.quarter_sigma_sq_dt * (Z1 * Z1 - 1.0);
+            vn = p.implicit_den * (v + p.k_theta_dt + (p.sigma_sqrt_dt * sqv) * Z1 + corr);
+        }
+        S = Sn;
+        v = fmax(vn, 0.0);
+    } else {
+        const double m = v * p.exp_mkdt + p.theta_m;
+        const double s2 = v * p.s2f1 + p.s2f2;
+        double vn, logM;  // logM: log of the martingale factor
+        if (m <= p.eps) {
+            vn = 0.0;
+            logM = 0.0;
+        } else {
+            const double m2 = m * m;
+            if (s2 <= p.eps * m2) {
+                vn = m;
+                logM = 0.0;
+            } else if (s2 <= p.psi_c * m2) {
+                const double two_ip = 2.0 * m2 * (1.0 / s2);  // 2 / psi
+                const double b2 = two_ip - 1.0 + ::sqrt(two_ip * (two_ip - 1.0));
+                const double a = m * (1.0 / (1.0 + b2));
+                const double bz = ::sqrt(b2) + Z1;
+                vn = a * bz * bz;
+                const double Aa = fmin(p.A * a, 0.5 - p.eps * a);  // min(A, 1/(2a) - eps) a
+                const double term = 1.0 - 2.0 * Aa;
+                logM = Aa * b2 * (1.0 / term) - 0.5 * ::log(term);
+            } else {
+                const double inv_m = 1.0 / m;
+                const double psi = s2 * inv_m * inv_m;
+                const double pz = (psi - 1.0) / (psi + 1.0);
+                const double beta = (1.0 - pz) * inv_m;
+                const double U = 0.5 * (1.0 + ::erf(Z1 * p.inv_sqrt2));
+                if (U <= pz) {
+                    vn = 0.0;
+                } else {
+                    const double safe_U = fmin(U, 1.0 - p.eps);
+                    vn = ::log((1.0 - pz) / (1.0 - safe_U)) / beta;
+                }
+                const double safe_A = fmin(p.A, beta - p.eps);
+                const double M = pz + (beta * (1.0 - pz)) / (beta - safe_A);
+                logM = ::log(M);
+            }
+        }
+        const double K0 = -logM - p.K1_half_K3 * v;
+        const double isig = p.K3 * v + p.K4 * vn;
+        const double ex = p.r_minus_q_dt + K0 + (p.K1 * v + p.K2 * vn) + ::sqrt(isig) * Z2;
+        S = S * ::exp(ex);
+        v = vn;
+    }
+}
+
 // Bates jump part after the (drift-compensated) Heston step: MSchemes.hpp:493-526.
 // Knuth's Poisson draw: multiply uniforms until the product drops below exp(-lambda dt).
 // `prod` holds the first uniform, already known to be >= exp(-lambda dt) (a jump).

@@ -15,7 +15,7 @@ namespace qk {
 // One path of one task.  Mirrors MarkovianIntegrationKernel::operator()
 // (include/core/schemes/markovian/MSolver.hpp:98-130): start at (S0, v0), step
 // n_steps times, track the running average / max / min after every step.
-// SINK is called after each step with (step index, S, v) (FP64: a function giving S).
+// SINK is called after each step with (step index, S, v) (FP32).
 // ----------------------------------------------------------------------------
 template <class R>
 struct PathState {
@@ -25,8 +25,8 @@ struct PathState {
 };
 
 struct NoSink {
-    template <class S, class R>
-    __device__ __forceinline__ void operator()(int, S, R) const {}
+    template <class R>
+    __device__ __forceinline__ void operator()(int, R, R) const {}
 };
 
 // The FP64 functions' tables of a block (FP32 kernels hold none).
@@ -54,12 +54,10 @@ struct SlabSink {
     int stride;     // steps between stored dates
     int left;       // steps until the next stored date
     // Called once per step, in order: every stride-th step is stored.
-    template <class Spot>
-    __device__ __forceinline__ void operator()(int, Spot spot, R v) {
+    __device__ __forceinline__ void operator()(int, R S, R v) {
         if (--left == 0) {
             left = stride;
-            if constexpr (sizeof(R) == 8) slab_S[pos] = spot();
-            else slab_S[pos] = spot;
+            slab_S[pos] = S;
             if (slab_v) slab_v[pos] = v;
             pos += ld;
         }
@@ -175,9 +173,9 @@ __device__ __noinline__ double2 jump_log2_f64(const TaskDev &t, uint32_t word, u
 // FP64 paths: NP paths of one lane (1; 2: an antithetic pair, NEG, or two independent
 // paths), stepped on the logarithm of the spot (step64).  Sums, maxima and minima are
 // those of S / S0; st holds the spot's on return.
-template <int MODEL, int SCHEME, int TRK, int NP, bool NEG, class Gen, class Sink>
+template <int MODEL, int SCHEME, int TRK, int NP, bool NEG, class Gen>
 __device__ __forceinline__ void simulate_f64(const Tab64 &tab, const StepConst<double> &p, const TaskDev &t,
-                                             const Gen &gen, uint32_t path, PathState<double> (&st)[NP], Sink &&sink) {
+                                             const Gen &gen, uint32_t path, PathState<double> (&st)[NP]) {
     const double S0 = t.S0, v0 = t.v0;
     const int n_steps = t.n_steps;
     const uint32_t kmin = t.jump_kmin64;
@@ -240,7 +238,6 @@ __device__ __forceinline__ void simulate_f64(const Tab64 &tab, const StepConst<d
                     st[i].smax = r > st[i].smax ? r : st[i].smax;
                     st[i].smin = r < st[i].smin ? r : st[i].smin;
                 }
-                sink(n, [&, i] { return S0 * rel_spot64<SCHEME>(tab, s[i]); }, s[i].v);
             }
         };
         for (int n = n0; n < n1; n += 2) {
@@ -273,13 +270,51 @@ __device__ __forceinline__ void simulate_f64(const Tab64 &tab, const StepConst<d
     }
 }
 
+// FP64 path stepped on the spot (step_spot64), stored by the sink.
+template <int MODEL, int SCHEME, class Gen>
+__device__ __forceinline__ void simulate_spot_f64(const StepConst<double> &p, const TaskDev &t, const Gen &gen,
+                                                  uint32_t path, SlabSink<double> &sink) {
+    double S = t.S0, v = t.v0;
+    const int n_steps = t.n_steps;
+    const uint32_t kmin = t.jump_kmin64;
+    const PhiloxPath pp = gen.path(path);
+    const uint4 *row = gen.rows;
+    U4 wp{0u, 0u, 0u, 0u};  // Poisson words of steps 4m .. 4m+3
+    auto step = [&](int n, uint32_t wa, uint32_t wb, bool odd) {
+        double z1, z2;
+        Math<double>::box_muller(wa, wb, z1, z2);
+        step_spot64<SCHEME>(p, S, v, z1, z2);
+        if constexpr (MODEL == kBates) {
+            const uint32_t word = (n & 2) ? (odd ? wp.w : wp.z) : (odd ? wp.y : wp.x);
+            if (word >= kmin) {
+                const double first = Math<double>::u01(word);
+                PhiloxJumpDraws<double> d{t.key0, t.key1, path, t.stream, static_cast<uint32_t>(n), first, 1, 0, U4{0, 0, 0, 0}};
+                if (first >= p.exp_m_lambda_dt) S *= jump_factor<double>(p, first, d);
+            }
+        }
+        sink(n, S, v);
+    };
+    for (int n = 0; n < n_steps; n += 2, ++row) {
+        if ((n & (kRowSteps - 1)) == 0) {
+            gen.fill(n);
+            row = gen.rows;
+        }
+        const U4 w = gen.block(row, pp);
+        if constexpr (MODEL == kBates) {
+            if ((n & 3) == 0) wp = gen.block(gen.rows + 32 + ((n & (kRowSteps - 1)) >> 2), pp);
+        }
+        step(n, w.x, w.y, false);
+        if (n + 1 < n_steps) step(n + 1, w.z, w.w, true);
+    }
+}
+
 // TRK: the path state to keep (kTrack*).
 template <class R, int MODEL, int SCHEME, int TRK = kTrackAll, class Gen, class Sink>
 __device__ __forceinline__ void simulate_path(const Tab64 *tab, const StepConst<R> &p, const TaskDev &t, const Gen &gen,
                                               uint32_t path, PathState<R> &st, Sink &&sink) {
     if constexpr (sizeof(R) == 8) {
         PathState<double> one[1];
-        simulate_f64<MODEL, SCHEME, TRK, 1, false>(*tab, p, t, gen, path, one, sink);
+        simulate_f64<MODEL, SCHEME, TRK, 1, false>(*tab, p, t, gen, path, one);
         st = one[0];
     } else {
         const float S0 = static_cast<float>(t.S0), v0 = static_cast<float>(t.v0);
@@ -601,7 +636,7 @@ __global__ void __launch_bounds__(path_block_max<R>(),
                 with_keys([&](const auto &gen) {
                     if constexpr (sizeof(R) == 8) {
                         PathState<double> two[2];
-                        simulate_f64<MODEL, SCHEME, TRK, 2, NEG>(*tables.get(), p, t, gen, pa, two, NoSink{});
+                        simulate_f64<MODEL, SCHEME, TRK, 2, NEG>(*tables.get(), p, t, gen, pa, two);
                         sa = two[0];
                         sb = two[1];
                     } else {
@@ -825,15 +860,11 @@ __global__ void __launch_bounds__(128) merge_task_chunks_kernel(const TaskDev *_
 // variant follows), S (and v)
 // after every `stride`-th step stored as SoA rows slab[date][path] (coalesced:
 // consecutive threads write consecutive columns).  Specialised per kind, with the
-// Philox round keys in the kernel parameters.  FP64: grid-stride over the paths, so that
-// a block's function tables are filled once.
+// Philox round keys in the kernel parameters.
 template <class R, int MODEL, int SCHEME>
-__global__ void __launch_bounds__(kPathBlock, sizeof(R) == 4 ? kPathMinBlocksFp32 : kPathMinBlocksQe64) slab_paths_kernel(const TaskDev *__restrict__ task, int64_t first_path,
-                                                               int64_t count, int stride, R *__restrict__ slab_S,
-                                                               R *__restrict__ slab_v, int64_t ld,
-                                                               const PhiloxRoundKeys rk) {
-    __shared__ BlockTables<R> tables;
-    tables.fill();
+__global__ void __launch_bounds__(kPathBlock, sizeof(R) == 4 ? kPathMinBlocksFp32 : kPathMinBlocksQe64)
+    slab_paths_kernel(const TaskDev *__restrict__ task, int64_t first_path, int64_t count, int stride,
+                      R *__restrict__ slab_S, R *__restrict__ slab_v, int64_t ld, const PhiloxRoundKeys rk) {
     const TaskDev &t = *task;
     const StepConst<R> p = task_const<R>(t);
     constexpr int kRows = philox_rows<R, MODEL>();
@@ -841,13 +872,16 @@ __global__ void __launch_bounds__(kPathBlock, sizeof(R) == 4 ? kPathMinBlocksFp3
     const WarpPhilox<kRows, ParamKeys> gen{ParamKeys{rk}, s_rows[threadIdx.x >> 5], t.stream};
     // whole warps (the generator's rows are the warp's work): a lane beyond the last path
     // repeats that path and stores its values again
-    const int lane = threadIdx.x & 31;
-    for (int64_t i0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x - lane; i0 < count;
-         i0 += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int64_t i = std::min(i0 + lane, count - 1);
-        SlabSink<R> sink{slab_S, slab_v, ld, i, stride, stride};
+    const int64_t i0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i0 - static_cast<int64_t>(threadIdx.x & 31) >= count) return;
+    const int64_t i = std::min(i0, count - 1);
+    const uint32_t path = static_cast<uint32_t>(first_path + i);
+    SlabSink<R> sink{slab_S, slab_v, ld, i, stride, stride};
+    if constexpr (sizeof(R) == 8) {
+        simulate_spot_f64<MODEL, SCHEME>(p, t, gen, path, sink);
+    } else {
         PathState<R> st;
-        simulate_path<R, MODEL, SCHEME, kTrackNone>(tables.get(), p, t, gen, static_cast<uint32_t>(first_path + i), st, sink);
+        simulate_path<R, MODEL, SCHEME, kTrackNone>(nullptr, p, t, gen, path, st, sink);
     }
 }
 
