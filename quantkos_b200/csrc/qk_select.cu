@@ -83,6 +83,8 @@ __global__ void __launch_bounds__(kSelectBlock) select_pass_kernel(const double 
     __threadfence();
     for (int r = warp; r < n_ranks; r += kSelectBlock / 32) {
         const int g = s_group[r];
+        // one lane reads the rank that one lane replaces below: the shuffle orders the two
+        const unsigned long long want = __shfl_sync(0xffffffffu, lane == 0 ? st->rank[r] : 0ull, 0);
         unsigned c[8], sum = 0;
         for (int j = 0; j < 8; ++j) sum += c[j] = __ldcg(&st->hist[g][8 * lane + j]);
         unsigned before = sum;  // inclusive, then exclusive, sum over the lanes
@@ -91,7 +93,6 @@ __global__ void __launch_bounds__(kSelectBlock) select_pass_kernel(const double 
             if (lane >= off) before += o;
         }
         before -= sum;
-        const unsigned long long want = st->rank[r];
         if (want >= before && want < static_cast<unsigned long long>(before) + sum) {
             unsigned long long left = want - before;
             int j = 0;
