@@ -258,6 +258,7 @@ TaskDev make_task(const qk_contract &b, int ppt, int lane_mode) {
         std::min(std::max(std::ceil(t.cd.exp_m_lambda_dt * 4294967296.0 - 0.5), 0.0), 4294967295.0));
     t.lane_mode = b.antithetic ? kLanePair : lane_mode;
     t.track = path_state(b, b.precision);
+    t.fold_steps = qe_fold_steps(t.cd);
     const int64_t units = lane_units(b.n_paths, t.lane_mode);
     const int64_t tile_units = static_cast<int64_t>(kWarpTilePaths) * ppt;
     t.n_tiles = static_cast<int32_t>((units + tile_units - 1) / tile_units);

@@ -20,6 +20,24 @@ extern thread_local std::string g_last_error;  // message of the last failing ca
 // 442-563) on the fields a contract carries, plus this engine's own limits.
 qk_status validate_contract(const qk_contract &c, const qk_greeks *g);
 
+// The largest a of a QE step's quadratic regime: a = h / (m + G) <= h / m, a mediant of two
+// fixed ratios (see make_step_const).
+template <class R>
+inline double qe_a_max(const StepConst<R> &d) {
+    return std::max(d.h_f1 / d.exp_mkdt, d.theta_m > 0.0 ? d.h_f2 / d.theta_m : 0.0);
+}
+
+// FP64 QE: steps between two folds of the martingale product.  As 1 - sum, the product has
+// the rounding of numbers of the order of 1: 16 steps where it stays above 1/2 that long (any
+// rho <= 0; rho > 0 at steps of a month), fewer otherwise, at least the two of a Philox block.
+inline int qe_fold_steps(const StepConst<double> &d) {
+    if (!(d.h_psi_plain > 0.0)) return 16;  // no step has a factor
+    const double least = 1.0 - std::max(d.two_A * qe_a_max(d), 0.0);  // least factor 1 - 2 A a
+    int n = 16;
+    while (n > 2 && !(least > 0.0 && std::pow(least, n) >= 0.5)) n /= 2;
+    return n;
+}
+
 // Per-step invariants exactly as the reference constructors compute them
 // (MSchemes.hpp:102-123, 197-219, 303-353, 480-487, 535-550), in double, then
 // rounded to R.  eps is the QE guard (1e-12 in FP64 builds, 1e-6 in FP32 builds).
@@ -87,8 +105,9 @@ inline StepConst<R> make_step_const(const qk_contract &c, double dt, double eps)
     d.l_half_dt = d.half_dt * kLog2e;
     d.l_sqrt_dt = d.sqrt_dt * kLog2e;
     d.l_K2 = d.K2 * kLog2e;
-    d.l_A = d.A * kLog2e;
-    d.l_c1 = -0.5 * d.K3 * kLog2e;  // K1 - (K1 + K3 / 2)
+    // differences of the rounded constants themselves (exact): what the reference's sums come to
+    d.l_c1 = (d.K1 - d.K1_half_K3) * kLog2e;
+    d.l_c2 = (d.K2 - d.A) * kLog2e;
     d.l_sqrt_K3 = std::sqrt(d.K3) * kLog2e;
     d.h_f1 = 0.5 * d.s2f1;
     d.h_f2 = 0.5 * d.s2f2;
@@ -98,9 +117,11 @@ inline StepConst<R> make_step_const(const qk_contract &c, double dt, double eps)
     // two fixed ratios: where 2 (A + eps) times the larger stays below 1 (it does at any usual
     // parameters) min(A a, 1/2 - eps a) is A a on every step, and the steps' plain form of
     // the quadratic regime needs no clamp.  Elsewhere no step takes the plain form.
-    const double a_max = std::max(d.h_f1 / d.exp_mkdt, d.theta_m > 0.0 ? d.h_f2 / d.theta_m : 0.0);
+    const double a_max = qe_a_max(d);
     const bool plain = 2.0 * (d.A + eps) * a_max <= 1.0 - 1.0 / 1024.0 && std::fabs(d.two_A) * a_max < 1e12;
-    d.h_psi_plain = plain ? 0.5 * d.psi_c : -1.0;
+    // (FP64 keeps 1 - 2 A a of two steps above 1/4 as well, see qe_fold_steps)
+    const bool two_steps = sizeof(R) == 4 || d.two_A * a_max <= 0.5;
+    d.h_psi_plain = plain && two_steps ? 0.5 * d.psi_c : -1.0;
     // The paired FP32 step knows 2 / psi to 2^-21 (a reciprocal good to one unit in the last
     // place, two roundings): within these bounds, 2^-18 inside the regime's, the one-path
     // step's comparisons of s^2 give the quadratic regime too, and a step between the two

@@ -57,7 +57,7 @@ struct StepConst {
     R exp_m_lambda_dt, mu_j, sigma_j;              // Bates
     // The steps on the base-2 logarithm of the spot: increments scaled by log2(e)
     R l_drift, l_half_dt, l_sqrt_dt;               // (r - q) dt, dt / 2, sqrt(dt)
-    R l_K2, l_A, l_c1, l_sqrt_K3;                  // QE: K2, A, -K3 / 2 (the coefficient of v), sqrt(K3) (K3 = K4)
+    R l_K2, l_c1, l_c2, l_sqrt_K3;                 // QE: K2, K1 - K1_half_K3, K2 - A, sqrt(K3) (K3 = K4)
     R h_f1, h_f2, h_eps, two_A;                    // QE: s^2 / 2 = v h_f1 + h_f2, eps / 2, 2 A
     R h_psi_plain;                                 // psi_c / 2, or -1 where A a could reach its clamp (make_step_const)
     R ip_lo, ip_hi;                                // FP32 QE: bounds of 2 / psi in the plain quadratic regime
@@ -106,6 +106,7 @@ struct TaskDev {
     int32_t n_chunks;      // merge chunks of the task: ceil(n_tiles / kMergeChunkTiles)
     int32_t lane_mode;     // kLaneOne / kLanePair / kLaneTwo: what a lane simulates; tiles count lane units
     int32_t track;         // path state that some leg reads (kTrack*)
+    int32_t fold_steps;    // FP64 QE: steps between two folds of the martingale product (qe_fold_steps)
     PayoffSpec pay[QK_MAX_PAYOFFS];
 };
 

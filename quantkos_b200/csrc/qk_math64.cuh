@@ -111,7 +111,7 @@ __device__ __forceinline__ double rsqrt_approx64(double x) {
 }
 __device__ __forceinline__ double rsqrt64(double x) {
     const double y = rsqrt_approx64(x);
-    const double e = fma(-x * y, y, 1.0);
+    const double e = fma(-x, y * y, 1.0);  // y * y is exact: the approximation's low word is zero
     return fma(y * e, fma(e, 0.375, 0.5), y);
 }
 __device__ __forceinline__ double sqrt_from64(double x, double y) {

@@ -186,7 +186,7 @@ __device__ __forceinline__ void simulate_f64(const Tab64 &tab, const StepConst<d
     Path64 s[NP];
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
-        s[i] = Path64{0.0, 1.0, v0};
+        s[i] = Path64{0.0, 1.0, 0.0, v0};
         st[i].ssum = 0.0;
         st[i].smax = st[i].smin = kLogRange ? 0.0 : 1.0;
     }
@@ -194,14 +194,15 @@ __device__ __forceinline__ void simulate_f64(const Tab64 &tab, const StepConst<d
     PhiloxPath pp[ND];
 #pragma unroll
     for (int i = 0; i < ND; ++i) pp[i] = gen.path(path + i);
-    for (int n0 = 0; n0 < n_steps; n0 += kSumChunk) {
-        const int n1 = min(n0 + kSumChunk, n_steps);
+    const int chunk = SCHEME == kQE ? t.fold_steps : kSumChunk;
+    U4 w[ND], wp[ND];
+    for (int n0 = 0; n0 < n_steps; n0 += chunk) {
+        const int n1 = min(n0 + chunk, n_steps);
         double blk[NP];
 #pragma unroll
         for (int i = 0; i < NP; ++i) blk[i] = 0.0;
         if ((n0 & (kRowSteps - 1)) == 0) gen.fill(n0);
         const uint4 *row = gen.rows + ((n0 & (kRowSteps - 1)) >> 1);
-        U4 w[ND], wp[ND];
         auto step = [&](int n, bool odd) {
 #pragma unroll
             for (int i = 0; i < NP; ++i) {
