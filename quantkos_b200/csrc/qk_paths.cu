@@ -256,12 +256,14 @@ __device__ __forceinline__ void simulate_f64(const Tab64 &tab, const StepConst<d
 #pragma unroll
         for (int i = 0; i < NP; ++i) {
             if constexpr (TRK & kTrackSum) st[i].ssum += blk[i];
-            fold64<SCHEME>(tab, s[i]);
+            if (n1 < n_steps) fold64<SCHEME>(tab, s[i]);
         }
     }
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
-        st[i].S = S0 * exp2_64(tab, s[i].x);
+        // formed as the extremes are: a path that ends at its maximum or minimum has them equal
+        // (a lookback then pays exactly nothing)
+        st[i].S = S0 * rel_spot64<SCHEME>(tab, s[i]);
         st[i].v = s[i].v;
         if constexpr (TRK & kTrackSum) st[i].ssum *= S0;
         if constexpr (TRK & kTrackRange) {

@@ -72,3 +72,19 @@ def test_qe_prices_against_long_double(qk, handle, leg):
         err.append(float(got / np.longdouble(r["price"]) - 1))
     assert len(err) == 10
     assert math.sqrt(np.mean(np.square(err))) < 1e-15, err
+
+
+@pytest.mark.parametrize("antithetic", [False, True])
+@pytest.mark.parametrize("model,scheme", [(0, 0), (0, 1), (0, 2), (1, 2)])
+@pytest.mark.parametrize("n_steps", [1, 3, 16, 17])
+def test_lookback_of_a_path_ending_at_its_extreme_pays_nothing(qk, handle, oracle, n_steps, model, scheme, antithetic):
+    """Floating lookbacks on a spot of 20,000 without normalisation: a unit in the last place of
+    the spot passes the in-the-money threshold of 1e-12, so the terminal spot and the running
+    extreme it reaches have to be the same number.  The oracle takes both from one value."""
+    k = qk.make_contract(S0=20_000.0, v0=0.04, model=model, scheme=scheme, lambda_j=0.2 if model else 0.0, mu_j=-0.05,
+                         sigma_j=0.1, n_steps=n_steps, T=0.1, n_paths=4000, seed=21, precision=qk.FP64, normalize=False,
+                         antithetic=antithetic, payoffs=[qk.payoff(qk.LOOKBACK_FLOATING, qk.CALL, 20_000.0),
+                                                         qk.payoff(qk.LOOKBACK_FLOATING, qk.PUT, 20_000.0)])
+    for got, want in zip(qk.price_batch([k], None, handle)[0]["legs"], oracle.price(k)["legs"]):
+        assert got["prob_itm"] == pytest.approx(want["prob_itm"], abs=1e-9)
+        assert got["price"] == pytest.approx(want["price"], rel=1e-9)
