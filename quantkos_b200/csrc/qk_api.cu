@@ -876,8 +876,9 @@ qk_status price_contracts(qk_handle *h, const qk_contract *c, int32_t n, const q
     h->lsm_launches = 0;
     h->lsm_jobs = 0;
     // antithetic tasks keep no payoffs per path; a plan in another precision than the
-    // contract's (the plain method on an FP32 contract) simulates other payoffs
-    const bool with_payoffs = dist && h->plan.tasks.size() == 1 && h->plan.american.empty() &&
+    // contract's (the plain method on an FP32 contract) simulates other payoffs; one leg's
+    // payoffs give no records of the others
+    const bool with_payoffs = dist && n == 1 && h->plan.tasks.size() == 1 && h->plan.tasks[0].n_payoffs == 1 &&
                               h->plan.tasks[0].lane_mode != kLanePair && h->plan.tasks[0].precision == c->precision;
     double *payoffs = nullptr;
     const size_t head = select_scratch_bytes(), order_at = QK_MAX_PAYOFFS * sizeof(Moments);

@@ -12,6 +12,7 @@
 #include <string>
 #include <vector>
 
+#include "qk_engine.h"
 #include "qk_kernels.h"
 
 static int g_failed = 0;
@@ -79,9 +80,84 @@ static void section_select() {
     }
 }
 
+// ---------------------------------------------------------------- contracts
+static qk_payoff leg(int type, int right, double K, double B = 0.0) {
+    qk_payoff p{};
+    p.type = type;
+    p.right = right;
+    p.strike = K;
+    p.barrier = B;
+    return p;
+}
+
+static qk_contract contract(int precision, int model, int scheme, int64_t n_paths, int n_steps, std::vector<qk_payoff> legs) {
+    qk_contract c{};
+    c.S0 = 100.0;
+    c.v0 = 0.04;
+    c.r = 0.03;
+    c.model = model;
+    c.scheme = scheme;
+    c.kappa = 2.0;
+    c.theta = 0.04;
+    c.sigma = 0.3;
+    c.rho = -0.7;
+    c.lambda_j = model == QK_BATES ? 0.4 : 0.0;
+    c.mu_j = -0.05;
+    c.sigma_j = 0.1;
+    c.psi_c = 1.5;
+    c.T = n_steps / 252.0;
+    c.n_steps = n_steps;
+    c.n_paths = n_paths;
+    c.seed = 0x1234567890ABull;
+    c.precision = precision;
+    c.normalize = 1;
+    c.n_payoffs = static_cast<int>(legs.size());
+    for (size_t i = 0; i < legs.size(); ++i) c.payoffs[i] = legs[i];
+    return c;
+}
+
+static bool same_legs(const qk_result &a, const qk_result &b, int n) {
+    bool same = a.n_payoffs == b.n_payoffs;
+    for (int k = 0; k < n; ++k)
+        same &= a.p[k].price == b.p[k].price && a.p[k].std_error == b.p[k].std_error && a.p[k].prob_itm == b.p[k].prob_itm;
+    return same;
+}
+
+// ---------------------------------------------------------------- price beside a distribution
+// One leg: priced from the stored payoffs, the same bits as without; several legs: not
+// answered from them, and the prices are those without.
+static void section_distribution() {
+    qk_handle *h = nullptr;
+    if (qk_create(0, &h) != QK_OK) {
+        check(false, std::string("qk_create: ") + qk_last_error());
+        return;
+    }
+    for (int precision : {QK_FP32, QK_FP64})
+        for (int64_t n : {1, 33, 65, 4097, 100003})
+            for (int legs = 1; legs <= 2; ++legs) {
+                std::vector<qk_payoff> l{leg(QK_ASIAN, QK_CALL, 100.0)};
+                if (legs == 2) l.push_back(leg(QK_EUROPEAN, QK_PUT, 105.0));
+                const qk_contract c = contract(precision, QK_BATES, QK_ANDERSEN_QE, n, 20, l);
+                qk_result alone{}, beside{};
+                double order[3];
+                qk::PayoffRanks dist;
+                dist.ranks.r[1] = static_cast<unsigned long long>(n) / 2;
+                dist.ranks.r[2] = static_cast<unsigned long long>(n) - 1;
+                dist.n_ranks = 3;
+                dist.out = order;
+                bool ok = qk::price_contracts(h, &c, 1, nullptr, &alone, false) == QK_OK &&
+                          qk::price_contracts(h, &c, 1, nullptr, &beside, false, &dist) == QK_OK;
+                ok = ok && same_legs(alone, beside, legs) && dist.done == (legs == 1);
+                check(ok, "distribution precision " + std::to_string(precision) + " paths " + std::to_string(n) + " legs " +
+                              std::to_string(legs));
+            }
+    qk_destroy(h);
+}
+
 int main(int argc, char **argv) {
     const std::string section = argc > 1 ? argv[1] : "";
     if (section == "select") section_select();
+    else if (section == "distribution") section_distribution();
     else check(false, "unknown section " + section);
     return g_failed != 0;
 }

@@ -37,3 +37,9 @@ def test_select_equals_sort(variants):
     """Ranks next to one another, ties, neighbouring bit patterns, subnormals and infinities, at
     sizes around a block and with several values per thread: bit for bit."""
     variants("select", 36)
+
+
+def test_price_beside_a_distribution(variants):
+    """A one-leg contract's price from its stored payoffs has the bits of the price alone; a
+    contract of several legs is not priced from one leg's payoffs."""
+    variants("distribution", 20)
