@@ -17,9 +17,9 @@
 //     approximations by one third-order step (Householder), without the library's
 //     special-case branches: callers guard the arguments.
 //
-// Largest relative errors measured against the library (67 million arguments): -2 ln u
-// 4.4e-16, 2^x 3.3e-16, reciprocal 1.1e-16, the square roots 2.2e-16, a normal 6.1e-16 of
-// its radius.  The tables (14 KB) live in shared memory, filled at the start of a kernel by
+// Largest relative errors against long double (a million arguments each): -2 ln u 3.7e-16, 2^x
+// 2.5e-16, reciprocal and reciprocal square root 1.2e-16, square root 1.7e-16, a normal
+// 4.6e-16 of its radius.  The tables (14 KB) live in shared memory, filled at the start of a kernel by
 // the block's threads with the CUDA functions: about 0.5 us, no table in global memory to
 // load.  Plain FP64 Heston Euler European, 1,048,576 x 252: 286 warp instructions per 32
 // path-steps and 2.77 ms with the library's functions on the spot, 106 and 1.21 ms with

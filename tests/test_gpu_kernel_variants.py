@@ -43,3 +43,21 @@ def test_price_beside_a_distribution(variants):
     """A one-leg contract's price from its stored payoffs has the bits of the price alone; a
     contract of several legs is not priced from one leg's payoffs."""
     variants("distribution", 20)
+
+
+def test_launch_shapes_give_the_same_records(variants):
+    """Tile records of one task, bit for bit: one warp per tile, persistent blocks of 128, 256 and
+    512 threads in one block and in 37, and with the term table."""
+    variants("shapes", 65)
+
+
+def test_slabs_with_and_without_a_term_table(variants):
+    """400,003 paths of both models, bit for bit: two paths per thread with the table and without,
+    one path per thread."""
+    variants("slabs", 13)
+
+
+def test_fp64_functions_against_long_double(variants):
+    """The path kernels' own logarithm, exponential, reciprocal, roots and Box-Muller: a million
+    arguments each, the edges of the words and of the tables, next to 1, out of range."""
+    variants("functions", 11)
