@@ -44,15 +44,16 @@ N_PATHS = 16_777_216
 N_STEPS = 252
 WORKLOAD = "bates_qe_5payoff_16777216x252_fp32"
 METRIC = "path-steps/s"
-# Algorithmic SFU (MUFU) work per path-step of the fused Bates-QE kernel, counted
-# from the step formulas as implemented, quadratic QE branch (taken by nearly every
-# step at these parameters): Box-Muller lg2, sqrt, sin, cos; QE rcp(s2),
-# sqrt(x(x-1)), rcp(1+b2), sqrt(b2), rcp(term), lg2(term); spot update
-# sqrt(K3 v + K4 v'), ex2.  The SFU pipe (16 lanes/clk/SM) then bounds the kernel
-# at (measured SFU op rate) / 12 path-steps/s; the FP32/integer work (Philox, the
-# QE algebra) fits under that bound on the 128-lane issue.  A launch of one contract
-# reads two of the twelve (rcp(term), lg2(term)) from a table of the SFU's own results.
-SFU_PER_STEP = 12.0
+# SFU (MUFU) work per path-step of the fused QE kernels, counted from the step formulas as
+# implemented, quadratic QE branch (taken by nearly every step at these parameters):
+# Box-Muller lg2, sqrt, sin, cos; QE rcp(s2), sqrt(x(x-1)), rcp(1+b2), sqrt(b2), rcp(term),
+# lg2(term); spot update sqrt(K3 v + K4 v'), ex2: twelve.  A large launch of one contract
+# with two paths per lane reads rcp(term) and lg2(term) from a table of the SFU's own
+# results: ten are left for the SFU pipe (16 lanes/clk/SM), which bounds such a launch at
+# (measured SFU op rate) / 10 path-steps/s; the FP32/integer work (Philox, the QE algebra)
+# fits under that bound on the 128-lane issue.
+SFU_PER_STEP = 10.0
+TABLE_SFU_OPS = 2  # the SFU operations that the table replaces
 # Algorithmic scalar lane operations per path-step of the FP32 kinds (from the formulas
 # as implemented; one-path-per-lane count), for the issue-slot bound (every operation,
 # SFU ones included, takes an issue slot; an SM issues 4 warp instructions = 128 lane
@@ -472,7 +473,7 @@ def run_other_workload(args) -> None:
         # every FP32 kernel kind on one large contract (16.8M x 252, one European leg, the
         # headline market; Bates jumps as in the headline) at the handle's default shape:
         # path-kernel time against each kind's SFU bound (Euler and Milstein: Box-Muller
-        # lg2, sqrt, sin, cos + sqrt(v), ex2 = 6 ops per path-step; QE: 12)
+        # lg2, sqrt, sin, cos + sqrt(v), ex2 = 6 ops per path-step; QE: 10 with the table)
         sfu_ops = h.measure_sfu()
         issue_ops = 8.0 * sfu_ops  # lane operations per second the SMs can issue (128 vs 16 per cycle)
         kinds, total = [], 0.0
@@ -480,6 +481,8 @@ def run_other_workload(args) -> None:
             for model in (qk.HESTON, qk.BATES):
                 for scheme, sname in ((qk.EULER, "euler"), (qk.IMPLICIT_MILSTEIN, "milstein"), (qk.ANDERSEN_QE, "qe")):
                     n_sfu, n_issue = algorithmic_ops(sname, model == qk.BATES)
+                    if scheme == qk.ANDERSEN_QE:
+                        n_sfu -= TABLE_SFU_OPS
                     c = qk.make_contract(S0=100.0, v0=0.04, r=0.03, q=0.0, model=model, scheme=scheme, kappa=2.0,
                                          theta=0.04, sigma=0.3, rho=-0.7,
                                          lambda_j=0.1 if model == qk.BATES else 0.0, mu_j=-0.05, sigma_j=0.10,
@@ -576,7 +579,7 @@ def run_other_workload(args) -> None:
                     gpu_launches=args.steps * t["launches"])
         line["roofline"]["frac"] = line["roofline"]["achieved"] / line["roofline"]["peak"]
         # the forward kernel (Heston QE paths, FP32, writing the 50 exercise-date slabs):
-        # SFU-bound like the path kernels, 12 SFU operations per path-step
+        # SFU-bound like the path kernels, 10 SFU operations per path-step with the table
         sfu_ops = h.measure_sfu()
         fwd_ms = line["roofline"]["forward_ms"]
         line["forward"] = {"kernel": "slab_paths_two_kernel<float, Heston, QE>", "ms": fwd_ms,
@@ -850,7 +853,7 @@ def main() -> None:
                          "unit": "Gpath-steps/s", "frac": achieved_ps / peak_ps, "traffic": traffic,
                          "kernel": "price_tiles_kernel<float>", "kernel_ms": kern_ms,
                          "peak_source": f"measured SFU rate {sfu_ops / 1e12:.3f} Tops/s (qk_measure_sfu); "
-                                        f"{SFU_PER_STEP:.0f} SFU ops per path-step (algorithmic)"},
+                                        f"{SFU_PER_STEP:.0f} SFU ops per path-step (two of the step's twelve come from a table)"},
             "cpu_baseline": cpu,
             "heston_qe_european": hqe,
             "antithetic": anti,
