@@ -659,14 +659,17 @@ __device__ __forceinline__ double rel_spot64(const Tab64 &t, const Path64 &s) {
 }
 
 // ----------------------------------------------------------------------------
-// FP64 steps on the spot itself with the CUDA library's functions: the paths of the
-// exercise-date slabs and of the path dump.  An American price hangs on exercise decisions,
-// and in the reference's mode those come from unscaled normal equations whose smallest pivot
-// is 1e-7 beside sums of 1e5: last bits of the spots reach the fit, one flipped decision
-// spreads to a thousand at earlier dates, and the price moves by 1e-4 of itself (4e-4 for
-// Bates QE, 300,001 x 100, with step64's paths, on one of 84 contracts tried).  These steps
-// keep the spots, and with them those prices, bit for bit.  Heston Milstein in the
-// reference's mode, 300,001 x 100: 1,154 us with step64's paths, 1,283 us with these.
+// FP64 steps on the spot itself with the CUDA library's functions: the paths of American
+// contracts in the reference's mode (Laguerre basis) and of the path dump.  An American
+// price hangs on exercise decisions, and in that mode those come from unscaled normal
+// equations whose smallest pivot is 1e-7 beside sums of 1e5: last bits of the spots reach
+// the fit, one flipped decision spreads to a thousand at earlier dates, and the price moves
+// by 1e-4 of itself (with step64's paths on 3 of 164 contracts tried, up to 4e-4).  These
+// steps keep the spots, and with them those prices, bit for bit.  The six-term basis is
+// centred, scaled and solved with a condition check: 400 of its contracts priced with
+// step64's paths differ by at most 3e-13, and they keep those paths.  300,001 x 100 on every
+// date, Laguerre: Heston Milstein 1,134 us with step64's paths, 1,261 us with these; six
+// terms, 25 dates: Heston QE 509 us, 840 us.
 // ----------------------------------------------------------------------------
 template <int SCHEME>
 __device__ __forceinline__ void step_spot64(const StepConst<double> &p, double &S, double &v, double Z1, double Z2) {
@@ -769,7 +772,9 @@ __device__ __forceinline__ void bates_jump(const StepConst<R> &p, R &S, Draws &d
     if (first >= p.exp_m_lambda_dt) S *= jump_factor<R>(p, first, d);
 }
 
-// One step on the spot itself, with the pricing kernels' step code (the fed-draw trace).
+// One step on the spot itself for the fed-draw trace: the pricing kernels' scheme steps, but
+// with the martingale product folded and the spot formed after every step, and in FP64 the
+// jumps of jump_factor on the fed draws (the pricing kernels': jump_log2_f64).
 template <class R, int MODEL, int SCHEME, class Draws>
 __device__ __forceinline__ void evolve_step(const Tab64 *tab, const StepConst<R> &p, R &S, R &v, Draws &d) {
     R Z1, Z2;

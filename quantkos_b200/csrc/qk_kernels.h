@@ -51,9 +51,11 @@ constexpr int kMergeChunkTiles = 512;
 cudaError_t launch_merge(int n_tasks, int64_t n_chunks, cudaStream_t s, const TaskDev *tasks, const Moments *partials,
                          Moments *chunks, TaskMoments *out, unsigned long long *cursors, int64_t *launches);
 // has_table: the task has a term table (TaskDev::term_lo; two paths per thread only).
+// spot_steps: FP64 paths step the spot with the CUDA library's functions (step_spot64), else
+// its logarithm (step64).
 cudaError_t launch_slab_paths(int precision, int model, int scheme, uint64_t seed, cudaStream_t s, const TaskDev *task,
                               int64_t first_path, int64_t count, int stride, void *slab_S, void *slab_v, int64_t ld,
-                              int sm_count, int paths_per_thread = 1, bool has_table = false);
+                              int sm_count, int paths_per_thread = 1, bool has_table = false, bool spot_steps = true);
 cudaError_t launch_step_trace(int precision, cudaStream_t s, const TaskDev *task, const double *z, const double *u,
                               int umax, int n, double *S_out, double *v_out, int *status);
 // Leg-0 payoffs of paths first .. first + count - 1 of the task (undiscounted, normalised).

@@ -1247,7 +1247,8 @@ qk_status run_lsm_contracts(qk_handle *h, Plan &plan, bool plain, std::vector<Mo
         QK_CUDA_LSM(launch_slab_paths(prec, b.model, b.scheme, b.seed, s,
                                       static_cast<const TaskDev *>(h->lsm_task.ptr) + k, 0, b.n_paths, stride,
                                       L.slab_S.ptr, use_v ? L.slab_v.ptr : nullptr, ld, h->sm_count,
-                                      prec == QK_FP32 ? 2 : 1, tasks[k].term_lo != 0));
+                                      prec == QK_FP32 ? 2 : 1, tasks[k].term_lo != 0,
+                                      b.lsm_basis == QK_LSM_LAGUERRE3));
         h->lsm_launches++;
         QK_CUDA_LSM(cudaEventRecord(h->lsm_events[3 * k + 1], s));
         LsmArgs a;

@@ -9,7 +9,10 @@
 //   * logarithm and power of two by a table of 256 points and a short Taylor polynomial
 //     (Tang, ACM TOMS 16, 1990 and 15, 1989), the reduced argument formed exactly by an
 //     FMA; the table point next to 1 is 1 itself, so -2 ln u keeps its relative accuracy
-//     as u approaches 1;
+//     as u approaches 1.  The steps of the argument reduction on the bits (subtracting an
+//     offset's high word to get exponent and table index at once, pairs of 1 / c and log c,
+//     a shift by 1.5 * 2^52 / N whose low word is the index) are those of Arm's Optimized
+//     Routines (log and exp2); polynomials and tables are formed here;
 //   * sine and cosine of 2 pi (u - 1/2) from the integer word behind u: its top 9 bits
 //     pick a table angle, the other 23 are the (exact) remainder, and the addition
 //     theorem joins them;
@@ -19,12 +22,12 @@
 //
 // Largest relative errors against long double (a million arguments each): -2 ln u 3.7e-16, 2^x
 // 2.5e-16, reciprocal and reciprocal square root 1.2e-16, square root 1.7e-16, a normal
-// 4.6e-16 of its radius.  The tables (14 KB) live in shared memory, filled at the start of a kernel by
-// the block's threads with the CUDA functions: about 0.5 us, no table in global memory to
-// load.  Plain FP64 Heston Euler European, 1,048,576 x 252: 286 warp instructions per 32
-// path-steps and 2.77 ms with the library's functions on the spot, 106 and 1.21 ms with
-// these on its logarithm (FP64 pipe 53% busy in both, 52% now at less than half the work:
-// FP64 and the generator's wide multiplies share issue and register ports).
+// 4.6e-16 of its radius.  The tables (14 KB) live in shared memory, filled at the start of a
+// kernel by the block's threads with the CUDA functions: about 0.5 us, no table in global
+// memory to load.  Plain FP64 Heston Euler European, 1,048,576 x 252: 286 warp instructions
+// per 32 path-steps and 2.77 ms with the library's functions on the spot, 106 and 1.21 ms
+// with these on its logarithm (FP64 pipe 53% busy in both, 52% now at less than half the
+// work: FP64 and the generator's wide multiplies share issue and register ports).
 #pragma once
 
 #include <cstdint>

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "qk_device.cuh"
 #include "qk_kernels.h"
@@ -15,7 +16,7 @@ namespace qk {
 // One path of one task.  Mirrors MarkovianIntegrationKernel::operator()
 // (include/core/schemes/markovian/MSolver.hpp:98-130): start at (S0, v0), step
 // n_steps times, track the running average / max / min after every step.
-// SINK is called after each step with (step index, S, v) (FP32).
+// SINK is called after each step with (step index, S, v); simulate_f64 gives a function for S.
 // ----------------------------------------------------------------------------
 template <class R>
 struct PathState {
@@ -25,8 +26,8 @@ struct PathState {
 };
 
 struct NoSink {
-    template <class R>
-    __device__ __forceinline__ void operator()(int, R, R) const {}
+    template <class S, class R>
+    __device__ __forceinline__ void operator()(int, S, R) const {}
 };
 
 // The FP64 functions' tables of a block (FP32 kernels hold none).
@@ -54,10 +55,12 @@ struct SlabSink {
     int stride;     // steps between stored dates
     int left;       // steps until the next stored date
     // Called once per step, in order: every stride-th step is stored.
-    __device__ __forceinline__ void operator()(int, R S, R v) {
+    template <class Spot>
+    __device__ __forceinline__ void operator()(int, Spot spot, R v) {
         if (--left == 0) {
             left = stride;
-            slab_S[pos] = S;
+            if constexpr (std::is_same_v<Spot, R>) slab_S[pos] = spot;
+            else slab_S[pos] = spot();
             if (slab_v) slab_v[pos] = v;
             pos += ld;
         }
@@ -173,9 +176,9 @@ __device__ __noinline__ double2 jump_log2_f64(const TaskDev &t, uint32_t word, u
 // FP64 paths: NP paths of one lane (1; 2: an antithetic pair, NEG, or two independent
 // paths), stepped on the logarithm of the spot (step64).  Sums, maxima and minima are
 // those of S / S0; st holds the spot's on return.
-template <int MODEL, int SCHEME, int TRK, int NP, bool NEG, class Gen>
+template <int MODEL, int SCHEME, int TRK, int NP, bool NEG, class Gen, class Sink>
 __device__ __forceinline__ void simulate_f64(const Tab64 &tab, const StepConst<double> &p, const TaskDev &t,
-                                             const Gen &gen, uint32_t path, PathState<double> (&st)[NP]) {
+                                             const Gen &gen, uint32_t path, PathState<double> (&st)[NP], Sink &&sink) {
     const double S0 = t.S0, v0 = t.v0;
     const int n_steps = t.n_steps;
     const uint32_t kmin = t.jump_kmin64;
@@ -239,6 +242,7 @@ __device__ __forceinline__ void simulate_f64(const Tab64 &tab, const StepConst<d
                     st[i].smax = r > st[i].smax ? r : st[i].smax;
                     st[i].smin = r < st[i].smin ? r : st[i].smin;
                 }
+                sink(n, [&, i] { return S0 * rel_spot64<SCHEME>(tab, s[i]); }, s[i].v);
             }
         };
         for (int n = n0; n < n1; n += 2) {
@@ -317,7 +321,7 @@ __device__ __forceinline__ void simulate_path(const Tab64 *tab, const StepConst<
                                               uint32_t path, PathState<R> &st, Sink &&sink) {
     if constexpr (sizeof(R) == 8) {
         PathState<double> one[1];
-        simulate_f64<MODEL, SCHEME, TRK, 1, false>(*tab, p, t, gen, path, one);
+        simulate_f64<MODEL, SCHEME, TRK, 1, false>(*tab, p, t, gen, path, one, sink);
         st = one[0];
     } else {
         const float S0 = static_cast<float>(t.S0), v0 = static_cast<float>(t.v0);
@@ -572,7 +576,7 @@ __global__ void __launch_bounds__(path_block_max<R>(),
                        Moments *__restrict__ partials, const PhiloxRoundKeys rk) {
     // Every warp is an independent worker: it pops a tile (kWarpTilePaths * ppt paths of one
     // task), keeps the tile's running moments per leg in its own shared-memory slots and
-    // writes one record per leg.  No block-wide barrier anywhere.
+    // writes one record per leg.  No block-wide barrier once the tables are filled.
     __shared__ Moments s_acc[path_block_max<R>() / 32][QK_MAX_PAYOFFS];
     // the Asian running sums of a lane's two independent paths (simulate_two); one slot per
     // thread (antithetic pairs keep theirs in registers, which measures faster there)
@@ -639,7 +643,7 @@ __global__ void __launch_bounds__(path_block_max<R>(),
                 with_keys([&](const auto &gen) {
                     if constexpr (sizeof(R) == 8) {
                         PathState<double> two[2];
-                        simulate_f64<MODEL, SCHEME, TRK, 2, NEG>(*tables.get(), p, t, gen, pa, two);
+                        simulate_f64<MODEL, SCHEME, TRK, 2, NEG>(*tables.get(), p, t, gen, pa, two, NoSink{});
                         sa = two[0];
                         sb = two[1];
                     } else {
@@ -863,8 +867,9 @@ __global__ void __launch_bounds__(128) merge_task_chunks_kernel(const TaskDev *_
 // variant follows), S (and v)
 // after every `stride`-th step stored as SoA rows slab[date][path] (coalesced:
 // consecutive threads write consecutive columns).  Specialised per kind, with the
-// Philox round keys in the kernel parameters.
-template <class R, int MODEL, int SCHEME>
+// Philox round keys in the kernel parameters.  SPOT (FP64): paths stepped on the spot
+// (step_spot64), which the reference's regression and the dump need; else step64's.
+template <class R, int MODEL, int SCHEME, bool SPOT>
 __global__ void __launch_bounds__(kPathBlock, sizeof(R) == 4 ? kPathMinBlocksFp32 : kPathMinBlocksQe64)
     slab_paths_kernel(const TaskDev *__restrict__ task, int64_t first_path, int64_t count, int stride,
                       R *__restrict__ slab_S, R *__restrict__ slab_v, int64_t ld, const PhiloxRoundKeys rk) {
@@ -876,15 +881,17 @@ __global__ void __launch_bounds__(kPathBlock, sizeof(R) == 4 ? kPathMinBlocksFp3
     // whole warps (the generator's rows are the warp's work): a lane beyond the last path
     // repeats that path and stores its values again
     const int64_t i0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i0 - static_cast<int64_t>(threadIdx.x & 31) >= count) return;
+    const bool warp_has_paths = i0 - static_cast<int64_t>(threadIdx.x & 31) < count;
     const int64_t i = std::min(i0, count - 1);
     const uint32_t path = static_cast<uint32_t>(first_path + i);
     SlabSink<R> sink{slab_S, slab_v, ld, i, stride, stride};
-    if constexpr (sizeof(R) == 8) {
-        simulate_spot_f64<MODEL, SCHEME>(p, t, gen, path, sink);
+    if constexpr (SPOT) {
+        if (warp_has_paths) simulate_spot_f64<MODEL, SCHEME>(p, t, gen, path, sink);
     } else {
+        __shared__ BlockTables<R> tables;
+        tables.fill();
         PathState<R> st;
-        simulate_path<R, MODEL, SCHEME, kTrackNone>(nullptr, p, t, gen, path, st, sink);
+        if (warp_has_paths) simulate_path<R, MODEL, SCHEME, kTrackNone>(tables.get(), p, t, gen, path, st, sink);
     }
 }
 
@@ -930,15 +937,15 @@ SlabKernel<float> slab_two_kernel_for(int model, int scheme, bool table) {
     }
 }
 
-template <class R>
+template <class R, bool SPOT>
 SlabKernel<R> slab_kernel_for(int model, int scheme) {
     switch (model * 3 + scheme) {
-        case 0: return slab_paths_kernel<R, kHeston, kEuler>;
-        case 1: return slab_paths_kernel<R, kHeston, kMilstein>;
-        case 2: return slab_paths_kernel<R, kHeston, kQE>;
-        case 3: return slab_paths_kernel<R, kBates, kEuler>;
-        case 4: return slab_paths_kernel<R, kBates, kMilstein>;
-        default: return slab_paths_kernel<R, kBates, kQE>;
+        case 0: return slab_paths_kernel<R, kHeston, kEuler, SPOT>;
+        case 1: return slab_paths_kernel<R, kHeston, kMilstein, SPOT>;
+        case 2: return slab_paths_kernel<R, kHeston, kQE, SPOT>;
+        case 3: return slab_paths_kernel<R, kBates, kEuler, SPOT>;
+        case 4: return slab_paths_kernel<R, kBates, kMilstein, SPOT>;
+        default: return slab_paths_kernel<R, kBates, kQE, SPOT>;
     }
 }
 
@@ -1138,7 +1145,7 @@ cudaError_t launch_merge(int n_tasks, int64_t n_chunks, cudaStream_t s, const Ta
 
 cudaError_t launch_slab_paths(int precision, int model, int scheme, uint64_t seed, cudaStream_t s, const TaskDev *task,
                               int64_t first_path, int64_t count, int stride, void *slab_S, void *slab_v, int64_t ld,
-                              int sm_count, int paths_per_thread, bool has_table) {
+                              int sm_count, int paths_per_thread, bool has_table, bool spot_steps) {
     const PhiloxRoundKeys rk = philox_round_keys(static_cast<uint32_t>(seed & 0xFFFFFFFFull),
                                                  static_cast<uint32_t>(seed >> 32));
     if (paths_per_thread == 2) {
@@ -1154,12 +1161,14 @@ cudaError_t launch_slab_paths(int precision, int model, int scheme, uint64_t see
         return cudaGetLastError();
     }
     const int64_t blocks = (count + kPathBlock - 1) / kPathBlock;
+    const auto launch = [&](auto kernel, auto *S, auto *v) {
+        kernel<<<static_cast<unsigned>(blocks), kPathBlock, 0, s>>>(task, first_path, count, stride, S, v, ld, rk);
+    };
     if (precision == QK_FP32)
-        slab_kernel_for<float>(model, scheme)<<<static_cast<unsigned>(blocks), kPathBlock, 0, s>>>(
-            task, first_path, count, stride, static_cast<float *>(slab_S), static_cast<float *>(slab_v), ld, rk);
+        launch(slab_kernel_for<float, false>(model, scheme), static_cast<float *>(slab_S), static_cast<float *>(slab_v));
     else
-        slab_kernel_for<double>(model, scheme)<<<static_cast<unsigned>(blocks), kPathBlock, 0, s>>>(
-            task, first_path, count, stride, static_cast<double *>(slab_S), static_cast<double *>(slab_v), ld, rk);
+        launch(spot_steps ? slab_kernel_for<double, true>(model, scheme) : slab_kernel_for<double, false>(model, scheme),
+               static_cast<double *>(slab_S), static_cast<double *>(slab_v));
     return cudaGetLastError();
 }
 
@@ -1242,7 +1251,9 @@ static cudaError_t preload_path_kernels_of() {
                 for (int lane = 0; lane < 3 && e == cudaSuccess; ++lane)
                     for (int trk = 0; trk < 4 && e == cudaSuccess; ++trk)
                         e = cudaFuncGetAttributes(&fa, price_kernel_for<R>(model, scheme, uk != 0, lane, trk));
-            if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, slab_kernel_for<R>(model, scheme));
+            if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, slab_kernel_for<R, false>(model, scheme));
+            if constexpr (sizeof(R) == 8)
+                if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, slab_kernel_for<R, true>(model, scheme));
             for (int tab = 0; tab < 2 && e == cudaSuccess; ++tab)
                 e = cudaFuncGetAttributes(&fa, slab_two_kernel_for(model, scheme, tab != 0));
             for (int trk = 0; trk < 4 && e == cudaSuccess; ++trk)
