@@ -146,7 +146,8 @@ struct WarpPhilox {
 
 // ============================================================================
 // Arithmetic policy.  FP32 uses the SFU (MUFU) approximations explicitly; FP64 uses the
-// functions of qk_math64.cuh in the path loop and the CUDA library in rare code.
+// functions of qk_math64.cuh in the path loop, the CUDA library in rare code and in
+// step_spot64.
 // ============================================================================
 template <class R>
 struct Math;
@@ -325,7 +326,8 @@ struct FedStep {
 // ============================================================================
 // Scheme steps: Heston + Euler (include/core/schemes/markovian/MSchemes.hpp:133-156),
 // + implicit Milstein (MSchemes.hpp:229-253), + Andersen QE with martingale correction
-// (MSchemes.hpp:363-442), in FP32 on the spot and in FP64 on its logarithm.  QE's
+// (MSchemes.hpp:363-442), in FP32 on the spot and in FP64 on its logarithm (step_spot64: on
+// the spot).  QE's
 // quadratic-branch martingale term log(exp(X)/sqrt(t)) is evaluated as X - log(t)/2 (the
 // same quantity without an exp/rsqrt/log round trip).
 // ============================================================================
