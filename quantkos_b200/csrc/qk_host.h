@@ -20,11 +20,17 @@ extern thread_local std::string g_last_error;  // message of the last failing ca
 // 442-563) on the fields a contract carries, plus this engine's own limits.
 qk_status validate_contract(const qk_contract &c, const qk_greeks *g);
 
-// The largest a of a QE step's quadratic regime: a = h / (m + G) <= h / m, a mediant of two
+// Above every a of a QE step's quadratic regime: a = h / (m + G) < h / m, a mediant of two
 // fixed ratios (see make_step_const).
 template <class R>
 inline double qe_a_max(const StepConst<R> &d) {
     return std::max(d.h_f1 / d.exp_mkdt, d.theta_m > 0.0 ? d.h_f2 / d.theta_m : 0.0);
+}
+
+// The least factor 1 - 2 A a of a QE step, where A > 0: G >= m sqrt(1 - psi_c / 2) in the
+// quadratic regime.
+inline double qe_least_factor(const StepConst<double> &d) {
+    return 1.0 - std::max(d.two_A * qe_a_max(d) / (1.0 + std::sqrt(std::max(0.0, 1.0 - 0.5 * d.psi_c))), 0.0);
 }
 
 // FP64 QE: steps between two folds of the martingale product.  As 1 - sum, the product has
@@ -32,7 +38,7 @@ inline double qe_a_max(const StepConst<R> &d) {
 // rho <= 0; rho > 0 at steps of a month), fewer otherwise, at least the two of a Philox block.
 inline int qe_fold_steps(const StepConst<double> &d) {
     if (!(d.h_psi_plain > 0.0)) return 16;  // no step has a factor
-    const double least = 1.0 - std::max(d.two_A * qe_a_max(d), 0.0);  // least factor 1 - 2 A a
+    const double least = qe_least_factor(d);
     int n = 16;
     while (n > 2 && !(least > 0.0 && std::pow(least, n) >= 0.5)) n /= 2;
     return n;
@@ -119,8 +125,8 @@ inline StepConst<R> make_step_const(const qk_contract &c, double dt, double eps)
     // the quadratic regime needs no clamp.  Elsewhere no step takes the plain form.
     const double a_max = qe_a_max(d);
     const bool plain = 2.0 * (d.A + eps) * a_max <= 1.0 - 1.0 / 1024.0 && std::fabs(d.two_A) * a_max < 1e12;
-    // (FP64 keeps 1 - 2 A a of two steps above 1/4 as well, see qe_fold_steps)
-    const bool two_steps = sizeof(R) == 4 || d.two_A * a_max <= 0.5;
+    // (FP64 keeps the factors of two steps above 1/4 as well, see qe_fold_steps)
+    const bool two_steps = sizeof(R) == 4 || qe_least_factor(d) >= 0.5;
     d.h_psi_plain = plain && two_steps ? 0.5 * d.psi_c : -1.0;
     // The paired FP32 step knows 2 / psi to 2^-21 (a reciprocal good to one unit in the last
     // place, two roundings): within these bounds, 2^-18 inside the regime's, the one-path
